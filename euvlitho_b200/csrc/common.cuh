@@ -46,6 +46,19 @@ __host__ __device__ __forceinline__ cplx csqrt_p(cplx z) {
   return mk(fabs(y) / (2.0 * t), copysign(t, y));
 }
 
+// Further terms of a batched GEMM, C = alpha A B + beta Cin + beta2 Cin2 + diag I:
+// Cin is C itself unless given, Cin2 is optional, both with C's leading dimension;
+// beta_b and beta2_b multiply beta and beta2 per batch entry (beta_b null: 1).
+struct GemmTerms {
+  const double2* cin = nullptr;
+  long long scin = 0;  // batch strides
+  const double2* beta_b = nullptr;
+  const double2* cin2 = nullptr;
+  long long scin2 = 0;
+  double2 beta2 = {0.0, 0.0};
+  const double2* beta2_b = nullptr;
+};
+
 // exp(z) for complex z.
 __host__ __device__ __forceinline__ cplx cexp_(cplx z) {
   double e = exp(z.x);

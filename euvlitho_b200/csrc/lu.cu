@@ -30,7 +30,7 @@ int zgemm_sub(int m, int n, int k, const double2* a, long long lda, long long sa
 int zgemm(int m, int n, int k, cplx alpha, const double* scale, const double2* a, long long lda,
           long long sa, const double2* b, long long ldb, long long sb, cplx beta, double2* c,
           long long ldc, long long sc, cplx diag, int batch, const int* steps, int step,
-          cudaStream_t stream);
+          cudaStream_t stream, const GemmTerms& terms = GemmTerms{});
 
 constexpr int LU_NB = 32;
 constexpr int LU_PANEL_THREADS = 512;

@@ -11,13 +11,15 @@
 //     X1 = c (G1^-1 G2 X2) - i s Y2,   Y1 = -i D s (G1^-1 G2 X2) + c Y2,
 // with c = cos(sqrt(D) d) and s = sin(sqrt(D) d)/sqrt(D) -- entire functions
 // of D, so no eigenvectors, square-root branches or W^-1 are needed.  At the
-// bottom (Ru cap, header.h:1292-1303) G2 X2 = diag(Bru (URUU+URUB)) and
-// Y2 = diag(alru (URUU-URUB)); at the top (header.h:1355-1391)
-// U0 = diag(klm) X + Y and FG = diag(1/klm) Y U0^-1, so
-//     Ax[:,s] = -diag(1/klm) Y U0^-1 (2 kz_s e_s) + e_s     (header.h:1394-1465).
-// c and s come from a degree-8 Taylor polynomial of A = D h^2 (Paterson-
-// Stockmeyer with A^2..A^4) at h = d/2^m, ||A||_1 <= 1, followed by m
-// double-angle steps s <- 2 s c, c <- 2 c^2 - I: every step is a GEMM.
+// bottom (Ru cap, header.h:1292-1303) G X2 = diag(Bru (URUU+URUB)) t and
+// Y2 = diag(alru (URUU-URUB)) t, i.e. the row relation P X2 + Q Y2 = 0 with
+// P = -diag(adm) G and Q = I, which the slices' c and s carry to the top; there
+// X1 = b + e, Y1 = diag(klm) (e - b) for incident e and reflected b
+// (header.h:1355-1391), one N x N system for b = Ax (header.h:1394-1465).
+// c and s are polynomials of D about its spectrum (slab polynomials below);
+// euv_matfun_cs, which takes any D, expands about 0 (a degree-8 Taylor
+// polynomial of A = D h^2 at h = d/2^m, then m double-angle steps s <- 2 s c,
+// c <- 2 c^2 - I).  Every step is a GEMM.
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
@@ -29,7 +31,7 @@ namespace euv {
 int zgemm(int m, int n, int k, cplx alpha, const double* scale, const double2* a, long long lda,
           long long sa, const double2* b, long long ldb, long long sb, cplx beta, double2* c,
           long long ldc, long long sc, cplx diag, int batch, const int* steps, int step,
-          cudaStream_t stream);
+          cudaStream_t stream, const GemmTerms& terms = GemmTerms{});
 int lu_factor(int n, double2* A, long long lda, long long sa, int* ipiv, int* info, int batch,
               cudaStream_t stream);
 // order (optional): per batch entry, ostride ints whose first nrhs mark the
@@ -41,7 +43,7 @@ int gemm_mixed(int m, int n, int k, cplx alpha, const double* scale, const doubl
                long long lda, long long sa, const double2* b, long long ldb, long long sb,
                cplx beta, double2* c, long long ldc, long long sc, cplx diag, int batch,
                const int* steps, int step, void* work, size_t work_bytes, int* status,
-               cudaStream_t stream, int reuse, const double2* cin);
+               cudaStream_t stream, int reuse, const GemmTerms& terms);
 size_t gemm_mixed_workspace_bytes(int m, int n, int k, int batch);
 
 // ||A||_1 bound for the degree-8 Taylor step of cos/sin(sqrt(A)): the dropped
@@ -207,17 +209,21 @@ struct SliceParams {
   cplx logeps;   // log(eps_abs)
 };
 
+// D gets the slab's normalised matrix (D - a I) / R, a and R of the unit in
+// shift (i a) and radius (poly_coef_kernel):
 // D(i,j) = k^2 eps[..] - i eta[..] kx_j (X) / - i zeta[..] ky_j (Y), minus kxy2_i
 // on the diagonal (header.h:416-443); G(i,j) = i(k delta_ij - kp_i/k sigma[..] kp_j)
-// (B1 = G W1, header.h:596-623).  want_d/want_g select the outputs.
+// (B1 = G W1, header.h:596-623).  D may be null; want_g = 1:
+// G, 2 E with G = i k (I - E), 3 the bottom boundary row -diag(adm) G.
 __global__ void build_dg_kernel(SliceParams p, const double2* spectra, const int* spec_of_unit,
                                 const int* lidx, const int* midx, const double* kx0,
-                                const double* ky0, const int* polar, double2* D, double2* G,
-                                int want_d, int want_g) {
+                                const double* ky0, const int* polar, const double2* adm,
+                                const double2* shift, const double* radius, double2* D,
+                                long long sd, double2* G, long long sg, int want_g) {
   // grid: x = column j, y = row chunk, z = unit (no 64-bit division per element)
   const int u = blockIdx.z, j = blockIdx.x;
   // the unit's and column's constants once per CTA: no FP64 division per element
-  __shared__ double s_c[8];  // 2pi/dx, 2pi/dy, 1/k, kx_j, ky_j, kx0, ky0
+  __shared__ double s_c[10];  // 2pi/dx, 2pi/dy, 1/k, kx_j, ky_j, kx0, ky0, a, 1/R
   if (threadIdx.x == 0) {
     const double twopi = 6.283185307179586476925286766559;
     const double dxu = p.dxs ? p.dxs[u] : p.dx, dyu = p.dys ? p.dys[u] : p.dy;
@@ -229,11 +235,15 @@ __global__ void build_dg_kernel(SliceParams p, const double2* spectra, const int
     s_c[4] = ky0[u] + gy * midx[j];
     s_c[5] = kx0[u];
     s_c[6] = ky0[u];
+    if (D != nullptr) {
+      s_c[7] = shift[u].y;   // shift holds i a
+      s_c[8] = -shift[u].x;
+      s_c[9] = 1.0 / radius[u];
+    }
   }
   __syncthreads();
   const int i = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= p.n) return;
-  const long long nn = (long long)p.n * p.n;
   const long long t = (long long)j * p.n + i;
   const int li = lidx[i], mi = midx[i], lj = lidx[j], mj = midx[j];
   const int l = li - lj + 2 * p.lmax, m = mi - mj + 2 * p.mmax;
@@ -245,7 +255,7 @@ __global__ void build_dg_kernel(SliceParams p, const double2* spectra, const int
   const double kxi = s_c[5] + gx * li, kyi = s_c[6] + gy * mi;
   const double kxj = s_c[3], kyj = s_c[4];
   const int pol = polar[u];
-  if (want_d) {
+  if (D != nullptr) {
     cplx eps = p.eps_m1 * F;
     if (dc) eps.x += 1.0;
     cplx leps = p.logeps * F;
@@ -256,8 +266,11 @@ __global__ void build_dg_kernel(SliceParams p, const double2* spectra, const int
     } else {
       v = v + (gy * (double)(m - 2 * p.mmax) * kyj) * leps;
     }
-    if (i == j) v.x -= kxi * kxi + kyi * kyi;
-    D[(long long)u * nn + t] = make_double2(v.x, v.y);
+    if (i == j) {
+      v.x -= kxi * kxi + kyi * kyi + s_c[7];
+      v.y -= s_c[8];
+    }
+    D[(long long)u * sd + t] = make_double2(s_c[9] * v.x, s_c[9] * v.y);
   }
   if (want_g) {
     cplx sig = p.sig_m1 * F;
@@ -266,33 +279,19 @@ __global__ void build_dg_kernel(SliceParams p, const double2* spectra, const int
     if (want_g == 2) {
       // E = diag(kp/k) sigma diag(kp/k), with G = i k (I - E)
       cplx v = (kpi * ik * (kpj * ik)) * sig;
-      G[(long long)u * nn + t] = make_double2(v.x, v.y);
+      G[(long long)u * sg + t] = make_double2(v.x, v.y);
     } else {
       // G = i (k delta - kp_i/k sig kp_j)
       cplx a = (-kpi * ik * kpj) * sig;
       if (i == j) a.x += p.k;
       cplx v = cmul_i(a);
-      G[(long long)u * nn + t] = make_double2(v.x, v.y);
+      if (want_g == 3) {
+        const double2 y = adm[(long long)u * p.n + i];
+        v = -(mk(y.x, y.y) * v);
+      }
+      G[(long long)u * sg + t] = make_double2(v.x, v.y);
     }
   }
-}
-
-// Z = s * (R + E R) with R = diag(v) (dense == 0) or R dense: the first factor
-// of the Euler product (I - E)^-1 = (I + E)(I + E^2)(I + E^4)...
-__global__ void euler_first_diag_kernel(int n, cplx s, const double2* E, const double2* v,
-                                        double2* Z) {
-  const long long nn = (long long)n * n;
-  const int b = blockIdx.y;
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nn) return;
-  const long long o = (long long)b * nn + t;
-  const int i = (int)(t % n), j = (int)(t / n);
-  const double2 vv = v[(long long)b * n + j];
-  const double2 e = E[o];
-  cplx r = mk(e.x, e.y) * mk(vv.x, vv.y);
-  if (i == j) r = r + mk(vv.x, vv.y);
-  r = s * r;
-  Z[o] = make_double2(r.x, r.y);
 }
 
 // ---------------------------------------------------------------- multilayer
@@ -331,12 +330,11 @@ __device__ __forceinline__ void apply_blk(const Blk& b, cplx& uu, cplx& ub) {
 }
 
 // Per order: URUU, URUB (header.h:5-363), alru, Bru (header.h:1292-1303), and
-// the bottom boundary data x2 = URUU+URUB, y2 = alru (URUU-URUB),
+// the admittance y2 / gx2 of the bottom boundary, y2 = alru (URUU-URUB) and
 // gx2 = Bru (URUU+URUB); klm = sqrt(k^2-kxy2) as a real root (header.h:1283).
 __global__ void multilayer_kernel(StackParams p, const int* lidx, const int* midx,
                                   const double* kx0, const double* ky0, const int* polar,
-                                  double2* x2, double2* y2, double2* gx2, double* klm,
-                                  int n_units) {
+                                  double2* adm, double* klm, int n_units) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= p.n * n_units) return;
   const int u = t / p.n, i = t % p.n;
@@ -374,11 +372,10 @@ __global__ void multilayer_kernel(StackParams p, const int* lidx, const int* mid
   apply_blk(TRU, uu, ub);  // URUU, URUB (header.h:361-362)
   const cplx bru = mk(0.0, k) - cmul_i(cdiv(mk(kp * kp / k, 0.0), p.eru));
   const cplx s = uu + ub, d = uu - ub;
-  x2[t] = make_double2(s.x, s.y);
-  cplx yv = alru * d;
-  y2[t] = make_double2(yv.x, yv.y);
-  cplx gv = bru * s;
-  gx2[t] = make_double2(gv.x, gv.y);
+  // a node of the total field (gx2 = 0) is the limit of a large admittance
+  const cplx gv = bru * s;
+  const cplx yv = (gv.x == 0.0 && gv.y == 0.0) ? mk(1e30, 0.0) : cdiv(alru * d, gv);
+  adm[t] = make_double2(yv.x, yv.y);
   klm[t] = sqrt(k2 - kxy2);  // NaN for evanescent orders, as the reference
 }
 
@@ -465,79 +462,450 @@ __global__ void taylor_prep_kernel(int n, int batch, const double2* D, const dou
   Ts[o] = make_double2(hb * tsx, hb * tsy);
 }
 
-// ---------------------------------------------------------------- elementwise
-// out[b](i,j) = alpha * A[b](i,j) * v[b][j] + beta * out[b](i,j)
-__global__ void colscale_kernel(int n, cplx alpha, const double2* A, const double2* v, cplx beta,
-                                double2* out) {
-  const long long nn = (long long)n * n;
-  const int b = blockIdx.y;
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nn) return;
-  const long long o = (long long)b * nn + t;
-  const int j = (int)(t / n);
-  double2 a = A[o], vv = v[(long long)b * n + j];
-  cplx r = alpha * (mk(a.x, a.y) * mk(vv.x, vv.y));
-  if (beta.x != 0.0 || beta.y != 0.0) {
-    double2 q = out[o];
-    r = r + beta * mk(q.x, q.y);
+// ---------------------------------------------------------------- slab polynomials
+// c = cos(sqrt(D) d) and s = sin(sqrt(D) d)/sqrt(D) as polynomials in D about
+// its spectrum.  D = k^2 T(eps) - diag(kxy^2) + (small commutator): the finite
+// Toeplitz section T(eps) of a two-valued pattern has its field of values on
+// the segment from 1 to eps_abs, the diagonal is real, and the log(eps) term is
+// a commutator of norm <= w.  So the field of values lies in a flat ellipse
+// around a (centre, foci a +- c, sum of semi-axes |c| rho), known from the
+// configuration alone, and a Chebyshev expansion on it converges like
+// tau^n / n!, tau = d (sum of semi-axes) / (4 |sqrt a|): about 1 for a 60 nm
+// slab, where the expansion about 0 needs ||D||_1 d^2 ~ 10^3 halved by 5 to 6
+// double-angle steps (two products each, and each doubles the error).
+// Evaluated as a polynomial in E = (D - a)/R by blocks of q powers (Paterson-
+// Stockmeyer): p = c_0 + B_0 + E^q (B_1 + E^q (...)), B_j = sum_{1..q} c_{qj+i}
+// E^i.  The identity part c_0 stays a number per unit: the matrices c - c_0 and
+// s - s_0 that enter later products are then small against c_0 and s_0, and so is
+// the error the split products make (their FP32 sums lose 2^-24 of the running
+// sum at every step; with the identity inside the operands the 2048 nm
+// eight-slice image was 1.6e-5 off, 7e-6 for the expansion about 0).  Products: q - 1 for the powers and
+// 2 (J - 1) for the two functions; q and J from poly_plan, a double-angle step
+// only where degree q * jcap is not enough (clips of a few hundred nm with
+// orders near grazing).  With the row recursion of euv_amp (no G^-1, no product
+// with the solved columns) the call takes 8 N^3 products instead of 25 for a 60
+// nm slab in the mixed form.  B200, whole image calls: four 1024 nm clips at N =
+// 625 (24 units, mixed) 11.64 -> 8.15 ms and 1.1e-5 -> 1.5e-6 of the exact image;
+// N = 961, 6 units, FP64 46.9 -> 27.2 ms; M3D at N = 2177, FP64 94.1 -> 53.5 ms.
+constexpr int PF_K = 24;       // largest degree
+constexpr int PF_Q = 6;        // largest q
+constexpr int PF_J = 6;        // largest block count (q = 4)
+constexpr int PF_SAMPLES = 64; // points on the ellipse
+constexpr double kPolyTolFp64 = 1e-16;
+constexpr double kPolyTolMixed = 5e-8;  // the split products carry ~1e-6
+
+struct PolyRegion {
+  cplx a, c;         // centre, focal half-axis (complex)
+  double rho, r;     // ellipse a + c (rho e^it + e^-it / rho)/2; scale of E
+};
+
+// kxy2 in [lo, hi] over the orders; w: norm bound of the commutator term.
+__host__ __device__ inline PolyRegion poly_region(double k, cplx eps_m1, double lo, double hi,
+                                                  double w) {
+  const cplx u = (0.5 * k * k) * eps_m1, v = mk(0.5 * (hi - lo), 0.0);
+  PolyRegion g;
+  g.a = mk(k * k + u.x - 0.5 * (hi + lo), u.y);
+  w += 1e-9 * k * k;
+  // parallelogram with corners +-p, +-q; foci along the principal direction
+  const cplx p = u + v, q = u - v;
+  const double lp = cabs(p), lq = cabs(q), len = lp > lq ? lp : lq;
+  cplx dir = csqrt_p(u * u + v * v);
+  const double ld = cabs(dir);
+  dir = ld > 0.0 ? (1.0 / ld) * dir : mk(1.0, 0.0);
+  double best_sum = 2.0 * len, best_c = 0.0;  // the circle through the far corner
+  for (int t = 1; t <= 16 && len > 0.0; ++t) {
+    const double cm = len * t / 16.0;
+    double rho = 1.0;
+    for (int i = 0; i < 2; ++i) {
+      const cplx x = cdiv(i ? q : p, cm * dir);
+      const double m = cabs(x + csqrt_p(x * x - mk(1.0, 0.0)));
+      const double r = m > 1.0 ? m : 1.0 / m;
+      if (r > rho) rho = r;
+    }
+    if (cm * rho < best_sum) {
+      best_sum = cm * rho;
+      best_c = cm;
+    }
   }
-  out[o] = make_double2(r.x, r.y);
+  // semi-axes, widened by the disc of radius w
+  const double minor2 = best_sum > 0.0 ? best_c * best_c / best_sum : 0.0;  // a - b
+  const double sa = 0.5 * (best_sum + minor2) + w, sb = 0.5 * (best_sum - minor2) + w;
+  double cm = sqrt((sa - sb) * (sa + sb));
+  if (cm < 0.02 * sa) cm = 0.02 * sa;  // near a circle: keep the foci apart
+  g.c = cm * dir;
+  g.rho = (sa + sb) / cm;
+  g.r = sa;
+  return g;
 }
 
-// out[b] = diag(v[b])
-__global__ void diag_kernel(int n, const double2* v, double2* out) {
-  const long long nn = (long long)n * n;
-  const int b = blockIdx.y;
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nn) return;
-  const int i = (int)(t % n), j = (int)(t / n);
-  out[(long long)b * nn + t] = (i == j) ? v[(long long)b * n + i] : make_double2(0.0, 0.0);
+// Degree that brings the first dropped term of both functions below tol: the
+// bound tau^n/n! with the smallest |sqrt z| on the ellipse, or, where the
+// ellipse comes near 0, the Taylor bound (h^2 |z|)^n / (2n)!.  PF_K + 1: more.
+__host__ __device__ inline int poly_degree(const PolyRegion& g, double h, double tol) {
+  const double a = cabs(g.a), sum = g.rho * cabs(g.c);
+  const double near = a - g.r;
+  const double tau = near > 0.0 ? 0.25 * h * sum / sqrt(near) : 1e300;
+  const double z = h * h * (a + g.r);
+  double t1 = 2.0, t2 = 2.0;
+  for (int n = 1; n <= PF_K + 1; ++n) {
+    t1 *= tau / n;
+    t2 *= z / ((2.0 * n - 1.0) * (2.0 * n));
+    if (t1 <= tol || t2 <= tol) return n > 1 ? n - 1 : 1;
+  }
+  return PF_K + 1;
 }
 
-// U0 = diag(klm) X + Y (header.h:1355-1371 in X,Y form)
-__global__ void u0_kernel(int n, const double* klm, const double2* X, const double2* Y,
-                          double2* U0) {
-  const long long nn = (long long)n * n;
-  const int b = blockIdx.y;
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nn) return;
-  const long long o = (long long)b * nn + t;
-  const int i = (int)(t % n);
-  const double kl = klm[(long long)b * n + i];
-  double2 x = X[o], y = Y[o];
-  U0[o] = make_double2(kl * x.x + y.x, kl * x.y + y.y);
+struct PolyPlan {
+  int q, jcap, j, m;  // powers, block limit; blocks and double-angle steps launched
+};
+
+// q from the slab alone (not from the orders or periods, so that clips of
+// different periods share a launch and a unit's arithmetic does not depend on
+// the others): the q with the fewest products at the degrees such slabs need.
+// tau0 = d k |eps - 1| / 4 is the pattern's part of tau.  Mixed (tol 5e-8):
+// 7.5 nm slices take degree 5-6 (q = 3: 4 products), 20-30 nm 7-8 (q = 4: 5),
+// 60 nm 10-11 (q = 5, J = 2..3: 6-8); FP64: 10-12 (q = 5) and 18-20 (q = 6).
+__host__ __device__ inline void poly_shape(int precision, double k, cplx eps_m1, double d, int* q,
+                                           int* jcap) {
+  const double tau0 = 0.25 * d * k * cabs(eps_m1);
+  if (precision == EUV_PREC_MIXED) {
+    *q = tau0 < 0.16 ? 3 : (tau0 < 0.5 ? 4 : 5);
+    *jcap = *q == 5 ? 3 : 4;
+  } else {
+    *q = tau0 < 0.2 ? 5 : 6;
+    *jcap = 4;
+  }
 }
 
-// E[b](i,s) = 2kz_s if i == src_order[b][s] else 0 (AS of header.h:1402-1409)
-__global__ void src_rhs_kernel(int n, int nsrc, const int* src_order, const double* src_2kz,
-                               double2* E) {
-  const int b = blockIdx.y;
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)n * nsrc) return;
-  const int i = (int)(t % n), s = (int)(t / n);
+// Blocks and double-angle steps of one unit: the fewest steps with which jcap
+// blocks reach the degree, at most m_max steps.  Returns false when they do not.
+__host__ __device__ inline bool poly_pick(const PolyRegion& g, double d, double tol, int q,
+                                          int jcap, int m_max, int* j, int* m) {
+  for (int mm = 0;; ++mm) {
+    const int deg = poly_degree(g, ldexp(d, -mm), tol);
+    const int jj = (deg + q - 1) / q;
+    if (jj <= jcap && deg <= PF_K) {
+      *j = jj;
+      *m = mm;
+      return true;
+    }
+    if (mm >= m_max) {
+      *j = jcap;
+      *m = mm;
+      return false;
+    }
+  }
+}
+
+struct PolySlices {
+  double k, dx, dy;
+  const double* dxs;
+  const double* dys;
+  int n, lmax, mmax, n_slices, n_units;
+  double tol;
+  cplx eps_m1[EUV_MAX_SLICES];
+  double leps[EUV_MAX_SLICES];  // |log eps|
+  double d[EUV_MAX_SLICES];
+  int q[EUV_MAX_SLICES], jcap[EUV_MAX_SLICES], j[EUV_MAX_SLICES], m[EUV_MAX_SLICES];
+};
+
+// Coefficients of block b, function f of (unit, slice): PF_Q complex values, the
+// factor of E^(i+1) at i.
+__host__ __device__ inline long long poly_coef_at(int n_units, int slice, int unit, int f, int b) {
+  return ((((long long)slice * n_units + unit) * 2 + f) * PF_J + b) * PF_Q;
+}
+// Identity parts [unit] of function f of a slice after t double-angle steps.
+__host__ __device__ inline long long poly_id_at(int n_units, int slice, int t, int f) {
+  return (((long long)slice * (kMaxSteps + 1) + t) * 2 + f) * n_units;
+}
+
+// One CTA of 64 threads per (unit, slice): the ellipse from the unit's own
+// orders, the two functions at 64 points of it, their Fourier coefficients there
+// (= Chebyshev coefficients times rho^n / 2) and from those the block
+// coefficients.  Latency of one small launch for all slices; it replaces the
+// three norm / scaling launches per slice of the expansion about 0.
+__global__ void __launch_bounds__(PF_SAMPLES)
+    poly_coef_kernel(PolySlices p, const int* lidx, const int* midx, const double* kx0,
+                     const double* ky0, const int* polar, double2* coef, double2* ident,
+                     double2* shift, double* radius, int* steps, int* status) {
+  const int u = blockIdx.x, sl = blockIdx.y, tid = threadIdx.x;
+  __shared__ double s_lo[2], s_hi[2], s_km[2];
+  __shared__ cplx s_f[2][PF_SAMPLES], s_w[PF_SAMPLES], s_a[2][PF_K + 1];
+  const double twopi = 6.283185307179586476925286766559;
+  const double gx = twopi / (p.dxs ? p.dxs[u] : p.dx), gy = twopi / (p.dys ? p.dys[u] : p.dy);
+  const bool pol_x = polar[u] == 0;
+  double lo = 1e300, hi = 0.0, km = 0.0;
+  for (int i = tid; i < p.n; i += PF_SAMPLES) {
+    const double kx = kx0[u] + gx * lidx[i], ky = ky0[u] + gy * midx[i];
+    const double v = kx * kx + ky * ky;
+    lo = fmin(lo, v);
+    hi = fmax(hi, v);
+    km = fmax(km, fabs(pol_x ? kx : ky));
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+    km = fmax(km, __shfl_xor_sync(0xffffffffu, km, off));
+  }
+  if ((tid & 31) == 0) {
+    s_lo[tid >> 5] = lo;
+    s_hi[tid >> 5] = hi;
+    s_km[tid >> 5] = km;
+  }
+  __syncthreads();
+  lo = fmin(s_lo[0], s_lo[1]);
+  hi = fmax(s_hi[0], s_hi[1]);
+  km = fmax(s_km[0], s_km[1]);
+  // every thread takes the same decisions from the same numbers
+  const double w = (pol_x ? gx * p.lmax : gy * p.mmax) * p.leps[sl] * km;
+  const PolyRegion g = poly_region(p.k, p.eps_m1[sl], lo, hi, w);
+  const int q = p.q[sl], jl = p.j[sl];
+  int jb, m;
+  bool ok = poly_pick(g, p.d[sl], p.tol, q, p.jcap[sl], p.m[sl], &jb, &m);
+  if (jb > jl) {  // more blocks than launched
+    jb = jl;
+    ok = poly_degree(g, ldexp(p.d[sl], -m), 100.0 * p.tol) <= q * jb;
+  }
+  const double h = ldexp(p.d[sl], -m);
+  {
+    double sn, cs;
+    sincospi(2.0 * tid / PF_SAMPLES, &sn, &cs);
+    s_w[tid] = mk(cs, -sn);  // e^{-i theta}
+    const cplx dz = g.c * mk(0.5 * (g.rho + 1.0 / g.rho) * cs, 0.5 * (g.rho - 1.0 / g.rho) * sn);
+    const cplx r = csqrt_p(g.a + dz), ra = csqrt_p(g.a), rs = r + ra;
+    // e^{i h sqrt z} as e^{i h sqrt a} e^{i h (sqrt z - sqrt a)}: the difference
+    // without cancellation
+    const cplx dphi = (rs.x == 0.0 && rs.y == 0.0) ? mk(0.0, 0.0) : h * cdiv(dz, rs);
+    const cplx ep = cexp_(cmul_i(h * ra)) * cexp_(cmul_i(dphi));
+    const cplx em = cexp_(-cmul_i(h * ra)) * cexp_(-cmul_i(dphi));
+    s_f[0][tid] = 0.5 * (ep + em);
+    const cplx x2 = (h * h) * (r * r);
+    s_f[1][tid] = cabs1(x2) < 1e-4
+                      ? h * (mk(1.0, 0.0) - (1.0 / 6.0) * x2 + (1.0 / 120.0) * (x2 * x2))
+                      : cdiv(0.5 * (ep - em), cmul_i(r));
+  }
+  __syncthreads();
+  const int deg = q * jb;
+  if (tid < 2 * (PF_K + 1)) {
+    const int f = tid / (PF_K + 1), n = tid % (PF_K + 1);
+    cplx s = mk(0.0, 0.0);
+    for (int t = 0; t < PF_SAMPLES; ++t) s = s + s_f[f][t] * s_w[(n * t) % PF_SAMPLES];
+    // a_n of sum a_n T_n: f^_n = a_n rho^n / 2 (n > 0)
+    double e = (n ? 2.0 : 1.0) / PF_SAMPLES;
+    for (int t = 0; t < n; ++t) e /= g.rho;
+    s_a[f][n] = n <= deg ? e * s : mk(0.0, 0.0);
+  }
+  __syncthreads();
+  // monomial coefficients in E = (z - a)/R: lane i of warp f collects the E^i
+  // terms of T_n(E R / c) with the three-term recurrence
+  const int f = tid >> 5, lane = tid & 31;
+  const cplx ratio = cdiv(mk(g.r, 0.0), g.c);
+  double tp = 0.0, tc = lane == 0 ? 1.0 : 0.0;  // T_{n-1}, T_n
+  cplx acc = mk(0.0, 0.0);
+  for (int n = 0; n <= deg; ++n) {
+    acc = acc + tc * s_a[f][n];
+    double up = __shfl_up_sync(0xffffffffu, tc, 1);
+    if (lane == 0) up = 0.0;
+    const double tn = n == 0 ? up : 2.0 * up - tp;
+    tp = tc;
+    tc = tn;
+  }
+  for (int t = 0; t < lane && t < PF_K; ++t) acc = acc * ratio;
+  double2* out = coef + poly_coef_at(p.n_units, sl, u, f, 0);
+  for (int b = 0; b < PF_J; ++b) {
+    const int i = lane - 1 - q * b;
+    if (lane < PF_Q) out[b * PF_Q + lane] = make_double2(0.0, 0.0);
+    __syncwarp();
+    if (b < jb && i >= 0 && i < q) out[b * PF_Q + i] = make_double2(acc.x, acc.y);
+  }
+  if (lane == 0) s_a[f][0] = acc;
+  __syncthreads();
+  if (tid == 0) {
+    const long long t = (long long)sl * p.n_units + u;
+    const cplx ia = cmul_i(g.a);
+    shift[t] = make_double2(ia.x, ia.y);
+    radius[t] = g.r;
+    steps[t] = m;
+    cplx c = s_a[0][0], sn = s_a[1][0];
+    for (int i = 0; i <= p.m[sl]; ++i) {
+      ident[poly_id_at(p.n_units, sl, i, 0) + u] = make_double2(c.x, c.y);
+      ident[poly_id_at(p.n_units, sl, i, 1) + u] = make_double2(sn.x, sn.y);
+      if (i < m) {
+        sn = 2.0 * (sn * c);
+        c = 2.0 * (c * c) - mk(1.0, 0.0);
+      }
+    }
+    if (!ok) atomicOr(status, EUV_STATUS_STEPS_CLAMPED);
+  }
+}
+
+// Blocks B_b of both functions for b = b0 (and b0 - 1 when NB = 2), [c | s] side
+// by side per unit, from E..E^q (one unit's powers nn apart, units sp apart).
+// HBM-bound: q reads and 2 NB writes of 16 bytes per element.
+template <int Q, int NB>
+__global__ void __launch_bounds__(256)
+    poly_block_kernel(int n, const double2* pw, long long sp, const double2* coef, int n_units,
+                      int slice, int b0, double2* top, double2* low, long long so) {
+  __shared__ double2 s_c[NB][2][Q];
+  const int u = blockIdx.z, j = blockIdx.x;
+  if (threadIdx.x < NB * 2 * Q) {
+    const int t = threadIdx.x, i = t % Q, f = (t / Q) % 2, b = t / (2 * Q);
+    s_c[b][f][i] = coef[poly_coef_at(n_units, slice, u, f, b0 - b) + i];
+  }
+  __syncthreads();
+  const int i = blockIdx.y * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const long long nn = (long long)n * n, t = (long long)j * n + i;
+  double2 x[Q];
+#pragma unroll
+  for (int e = 0; e < Q; ++e) x[e] = pw[(long long)u * sp + e * nn + t];
+#pragma unroll
+  for (int b = 0; b < NB; ++b)
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+      cplx v = mk(0.0, 0.0);
+#pragma unroll
+      for (int e = 0; e < Q; ++e) v = v + mk(s_c[b][f][e].x, s_c[b][f][e].y) * mk(x[e].x, x[e].y);
+      (b ? low : top)[(long long)u * so + f * nn + t] = make_double2(v.x, v.y);
+    }
+}
+
+template <int NB>
+static int poly_blocks(int q, int n, const double2* pw, long long sp, const double2* coef, int U,
+                       int slice, int b0, double2* top, double2* low, long long so,
+                       cudaStream_t stream) {
+  const dim3 g((unsigned)n, (unsigned)((n + 255) / 256), U);
+  switch (q) {
+    case 3: poly_block_kernel<3, NB><<<g, 256, 0, stream>>>(n, pw, sp, coef, U, slice, b0, top, low, so); break;
+    case 4: poly_block_kernel<4, NB><<<g, 256, 0, stream>>>(n, pw, sp, coef, U, slice, b0, top, low, so); break;
+    case 5: poly_block_kernel<5, NB><<<g, 256, 0, stream>>>(n, pw, sp, coef, U, slice, b0, top, low, so); break;
+    default: poly_block_kernel<6, NB><<<g, 256, 0, stream>>>(n, pw, sp, coef, U, slice, b0, top, low, so); break;
+  }
+  EUV_LAUNCH_CHECK();
+  return EUV_OK;
+}
+
+// ---------------------------------------------------------------- elementwise
+// Top interface (klm = diag of the vacuum wave numbers, columns scaled).  With
+// c = c0 + C, s = s0 + S, D = a + R E the rows c - i s klm and i D s - c klm are
+//   diag(v) + V,  V = C - i S klm,                          v = c0 - i s0 klm
+//   diag(w) + W,  W = i R E S + i a S + i R s0 E - C klm,    w = i a s0 - c0 klm
+// (W holds i R E S on entry), and M takes the diagonal parts' share of
+// P (diag(v) + V) + Q (diag(w) + W); Q = I when null, with W's whole share.
+// Batch strides: sc (C, S), sw (E, V, W, M), sp (P, Q).
+__global__ void top_rows_kernel(int n, const double* klm, const double2* shift,
+                                const double* radius, const double2* c0, const double2* s0,
+                                const double2* C, const double2* S, long long sc, const double2* E,
+                                double2* V, double2* W, double2* M, long long sw, const double2* P,
+                                const double2* Q, long long sp) {
+  const int b = blockIdx.z, j = blockIdx.x;
+  const int i = blockIdx.y * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const long long t = (long long)j * n + i;
+  const double kl = klm[(long long)b * n + j];
+  const cplx ia = mk(shift[b].x, shift[b].y), u0 = mk(c0[b].x, c0[b].y), u1 = mk(s0[b].x, s0[b].y);
+  const cplx v = u0 - kl * cmul_i(u1), w = ia * u1 - kl * u0;
+  const double2 c2 = C[b * sc + t], s2 = S[b * sc + t], e2 = E[b * sw + t], w2 = W[b * sw + t];
+  const double2 p2 = P[b * sp + t];
+  const cplx c = mk(c2.x, c2.y), s = mk(s2.x, s2.y);
+  const cplx vv = c - kl * cmul_i(s);
+  const cplx ww = mk(w2.x, w2.y) + ia * s + (radius[b] * cmul_i(u1)) * mk(e2.x, e2.y) - kl * c;
+  cplx m = mk(p2.x, p2.y) * v;
+  if (Q != nullptr) {
+    const double2 q2 = Q[b * sp + t];
+    m = m + mk(q2.x, q2.y) * w;
+  } else {
+    m = m + ww;
+    if (i == j) m = m + w;
+  }
+  V[b * sw + t] = make_double2(vv.x, vv.y);
+  W[b * sw + t] = make_double2(ww.x, ww.y);
+  M[b * sw + t] = make_double2(m.x, m.y);
+}
+
+// The same for the incident wave of the source columns (klm -> -klm), o =
+// src_order[s]: V2[:, s], W2[:, s], and the diagonal parts' share of the right-hand
+// side -(P (diag + V2) + Q (diag + W2)) in rhs; zero for empty slots.
+__global__ void source_rows_kernel(int n, int nsrc, const int* src_order, const double* klm,
+                                   const double2* shift, const double2* c0, const double2* s0,
+                                   const double2* C, const double2* S, long long sc,
+                                   const double2* V, const double2* W, long long sw,
+                                   const double2* P, const double2* Q, long long sp, double2* V2,
+                                   double2* W2, double2* rhs) {
+  const int b = blockIdx.z, s = blockIdx.x;
+  const int i = blockIdx.y * blockDim.x + threadIdx.x;
+  if (i >= n) return;
   const int o = src_order[(long long)b * nsrc + s];
-  double v = (i == o) ? src_2kz[(long long)b * nsrc + s] : 0.0;
-  E[(long long)b * n * nsrc + t] = make_double2(v, 0.0);
-}
-
-// Ax[b](i,s) = -(1/klm_i) YZ[b](i,s) + [i == src_order] (header.h:1449-1461)
-__global__ void ax_out_kernel(int n, int nsrc, const int* src_order, const double* klm,
-                              const double2* YZ, double2* ax) {
-  const int b = blockIdx.y;
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)n * nsrc) return;
-  const int i = (int)(t % n), s = (int)(t / n);
-  const int o = src_order[(long long)b * nsrc + s];
-  const long long off = (long long)b * n * nsrc + t;
+  const long long t = ((long long)b * nsrc + s) * n + i;
   if (o < 0) {
-    ax[off] = make_double2(0.0, 0.0);
+    V2[t] = W2[t] = rhs[t] = make_double2(0.0, 0.0);
     return;
   }
-  const double kl = klm[(long long)b * n + i];
-  double2 v = YZ[off];
-  double rx = -v.x / kl, ry = -v.y / kl;
-  if (i == o) rx += 1.0;
-  ax[off] = make_double2(rx, ry);
+  const long long e = (long long)o * n + i;
+  const double kl = klm[(long long)b * n + o];
+  const cplx ia = mk(shift[b].x, shift[b].y), u0 = mk(c0[b].x, c0[b].y), u1 = mk(s0[b].x, s0[b].y);
+  const cplx v = u0 + kl * cmul_i(u1), w = ia * u1 + kl * u0;
+  const double2 cv = C[b * sc + e], sv = S[b * sc + e], vv = V[b * sw + e], wv = W[b * sw + e];
+  const double2 pv = P[b * sp + e];
+  const cplx w2 = mk(wv.x + 2.0 * kl * cv.x, wv.y + 2.0 * kl * cv.y);
+  cplx r = mk(pv.x, pv.y) * v;
+  if (Q != nullptr) {
+    const double2 qv = Q[b * sp + e];
+    r = r + mk(qv.x, qv.y) * w;
+  } else {
+    r = r + w2;
+    if (i == o) r = r + w;
+  }
+  V2[t] = make_double2(vv.x - 2.0 * kl * sv.y, vv.y + 2.0 * kl * sv.x);
+  W2[t] = make_double2(w2.x, w2.y);
+  rhs[t] = make_double2(-r.x, -r.y);
+}
+
+// Bottom of several slices (Q = I): what of P c + i D s and c + i P s is not a
+// product of two matrices,
+//   R1 = c0 P + i a S + i R s0 E + i a s0,   R2 = C + i s0 P + c0.
+__global__ void bottom_rows_kernel(int n, const double2* shift, const double* radius,
+                                   const double2* c0, const double2* s0, const double2* C,
+                                   const double2* S, long long sc, const double2* E, long long se,
+                                   const double2* P, long long sp, double2* R1, double2* R2,
+                                   long long sr) {
+  const int b = blockIdx.z, j = blockIdx.x;
+  const int i = blockIdx.y * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const long long t = (long long)j * n + i;
+  const cplx ia = mk(shift[b].x, shift[b].y), u0 = mk(c0[b].x, c0[b].y), u1 = mk(s0[b].x, s0[b].y);
+  const double2 c2 = C[b * sc + t], s2 = S[b * sc + t], e2 = E[b * se + t], p2 = P[b * sp + t];
+  const cplx p = mk(p2.x, p2.y);
+  cplx r1 = u0 * p + ia * mk(s2.x, s2.y) + (radius[b] * cmul_i(u1)) * mk(e2.x, e2.y);
+  cplx r2 = mk(c2.x, c2.y) + cmul_i(u1) * p;
+  if (i == j) {
+    r1 = r1 + ia * u1;
+    r2 = r2 + u0;
+  }
+  R1[b * sr + t] = make_double2(r1.x, r1.y);
+  R2[b * sr + t] = make_double2(r2.x, r2.y);
+}
+
+// Ax[b](i,s) = r x + (1 - r) [i == src_order], r = src_2kz / (2 klm): x is the
+// reflected amplitude of a unit wave in order src_order, the caller's 2 kz its
+// weight (header.h:1394-1465); zero for empty slots.  In place.
+__global__ void ax_out_kernel(int n, int nsrc, const int* src_order, const double* src_2kz,
+                              const double* klm, double2* ax) {
+  const int b = blockIdx.z, s = blockIdx.x;
+  const int i = blockIdx.y * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const long long bs = (long long)b * nsrc + s;
+  const int o = src_order[bs];
+  if (o < 0) {
+    ax[bs * n + i] = make_double2(0.0, 0.0);
+    return;
+  }
+  const double r = src_2kz[bs] / (2.0 * klm[(long long)b * n + o]);
+  double2 v = ax[bs * n + i];
+  v.x = r * v.x + (i == o ? 1.0 - r : 0.0);
+  v.y = r * v.y;
+  ax[bs * n + i] = v;
 }
 
 // ---------------------------------------------------------------- workspace
@@ -586,17 +954,12 @@ struct Gemm {
                  long long lda, long long sa, const double2* b, long long ldb, long long sb,
                  cplx beta, double2* c, long long ldc, long long sc, cplx diag, int batch,
                  const int* steps = nullptr, int step = 0, int reuse = 0,
-                 const double2* cin = nullptr) const {
+                 const GemmTerms& terms = GemmTerms{}) const {
     if (precision == EUV_PREC_MIXED)
       return gemm_mixed(m, n, k, alpha, scale, a, lda, sa, b, ldb, sb, beta, c, ldc, sc, diag,
-                        batch, steps, step, mwork, mbytes, status, stream, reuse, cin);
-    if (cin != nullptr && cin != c) {
-      // FP64 GEMM: the beta term reads C, so C = Cin first (same shape)
-      const size_t span = (size_t)(batch - 1) * sc + (size_t)(n - 1) * ldc + m;
-      EUV_CUDA_TRY(cudaMemcpyAsync(c, cin, span * sizeof(double2), cudaMemcpyDeviceToDevice, stream));
-    }
+                        batch, steps, step, mwork, mbytes, status, stream, reuse, terms);
     return zgemm(m, n, k, alpha, scale, a, lda, sa, b, ldb, sb, beta, c, ldc, sc, diag, batch,
-                 steps, step, stream);
+                 steps, step, stream, terms);
   }
 };
 
@@ -661,39 +1024,24 @@ int matfun(int n, int batch, const double2* D, const double* thick, double2** pc
   return EUV_OK;
 }
 
-// Upper bound of max_b ||D_b||_1 from the config (Parseval: the window sum of
-// |F| is at most sqrt(window size)); used to bound the double-angle steps.
-static int derive_m_max(const euv_amp_desc* d) {
-  const double theta = theta_for(d->precision);
-  const double k = d->k;
-  const int lr2 = 4 * d->lmax + 1, mr2 = 4 * d->mmax + 1;
-  const double S = sqrt((double)lr2 * (double)mr2);
+// Launch shape of a slice's polynomials: q of the slab, and the blocks and
+// double-angle steps of the widest ellipse any unit of the descriptor can have
+// (smallest period, incidence up to k0_max on both axes).
+static PolyPlan poly_plan(const euv_amp_desc* d, int slice, double tol) {
   const double twopi = 6.283185307179586476925286766559;
-  // largest |kx|, |ky| over orders and families (family offsets < 2 pi/dx)
-  const double k0 = d->k0_max > 0 ? d->k0_max : k;
-  double kxm = twopi * (2 * d->lmax + 2) / d->dx + k0;
-  double kym = twopi * (2 * d->mmax + 2) / d->dy + k0;
-  int mm = 0;
-  for (int n = 0; n < d->n_slices; ++n) {
-    double er = d->eabs[n].re - 1.0, ei = d->eabs[n].im;
-    double ae = sqrt(er * er + ei * ei);
-    double lr = 0.5 * log(d->eabs[n].re * d->eabs[n].re + d->eabs[n].im * d->eabs[n].im);
-    double li = atan2(d->eabs[n].im, d->eabs[n].re);
-    double al = sqrt(lr * lr + li * li);
-    double etam = twopi * 2.0 * (d->lmax > d->mmax ? d->lmax : d->mmax) /
-                  (d->dx < d->dy ? d->dx : d->dy) * al;
-    double bound = 1.4142135623730951 *
-                   (k * k * (1.0 + ae * S) + etam * (kxm > kym ? kxm : kym) * S +
-                    kxm * kxm + kym * kym);
-    double v = bound * d->dabs[n] * d->dabs[n];
-    int m = 0;
-    while (v > theta && m < kMaxSteps) {
-      v *= 0.25;
-      ++m;
-    }
-    if (m > mm) mm = m;
-  }
-  return mm;
+  const double gx = twopi / d->dx, gy = twopi / d->dy;
+  const double k0 = d->k0_max > 0 ? d->k0_max : d->k;
+  const double kx = k0 + gx * d->lmax, ky = k0 + gy * d->mmax;
+  const cplx e = mk(d->eabs[slice].re, d->eabs[slice].im), em1 = e - mk(1.0, 0.0);
+  const double leps = hypot(0.5 * log(e.x * e.x + e.y * e.y), atan2(e.y, e.x));
+  const double wx = gx * d->lmax * kx, wy = gy * d->mmax * ky;
+  const PolyRegion g = poly_region(d->k, em1, 0.0, kx * kx + ky * ky, leps * (wx > wy ? wx : wy));
+  PolyPlan r;
+  poly_shape(d->precision, d->k, em1, d->dabs[slice], &r.q, &r.jcap);
+  const int limit = d->m_max > 0 && d->m_max < kMaxSteps ? d->m_max : kMaxSteps;
+  poly_pick(g, d->dabs[slice], tol, r.q, r.jcap, limit, &r.j, &r.m);
+  if (r.m > 0) r.j = r.jcap;  // a unit that needs fewer steps may need all the blocks
+  return r;
 }
 
 // Factors of the Euler product for (I - E)^-1, E = diag(kp/k) Sigma diag(kp/k).
@@ -725,53 +1073,37 @@ static int euler_factors(const euv_amp_desc* d) {
   return f;
 }
 
-struct AmpLayout {
-  size_t bytes;
-};
-
 // All workspace carving in one place so the size query and the run agree.
 struct AmpWork {
-  double2 *D, *G, *P2, *P3, *P4, *T1, *C, *S, *X, *Y, *Z, *W, *Gp;
-  double2 *x2, *y2, *gx2, *E, *YZ;
-  double *klm, *norm, *h, *h2, *h4, *thick;
+  double2 *pw, *pair[3];  // per unit: 6 powers, three pairs of N^2 matrices
+  double2 *adm, *V2, *W2, *coef, *ident, *shift;
+  double *klm, *radius;
   int *steps, *ipiv, *info, *capped;
   void* mwork;
   size_t mbytes;
 };
 
 static bool carve(const euv_amp_desc* d, Bump& bp, AmpWork& w) {
-  const long long N = d->n_orders, U = d->n_units, nn = N * N;
-  w.D = bp.take<double2>(U * nn);
-  w.G = bp.take<double2>(U * nn);
-  w.P2 = bp.take<double2>(U * nn);
-  w.P3 = bp.take<double2>(U * nn);
-  w.P4 = bp.take<double2>(U * nn);
-  w.T1 = bp.take<double2>(U * nn);
-  w.C = bp.take<double2>(U * nn);
-  w.S = bp.take<double2>(U * nn);
-  w.X = bp.take<double2>(U * nn);
-  w.Y = bp.take<double2>(U * nn);
-  w.Z = bp.take<double2>(U * nn);
-  w.W = bp.take<double2>(U * nn);
-  w.Gp = d->refresh_sigma ? bp.take<double2>(U * nn) : nullptr;
-  w.x2 = bp.take<double2>(U * N);
-  w.y2 = bp.take<double2>(U * N);
-  w.gx2 = bp.take<double2>(U * N);
-  w.E = bp.take<double2>(U * N * (d->n_src > 0 ? d->n_src : 1));
-  w.YZ = bp.take<double2>(U * N * (d->n_src > 0 ? d->n_src : 1));
+  const long long N = d->n_orders, U = d->n_units, nn = N * N, NS = d->n_slices;
+  const long long cols = U * N * (d->n_src > 0 ? d->n_src : 1);
+  w.pw = bp.take<double2>(6 * U * nn);
+  for (int i = 0; i < 3; ++i) w.pair[i] = bp.take<double2>(2 * U * nn);
+  w.adm = bp.take<double2>(U * N);
+  w.V2 = bp.take<double2>(cols);
+  w.W2 = bp.take<double2>(cols);
+  w.coef = bp.take<double2>(NS * U * 2 * PF_J * PF_Q);
+  w.ident = bp.take<double2>(NS * U * 2 * (kMaxSteps + 1));
+  w.shift = bp.take<double2>(NS * U);
   w.klm = bp.take<double>(U * N);
-  w.norm = bp.take<double>(U);
-  w.h = bp.take<double>(U);
-  w.h2 = bp.take<double>(U);
-  w.h4 = bp.take<double>(U);
-  w.thick = bp.take<double>(U * (d->n_slices > 0 ? d->n_slices : 1));
-  w.steps = bp.take<int>(U);
+  w.radius = bp.take<double>(NS * U);
+  w.steps = bp.take<int>(NS * U);
   w.ipiv = bp.take<int>(U * N);
   w.info = bp.take<int>(U);
   w.capped = bp.take<int>(1);
-  // the mixed products are N x N x N, and N x n_src x N for the interface (n_src may exceed N)
-  const int ncol = d->n_src > N ? d->n_src : (int)N;
-  w.mbytes = d->precision == EUV_PREC_MIXED ? gemm_mixed_workspace_bytes((int)N, ncol, (int)N, (int)U) : 0;
+  // the mixed products are N x N x N, N x 2N x N for the two functions together,
+  // and N x n_src x N for the source columns
+  const long long ncol = d->n_src > 2 * N ? d->n_src : 2 * N;
+  w.mbytes = d->precision == EUV_PREC_MIXED ? gemm_mixed_workspace_bytes((int)N, (int)ncol, (int)N, (int)U) : 0;
   w.mwork = w.mbytes ? bp.take<char>(w.mbytes) : nullptr;
   return bp.ok;
 }
@@ -834,11 +1166,8 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
   const int N = d->n_orders, U = d->n_units, NS = d->n_slices;
   const long long nn = (long long)N * N;
   const int bs = 256;
-  const dim3 ge(grid1(nn, bs), U);
   const dim3 gdg((unsigned)N, (unsigned)((N + bs - 1) / bs), U);  // build_dg: column, rows, unit
-  const cplx one = mk(1.0, 0.0), zero = mk(0.0, 0.0), mi = mk(0.0, -1.0);
-  int m_max = d->m_max > 0 ? d->m_max : derive_m_max(d);
-  if (m_max > kMaxSteps) m_max = kMaxSteps;
+  const cplx one = mk(1.0, 0.0), zero = mk(0.0, 0.0);
   // device-detected conditions go to the caller's status word, else to a
   // workspace word nobody reads
   int* status = d->d_status ? d->d_status : w.capped;
@@ -846,12 +1175,6 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
   int rc;
 
   if (!d->d_status) EUV_CUDA_TRY(cudaMemsetAsync(w.capped, 0, sizeof(int), stream));
-  // per-slice thickness arrays [slice][unit]
-  for (int n = 0; n < NS; ++n) {
-    fill_f64_kernel<<<grid1(U, 256), 256, 0, stream>>>(w.thick + (size_t)n * U, U, d->dabs[n]);
-    EUV_LAUNCH_CHECK();
-  }
-
   SliceParams sp;
   sp.k = d->k;
   sp.dx = d->dx;
@@ -895,169 +1218,245 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
   stp.dys = d->d_dy;
   stp.n = N;
   multilayer_kernel<<<grid1((long long)N * U, 128), 128, 0, stream>>>(
-      stp, d->d_lindex, d->d_mindex, d->d_kx0, d->d_ky0, d->d_polar, w.x2, w.y2, w.gx2, w.klm, U);
+      stp, d->d_lindex, d->d_mindex, d->d_kx0, d->d_ky0, d->d_polar, w.adm, w.klm, U);
   EUV_LAUNCH_CHECK();
 
   const double2* spec = reinterpret_cast<const double2*>(d_spectra);
-  MatfunBufs mb{w.P2, w.P3, w.P4, w.T1, w.W, w.norm, w.h, w.h2, w.h4, w.steps, status};
+  // polynomial shapes of the slices, and the units' coefficients in one launch
+  PolySlices ps;
+  ps.k = d->k;
+  ps.dx = d->dx;
+  ps.dy = d->dy;
+  ps.dxs = d->d_dx;
+  ps.dys = d->d_dy;
+  ps.n = N;
+  ps.lmax = d->lmax;
+  ps.mmax = d->mmax;
+  ps.n_slices = NS;
+  ps.n_units = U;
+  ps.tol = d->precision == EUV_PREC_MIXED ? kPolyTolMixed : kPolyTolFp64;
+  for (int n = 0; n < NS; ++n) {
+    const PolyPlan r = poly_plan(d, n, ps.tol);
+    const SliceParams q = slice_params(n);
+    ps.eps_m1[n] = q.eps_m1;
+    ps.leps[n] = cabs(q.logeps);
+    ps.d[n] = d->dabs[n];
+    ps.q[n] = r.q;
+    ps.jcap[n] = r.jcap;
+    ps.j[n] = r.j;
+    ps.m[n] = r.m;
+  }
+  poly_coef_kernel<<<dim3(U, NS), PF_SAMPLES, 0, stream>>>(ps, d->d_lindex, d->d_mindex, d->d_kx0,
+                                                           d->d_ky0, d->d_polar, w.coef, w.ident, w.shift,
+                                                           w.radius, w.steps, status);
+  EUV_LAUNCH_CHECK();
+
   // Mixed form: G^-1 by the Euler product (I - E)^-1 = prod_f (I + E^(2^f)),
   // f < euler_f, when the config bound on ||E||_2 makes it converge fast.
   const int euler_f = d->precision != EUV_PREC_MIXED ? 0
                       : d->euler_f > 0                ? d->euler_f
                       : d->euler_f < 0                ? 0
                                                       : euler_factors(d);
-  // factors f = 1..euler_f-1 applied to the partial product held in Zbuf (the
-  // f = 0 factor is applied by the caller); E^(2^f) ping-pongs between G and P2
-  // g_split: the caller's last GEMM had G as its A operand
-  auto euler_tail = [&](double2* Zbuf, bool g_split) -> int {
-    double2* P = w.G;
-    double2* Pn = w.P2;
-    double2* Zc = Zbuf;
-    double2* Zt = w.W;
-    for (int f = 1; f < euler_f; ++f) {
-      // P as A again: split by the previous factor's P Zc (or the caller's G Z)
-      const int ru = (f > 1 || g_split) ? kReuseA : 0;
-      int r2 = gemm(N, N, N, one, nullptr, P, N, nn, P, N, nn, zero, Pn, N, nn, zero, U, nullptr, 0,
-                    ru);
-      if (r2) return r2;
-      double2* t = P;
-      P = Pn;
-      Pn = t;
-      // Zt = P Zc + Zc (the beta term read from Zc)
-      r2 = gemm(N, N, N, one, nullptr, P, N, nn, Zc, N, nn, one, Zt, N, nn, zero, U, nullptr, 0, 0,
-                Zc);
-      if (r2) return r2;
-      t = Zc;
-      Zc = Zt;
-      Zt = t;
-    }
-    if (Zc != Zbuf)
-      EUV_CUDA_TRY(cudaMemcpyAsync(Zbuf, Zc, (size_t)U * nn * sizeof(double2), cudaMemcpyDeviceToDevice, stream));
+  // a batch of N-row matrices: first element and batch stride
+  struct Mat {
+    double2* p;
+    long long s;
+  };
+  // powers of E side by side per unit; pairs: [c | s], its other buffer, [P | Q]
+  Mat pw[6], cs[2] = {{w.pair[0], 2 * nn}, {w.pair[1], 2 * nn}}, pq = {w.pair[2], 2 * nn};
+  for (int i = 0; i < 6; ++i) pw[i] = Mat{w.pw + i * nn, 6 * nn};
+  auto build = [&](int slice, const Mat* E, const Mat* G, int want_g) -> int {
+    build_dg_kernel<<<gdg, bs, 0, stream>>>(
+        slice_params(slice), spec, d->d_spec, d->d_lindex, d->d_mindex, d->d_kx0, d->d_ky0,
+        d->d_polar, w.adm, w.shift + (size_t)slice * U, w.radius + (size_t)slice * U,
+        E ? E->p : nullptr, E ? E->s : 0, G ? G->p : nullptr, G ? G->s : 0, want_g);
+    EUV_LAUNCH_CHECK();
     return EUV_OK;
   };
-  double2* X = w.X;
-  double2* Y = w.Y;
+  // C = alpha scale A B + beta Cin (C itself unless given) + ..., N x n x N
+  struct Term {
+    const Mat* cin = nullptr;
+    const double2* beta_b = nullptr;
+    const Mat* cin2 = nullptr;
+    const double2* beta2_b = nullptr;
+    cplx beta2 = mk(1.0, 0.0);
+  };
+  auto mul = [&](cplx alpha, const double* scale, const Mat& A, const Mat& B, cplx beta,
+                 const Mat& C, int reuse, const Term& x = Term{}, int n = 0) -> int {
+    GemmTerms t;
+    t.cin = x.cin ? x.cin->p : C.p;
+    t.scin = x.cin ? x.cin->s : C.s;
+    t.beta_b = x.beta_b;
+    t.cin2 = x.cin2 ? x.cin2->p : nullptr;
+    t.scin2 = x.cin2 ? x.cin2->s : 0;
+    t.beta2 = make_double2(x.beta2.x, x.beta2.y);
+    t.beta2_b = x.beta2_b;
+    return gemm(N, n > 0 ? n : N, N, alpha, scale, A.p, N, A.s, B.p, N, B.s, beta, C.p, N, C.s,
+                zero, U, nullptr, 0, reuse, t);
+  };
+  auto swap = [](Mat& a, Mat& b) {
+    const Mat t = a;
+    a = b;
+    b = t;
+  };
+  // c - c0 and s - s0 of slice n, side by side per unit, in cs[0] on return; E in pw[0]
+  auto slab = [&](int n) -> int {
+    const int q = ps.q[n], J = ps.j[n], m = ps.m[n];
+    int r2;
+    // E^2; [E^3 | E^4] = E^2 [E | E^2]; [E^5 | E^6] = E^2 [E^3 | E^4]
+    if ((r2 = mul(one, nullptr, pw[0], pw[0], zero, pw[1], 0))) return r2;
+    if ((r2 = mul(one, nullptr, pw[1], pw[0], zero, pw[2], 0, Term{}, q > 3 ? 2 * N : N)))
+      return r2;
+    if (q > 4 && (r2 = mul(one, nullptr, pw[1], pw[2], zero, pw[4], kReuseA, Term{},
+                           q > 5 ? 2 * N : N)))
+      return r2;
+    const double2* pb = pw[0].p;
+    if (J > 1) {
+      if ((r2 = poly_blocks<2>(q, N, pb, 6 * nn, w.coef, U, n, J - 1, cs[0].p, cs[1].p, 2 * nn, stream)))
+        return r2;
+    } else if ((r2 = poly_blocks<1>(q, N, pb, 6 * nn, w.coef, U, n, 0, cs[0].p, nullptr, 2 * nn, stream))) {
+      return r2;
+    }
+    for (int b = J - 2; b >= 0; --b) {
+      if (b < J - 2 &&
+          (r2 = poly_blocks<1>(q, N, pb, 6 * nn, w.coef, U, n, b, cs[1].p, nullptr, 2 * nn, stream)))
+        return r2;
+      if ((r2 = mul(one, nullptr, pw[q - 1], cs[0], one, cs[1], b < J - 2 ? kReuseA : 0, Term{},
+                    2 * N)))
+        return r2;
+      swap(cs[0], cs[1]);
+    }
+    // double-angle steps s <- 2 s c, c <- 2 c^2 - I on the parts beside the
+    // identity: S <- 2 S C + 2 c0 S + 2 s0 C, C <- 2 C C + 4 c0 C; units with
+    // fewer steps copy through
+    const int* st = w.steps + (size_t)n * U;
+    for (int step = 0; step < m; ++step) {
+      const double2 *c = cs[0].p, *s = cs[0].p + nn;
+      GemmTerms t;
+      t.cin = s;
+      t.scin = t.scin2 = 2 * nn;
+      t.beta_b = w.ident + poly_id_at(U, n, step, 0);
+      t.cin2 = c;
+      t.beta2 = make_double2(2.0, 0.0);
+      t.beta2_b = w.ident + poly_id_at(U, n, step, 1);
+      if ((r2 = gemm(N, N, N, mk(2.0, 0.0), nullptr, s, N, 2 * nn, c, N, 2 * nn, mk(2.0, 0.0),
+                     cs[1].p + nn, N, 2 * nn, zero, U, st, step, 0, t)))
+        return r2;
+      t.cin = c;
+      t.cin2 = nullptr;
+      if ((r2 = gemm(N, N, N, mk(2.0, 0.0), nullptr, c, N, 2 * nn, c, N, 2 * nn, mk(4.0, 0.0),
+                     cs[1].p, N, 2 * nn, zero, U, st, step, kReuseB, t)))  // c as B again
+        return r2;
+      swap(cs[0], cs[1]);
+    }
+    return EUV_OK;
+  };
+  // The boundary relation P X + Q Y = 0 of the fields at the top of the slices
+  // done so far, carried upwards (rows combine, so no interface matrix is
+  // inverted): at the cap Y2 = diag(adm) G X2, i.e. P = -diag(adm) G, Q = I;
+  // through a slice X2 = c X1 + i s Y1, Y2 = i D s X1 + c Y1, so
+  //   P <- P c + i Q D s,   Q <- Q c + i P s,   D = a + R E.
+  const cplx pi_ = mk(0.0, 1.0), m1 = mk(-1.0, 0.0);
   for (int n = NS - 1; n >= 0; --n) {
-    SliceParams q = slice_params(n);
-    const bool bottom = (n == NS - 1);
-    const bool need_g = bottom || d->refresh_sigma;
+    const bool bottom = (n == NS - 1), top = (n == 0);
+    const Mat P = pq, Q{pq.p + nn, 2 * nn};
+    if (!bottom && d->refresh_sigma) {
+      // the slices' own 1/eps: X of slice n+1 is G_{n+1}^-1 G_n times X of slice
+      // n, so P <- P G_{n+1}^-1 G_n
+      Mat E = pw[0], En = pw[1], cur = P;
+      if (euler_f > 0) {
+        // P (I + E)(I + E^2)(I + E^4)... (I - E_n): both G are i k (I - E)
+        if ((rc = build(n + 1, nullptr, &E, 2))) return rc;
+        for (int f = 0; f < euler_f; ++f) {
+          const Mat dst = pw[2 + (f & 1)];
+          if ((rc = mul(one, nullptr, cur, E, one, dst, 0, Term{&cur}))) return rc;
+          cur = dst;
+          if (f + 1 < euler_f) {
+            if ((rc = mul(one, nullptr, E, E, zero, En, kReuseB))) return rc;  // E as B again
+            swap(E, En);
+          }
+        }
+        if ((rc = build(n, nullptr, &En, 2))) return rc;
+        if ((rc = mul(m1, nullptr, cur, En, one, P, 0, Term{&cur}))) return rc;
+      } else {
+        if ((rc = build(n + 1, nullptr, &E, 1))) return rc;
+        if ((rc = build(n, nullptr, &En, 1))) return rc;
+        if ((rc = lu_factor(N, E.p, N, E.s, w.ipiv, w.info, U, stream))) return rc;
+        flag_singular_kernel<<<grid1(U, 256), 256, 0, stream>>>(w.info, U, status);
+        EUV_LAUNCH_CHECK();
+        if ((rc = lu_solve(N, N, E.p, N, E.s, w.ipiv, En.p, N, En.s, U, stream))) return rc;
+        if ((rc = mul(one, nullptr, P, En, zero, pw[2], 0))) return rc;
+        EUV_CUDA_TRY(cudaMemcpy2DAsync(P.p, P.s * sizeof(double2), pw[2].p, pw[2].s * sizeof(double2),
+                                       nn * sizeof(double2), U, cudaMemcpyDeviceToDevice, stream));
+      }
+    }
     // bottom slice sigma is used for every slice unless refresh_sigma (header.h:1327-1353)
-    build_dg_kernel<<<gdg, bs, 0, stream>>>(q, spec, d->d_spec, d->d_lindex, d->d_mindex, d->d_kx0,
-                                           d->d_ky0, d->d_polar, w.D, w.G, 1,
-                                           need_g ? (euler_f > 0 ? 2 : 1) : 0);
-    EUV_LAUNCH_CHECK();
-    double2* Zp = X;
-    if (bottom && euler_f > 0) {
-      // mixed form: Z = G^-1 diag(gx2) = (1/ik) (I - E)^-1 diag(gx2) by the Euler
-      // product on the tensor cores (E was built in place of G)
-      euler_first_diag_kernel<<<ge, bs, 0, stream>>>(N, cdiv(one, mk(0.0, d->k)), w.G, w.gx2, w.Z);
+    if ((rc = build(n, &pw[0], bottom ? &P : nullptr, bottom ? 3 : 0))) return rc;
+    if ((rc = slab(n))) return rc;
+    const Mat C = cs[0], S{cs[0].p + nn, 2 * nn}, E = pw[0];
+    const double* rad = w.radius + (size_t)n * U;
+    const double2* ia = w.shift + (size_t)n * U;
+    // c = c0 + C, s = s0 + S, D = a + R E
+    const double2* c0 = w.ident + poly_id_at(U, n, ps.m[n], 0);
+    const double2* s0 = w.ident + poly_id_at(U, n, ps.m[n], 1);
+    if (top) {
+      // Top interface: X1 = b + e, Y1 = klm (e - b) for incident e and reflected
+      // b (header.h:1355-1465), so M b = rhs e with
+      //   M = P (c - i s klm) + Q (i D s - c klm),
+      //   rhs = -(P (c + i s klm) + Q (i D s + c klm)).
+      const int ns = d->n_src;
+      const Mat V = pw[1], W = pw[2], M = pw[3];  // the powers above E are free now
+      const long long sn = (long long)N * ns;
+      const Mat V2{w.V2, sn}, W2{w.W2, sn}, ax{reinterpret_cast<double2*>(d_ax), sn};
+      const double2* Qp = bottom ? nullptr : Q.p;
+      if ((rc = mul(pi_, rad, E, S, zero, W, 0))) return rc;
+      top_rows_kernel<<<gdg, bs, 0, stream>>>(N, w.klm, ia, rad, c0, s0, C.p, S.p, C.s, E.p, V.p,
+                                              W.p, M.p, E.s, P.p, Qp, P.s);
       EUV_LAUNCH_CHECK();
-      if ((rc = euler_tail(w.Z, false))) return rc;
-      Zp = w.Z;
-    } else if (bottom) {
-      // Z = G^-1 diag(Bru (URUU+URUB))
-      diag_kernel<<<ge, bs, 0, stream>>>(N, w.gx2, w.Z);
-      EUV_LAUNCH_CHECK();
-      if ((rc = lu_factor(N, w.G, N, nn, w.ipiv, w.info, U, stream))) return rc;
+      const dim3 gs((unsigned)ns, (unsigned)((N + bs - 1) / bs), U);
+      if (ns > 0) {
+        source_rows_kernel<<<gs, bs, 0, stream>>>(N, ns, d->d_src_order, w.klm, ia, c0, s0, C.p, S.p,
+                                                  C.s, V.p, W.p, V.s, P.p, Qp, P.s, V2.p, W2.p,
+                                                  ax.p);
+        EUV_LAUNCH_CHECK();
+      }
+      if ((rc = mul(one, nullptr, P, V, one, M, 0))) return rc;
+      if (ns > 0 && (rc = mul(m1, nullptr, P, V2, one, ax, kReuseA, Term{}, ns))) return rc;
+      if (!bottom) {
+        if ((rc = mul(one, nullptr, Q, W, one, M, 0))) return rc;
+        if (ns > 0 && (rc = mul(m1, nullptr, Q, W2, one, ax, kReuseA, Term{}, ns))) return rc;
+      }
+      if ((rc = lu_factor(N, M.p, N, M.s, w.ipiv, w.info, U, stream))) return rc;
       flag_singular_kernel<<<grid1(U, 256), 256, 0, stream>>>(w.info, U, status);
       EUV_LAUNCH_CHECK();
-      if ((rc = lu_solve(N, N, w.G, N, nn, w.ipiv, w.Z, N, nn, U, stream))) return rc;
-      Zp = w.Z;
-    } else if (d->refresh_sigma && euler_f > 0) {
-      // Z = (I - E_n)^-1 (I - E_{n+1}) X  (= G_n^-1 G_{n+1} X)
-      SliceParams qp = slice_params(n + 1);
-      build_dg_kernel<<<gdg, bs, 0, stream>>>(qp, spec, d->d_spec, d->d_lindex, d->d_mindex,
-                                             d->d_kx0, d->d_ky0, d->d_polar, nullptr, w.Gp, 0, 2);
-      EUV_LAUNCH_CHECK();
-      if ((rc = gemm(N, N, N, mk(-1.0, 0.0), nullptr, w.Gp, N, nn, X, N, nn, one, w.Z, N, nn, zero,
-                     U, nullptr, 0, 0, X))) return rc;  // Z = X - Gp X
-      if ((rc = gemm(N, N, N, one, nullptr, w.G, N, nn, w.Z, N, nn, one, w.W, N, nn, zero, U,
-                     nullptr, 0, 0, w.Z))) return rc;  // W = Z + G Z
-      EUV_CUDA_TRY(cudaMemcpyAsync(w.Z, w.W, (size_t)U * nn * sizeof(double2), cudaMemcpyDeviceToDevice, stream));
-      if ((rc = euler_tail(w.Z, true))) return rc;
-      Zp = w.Z;
-    } else if (d->refresh_sigma) {
-      // Z = G_n^-1 G_{n+1} X
-      SliceParams qp = slice_params(n + 1);
-      build_dg_kernel<<<gdg, bs, 0, stream>>>(qp, spec, d->d_spec, d->d_lindex, d->d_mindex,
-                                             d->d_kx0, d->d_ky0, d->d_polar, nullptr, w.Gp, 0, 1);
-      EUV_LAUNCH_CHECK();
-      if ((rc = gemm(N, N, N, one, nullptr, w.Gp, N, nn, X, N, nn, zero, w.Z, N, nn, zero, U))) return rc;
-      if ((rc = lu_factor(N, w.G, N, nn, w.ipiv, w.info, U, stream))) return rc;
-      flag_singular_kernel<<<grid1(U, 256), 256, 0, stream>>>(w.info, U, status);
-      EUV_LAUNCH_CHECK();
-      if ((rc = lu_solve(N, N, w.G, N, nn, w.ipiv, w.Z, N, nn, U, stream))) return rc;
-      Zp = w.Z;
+      if (ns > 0) {
+        // empty source slots (order < 0, zero columns) skip their CTAs
+        if ((rc = lu_solve(N, ns, M.p, N, M.s, w.ipiv, ax.p, N, sn, U, stream, d->d_src_order, ns)))
+          return rc;
+        ax_out_kernel<<<gs, bs, 0, stream>>>(N, ns, d->d_src_order, d->d_src_2kz, w.klm, ax.p);
+        EUV_LAUNCH_CHECK();
+      }
+      return EUV_OK;
     }
-    double2* C = w.C;
-    double2* S = w.S;
-    if ((rc = matfun(N, U, w.D, w.thick + (size_t)n * U, &C, &S, mb, m_max, gemm, stream))) return rc;
-    // buffers free after matfun: P2, P3, P4, T1, W minus the two now holding C/S
-    double2* pool[7] = {w.P2, w.P3, w.P4, w.T1, w.W, w.C, w.S};
-    double2* fr[5];
-    int nf = 0;
-    for (int i = 0; i < 7; ++i)
-      if (pool[i] != C && pool[i] != S && pool[i] != Zp) fr[nf++] = pool[i];
-    double2* Wb = fr[0];
-    double2* Xn = fr[1];
-    double2* Yn = fr[2];
-    // W = S Z ; Xn = C Z - i S Y ; Yn = -i D W + C Y, ordered so that three of
-    // the five products find one operand already split
-    if ((rc = gemm(N, N, N, one, nullptr, S, N, nn, Zp, N, nn, zero, Wb, N, nn, zero, U))) return rc;
-    if ((rc = gemm(N, N, N, one, nullptr, C, N, nn, Zp, N, nn, zero, Xn, N, nn, zero, U, nullptr, 0,
-                   kReuseB))) return rc;  // Zp as B again
+    const Mat R1 = cs[1], R2{cs[1].p + nn, 2 * nn};
     if (bottom) {
-      if ((rc = gemm(N, N, N, mi, nullptr, w.D, N, nn, Wb, N, nn, zero, Yn, N, nn, zero, U))) return rc;
-      colscale_kernel<<<ge, bs, 0, stream>>>(N, mi, S, w.y2, one, Xn);
+      // Q = I: R1 = P c + i D s, R2 = c + i P s
+      bottom_rows_kernel<<<gdg, bs, 0, stream>>>(N, ia, rad, c0, s0, C.p, S.p, C.s, E.p, E.s, P.p,
+                                                 P.s, R1.p, R2.p, R1.s);
       EUV_LAUNCH_CHECK();
-      colscale_kernel<<<ge, bs, 0, stream>>>(N, one, C, w.y2, one, Yn);
-      EUV_LAUNCH_CHECK();
+      if ((rc = mul(pi_, rad, E, S, one, R1, 0))) return rc;
+      if ((rc = mul(pi_, nullptr, P, S, one, R2, kReuseB))) return rc;  // S as B again
+      if ((rc = mul(one, nullptr, P, C, one, R1, kReuseA))) return rc;  // P as A again
     } else {
-      if ((rc = gemm(N, N, N, one, nullptr, C, N, nn, Y, N, nn, zero, Yn, N, nn, zero, U, nullptr,
-                     0, kReuseA))) return rc;  // C as A again
-      if ((rc = gemm(N, N, N, mi, nullptr, S, N, nn, Y, N, nn, one, Xn, N, nn, zero, U, nullptr, 0,
-                     kReuseB))) return rc;  // Y as B again
-      if ((rc = gemm(N, N, N, mi, nullptr, w.D, N, nn, Wb, N, nn, one, Yn, N, nn, zero, U))) return rc;
+      // T = Q s, R2 = Q c + i P s, R1 = P c + i T D
+      const Mat T = pw[1];
+      if ((rc = mul(one, nullptr, Q, S, one, T, 0, Term{&Q, s0}))) return rc;
+      if ((rc = mul(one, nullptr, Q, C, one, R2, kReuseA, Term{&Q, c0, &P, s0, pi_}))) return rc;
+      if ((rc = mul(one, nullptr, P, C, one, R1, kReuseB, Term{&P, c0, &T, ia}))) return rc;
+      if ((rc = mul(pi_, nullptr, P, S, one, R2, kReuseA))) return rc;  // P as A again
+      if ((rc = mul(pi_, rad, T, E, one, R1, 0))) return rc;
     }
-    if (n == 0) {
-      // top slice: the interface below reads Xn, Yn where they are (nothing
-      // after the loop writes the matrix-function buffers)
-      X = Xn;
-      Y = Yn;
-      break;
-    }
-    // move the new X, Y into the dedicated buffers for the next slice's matfun
-    EUV_CUDA_TRY(cudaMemcpyAsync(w.X, Xn, (size_t)U * nn * sizeof(double2),
-                                 cudaMemcpyDeviceToDevice, stream));
-    EUV_CUDA_TRY(cudaMemcpyAsync(w.Y, Yn, (size_t)U * nn * sizeof(double2),
-                                 cudaMemcpyDeviceToDevice, stream));
-    X = w.X;
-    Y = w.Y;
-  }
-  // top interface: U0 = klm X + Y, Z = U0^-1 E, Ax = -(1/klm) Y Z + e
-  u0_kernel<<<ge, bs, 0, stream>>>(N, w.klm, X, Y, w.G);
-  EUV_LAUNCH_CHECK();
-  if ((rc = lu_factor(N, w.G, N, nn, w.ipiv, w.info, U, stream))) return rc;
-  flag_singular_kernel<<<grid1(U, 256), 256, 0, stream>>>(w.info, U, status);
-  EUV_LAUNCH_CHECK();
-  const int ns = d->n_src;
-  if (ns > 0) {
-    dim3 gs(grid1((long long)N * ns, bs), U);
-    src_rhs_kernel<<<gs, bs, 0, stream>>>(N, ns, d->d_src_order, d->d_src_2kz, w.E);
-    EUV_LAUNCH_CHECK();
-    // empty source slots (order < 0, zero columns of E) skip their CTAs
-    if ((rc = lu_solve(N, ns, w.G, N, nn, w.ipiv, w.E, N, (long long)N * ns, U, stream,
-                       d->d_src_order, ns)))
-      return rc;
-    // Y Z for the source columns: a product, so the mixed form takes it on the
-    // tensor cores (split-FP16x3, ~1e-6 relative) like the matrix functions; the
-    // solve above stays FP64
-    if ((rc = gemm(N, ns, N, one, nullptr, Y, N, nn, w.E, N, (long long)N * ns, zero, w.YZ, N,
-                   (long long)N * ns, zero, U)))
-      return rc;
-    ax_out_kernel<<<gs, bs, 0, stream>>>(N, ns, d->d_src_order, w.klm, w.YZ,
-                                         reinterpret_cast<double2*>(d_ax));
-    EUV_LAUNCH_CHECK();
+    swap(pq, cs[1]);
   }
   return EUV_OK;
 }

@@ -32,6 +32,7 @@ struct GemmArgs {
   const double2* b;
   long long ldb, sb;
   double2* c;
+  GemmTerms t;
   long long ldc, sc;
   const int* steps;
   int step;
@@ -215,8 +216,14 @@ __global__ void __launch_bounds__(GTHREADS, MI == 2 ? 4 : 2) zgemm_kernel(GemmAr
 
   const double sc = p.scale ? p.scale[bz] : 1.0;
   const cplx alpha = mk(p.alpha.x * sc, p.alpha.y * sc);
-  const cplx beta = mk(p.beta.x, p.beta.y);
+  cplx beta = mk(p.beta.x, p.beta.y);
+  if (p.t.beta_b) beta = beta * mk(p.t.beta_b[bz].x, p.t.beta_b[bz].y);
   const bool use_beta = (p.beta.x != 0.0 || p.beta.y != 0.0);
+  const double2* Cin = p.t.cin ? p.t.cin + (long long)bz * p.t.scin : C;
+  const bool use_2 = p.t.cin2 != nullptr;
+  const double2* Cin2 = use_2 ? p.t.cin2 + (long long)bz * p.t.scin2 : C;
+  const cplx beta2 = use_2 ? mk(p.t.beta2.x, p.t.beta2.y) * mk(p.t.beta2_b[bz].x, p.t.beta2_b[bz].y)
+                           : mk(0.0, 0.0);
   const cplx dg = mk(p.diag.x, p.diag.y);
 #pragma unroll
   for (int mi = 0; mi < MI; ++mi) {
@@ -229,8 +236,12 @@ __global__ void __launch_bounds__(GTHREADS, MI == 2 ? 4 : 2) zgemm_kernel(GemmAr
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int col = n0 + wn + ni * 8 + (lane & 3) * 2 + e;
-        old[ni][e] = (use_beta && row < p.m && col < p.n) ? C[row + (long long)col * p.ldc]
-                                                          : make_double2(0.0, 0.0);
+        const bool in = row < p.m && col < p.n;
+        const long long at = row + (long long)col * p.ldc;
+        cplx o = mk(0.0, 0.0);
+        if (use_beta && in) o = beta * mk(Cin[at].x, Cin[at].y);
+        if (use_2 && in) o = o + beta2 * mk(Cin2[at].x, Cin2[at].y);
+        old[ni][e] = make_double2(o.x, o.y);
       }
 #pragma unroll
     for (int ni = 0; ni < 4; ++ni)
@@ -239,7 +250,7 @@ __global__ void __launch_bounds__(GTHREADS, MI == 2 ? 4 : 2) zgemm_kernel(GemmAr
         const int col = n0 + wn + ni * 8 + (lane & 3) * 2 + e;
         if (row < p.m && col < p.n) {
           cplx v = alpha * mk(accr[mi][ni][e], acci[mi][ni][e]);
-          if (use_beta) v = v + beta * mk(old[ni][e].x, old[ni][e].y);
+          v = v + mk(old[ni][e].x, old[ni][e].y);
           if (row == col) v = v + dg;
           C[row + (long long)col * p.ldc] = make_double2(v.x, v.y);
         }
@@ -306,7 +317,7 @@ int zgemm_sub(int m, int n, int k, const double2* a, long long lda, long long sa
 int zgemm(int m, int n, int k, cplx alpha, const double* scale, const double2* a, long long lda,
           long long sa, const double2* b, long long ldb, long long sb, cplx beta, double2* c,
           long long ldc, long long sc, cplx diag, int batch, const int* steps, int step,
-          cudaStream_t stream) {
+          cudaStream_t stream, const GemmTerms& terms) {
   GemmArgs p;
   p.m = m;
   p.n = n;
@@ -322,6 +333,7 @@ int zgemm(int m, int n, int k, cplx alpha, const double* scale, const double2* a
   p.ldb = ldb;
   p.sb = sb;
   p.c = c;
+  p.t = terms;
   p.ldc = ldc;
   p.sc = sc;
   p.steps = steps;
@@ -349,5 +361,5 @@ extern "C" int euv_zgemm(int m, int n, int k, euv_c64 alpha, const double* d_sca
   return euv::zgemm(m, n, k, euv::fromc(alpha), d_scale, reinterpret_cast<const double2*>(d_a),
                     lda, stride_a, reinterpret_cast<const double2*>(d_b), ldb, stride_b,
                     euv::fromc(beta), reinterpret_cast<double2*>(d_c), ldc, stride_c,
-                    euv::fromc(diag_add), batch, d_steps, step, (cudaStream_t)stream);
+                    euv::fromc(diag_add), batch, d_steps, step, (cudaStream_t)stream, euv::GemmTerms{});
 }

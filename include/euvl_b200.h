@@ -249,7 +249,9 @@ typedef struct {
   const int* d_src_order;  /* [U][n_src] order index of each source (-1: none) */
   const double* d_src_2kz; /* [U][n_src] 2*kz of each source (header.h:1401-1409) */
   int precision;         /* EUV_PREC_FP64 or EUV_PREC_MIXED */
-  int m_max;             /* upper bound on double-angle steps; <= 0: derived */
+  int m_max;             /* upper bound on double-angle steps; <= 0: derived.  The slab's
+                            polynomials take the spectra as those of an indicator with
+                            values in [0, 1] (euv_mask_spectrum) */
   double k0_max;         /* bound on |kx0|, |ky0| over the units (<= 0: k) */
   int* d_status;         /* optional device int: EUV_STATUS_* bits OR-ed in (NULL: none) */
   const double* d_dx;    /* optional [U] clip period of each unit (nm), so that clips of
