@@ -57,6 +57,9 @@ struct GemmTerms {
   long long scin2 = 0;
   double2 beta2 = {0.0, 0.0};
   const double2* beta2_b = nullptr;
+  // entries with need[b] <= need_above are left as they are (C untouched)
+  const int* need = nullptr;
+  int need_above = 0;
 };
 
 // exp(z) for complex z.

@@ -31,8 +31,8 @@
 //                4x(128x32) A + 4x(128x32) B fp16 = 64 KB);
 //   warp 1     : TMEM allocation (512 columns: four 128-column accumulators of
 //                a 128x128 tile) and the single-thread MMA issue loop;
-//   warps 2..5 : epilogue, tcgen05.ld of their 32 TMEM lanes (= rows), complex
-//                FP64 result written column by column (coalesced).
+//   warps 2..9 : epilogue, tcgen05.ld of 32 TMEM lanes (= rows) x 64 columns each,
+//                complex FP64 result written column by column (coalesced).
 // All waits are bounded (about 2 s); a timeout ORs EUV_STATUS_TIMEOUT into the
 // status word, drains the copies and MMAs in flight, frees TMEM and returns.
 #include <cuda_fp16.h>
@@ -54,9 +54,11 @@ constexpr int MX_PLANES = 4;
 constexpr int MX_A_TILE = MX_BM * MX_BK * 2;  // 8 KB
 constexpr int MX_B_TILE = MX_BN * MX_BK * 2;  // 8 KB
 constexpr int MX_STAGE_BYTES = MX_PLANES * (MX_A_TILE + MX_B_TILE);  // 64 KB
-constexpr int MX_THREADS = 192;
+constexpr int MX_EPI_WARPS = 8;
+constexpr int MX_THREADS = 64 + 32 * MX_EPI_WARPS;
 constexpr int MX_TMEM_COLS = 512;
-constexpr size_t MX_SMEM = (size_t)MX_STAGES * MX_STAGE_BYTES + 1024 + 256;
+constexpr int MX_COL_OFF = MX_STAGES * MX_STAGE_BYTES + 256;  // column factors, after the barriers
+constexpr size_t MX_SMEM = (size_t)MX_COL_OFF + MX_BN * sizeof(double) + 1024;
 constexpr unsigned long long MX_TIMEOUT_NS = 2000000000ull;
 // stage slot of each B plane (gmem order Re_hi, Re_lo, Im_hi, Im_lo)
 __device__ constexpr int kBSlot[4] = {0, 2, 1, 3};
@@ -144,6 +146,13 @@ struct KOrder {
   }
 };
 
+// NX: matrices the epilogue adds (0: none, 1: the beta term, 2: GemmTerms::cin2 too).
+// The epilogue cannot overlap the main loop (the four accumulators fill TMEM, the
+// stages shared memory, so an SM holds one CTA) and moves 256 KB per matrix and
+// tile: eight warps, the first chunk of the added matrices loaded and the rest
+// prefetched into L2 while the main loop runs, each later chunk's loads issued
+// one chunk ahead, scale factors as two numbers per element instead of an ldexp.
+template <int NX>
 __global__ void __launch_bounds__(MX_THREADS, 1)
     gemm_split3_kernel(const __grid_constant__ CUtensorMap tmA,
                        const __grid_constant__ CUtensorMap tmB, MixedArgs p) {
@@ -161,6 +170,7 @@ __global__ void __launch_bounds__(MX_THREADS, 1)
   const int m0 = blockIdx.x * MX_BM, n0 = blockIdx.y * MX_BN;
   double2* C = p.c + (long long)b * p.sc;
 
+  if (p.t.need != nullptr && p.t.need[b] <= p.t.need_above) return;
   if (p.steps != nullptr && p.step >= p.steps[b]) {
     // inactive double-angle step of this batch entry: C = A on this tile
     // (eight loads in flight per thread before their stores: the CTA holds a
@@ -304,66 +314,86 @@ __global__ void __launch_bounds__(MX_THREADS, 1)
       umma_commit(accum);  // always: the epilogue / teardown waits on it
     }
   } else {
-    // epilogue: warps 2..5 read TMEM lanes (warp % 4) * 32 .. +31 = tile rows
-    const int q = warp & 3;
+    // epilogue: warps 2..9; TMEM lanes (warp % 4) * 32 .. +31 = tile rows, two
+    // warps per lane quarter with 64 columns each
+    constexpr int EC = 8, NCH = MX_BN / 2 / EC;
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    const int cb = n0 + half * (MX_BN / 2);
+    const int row = m0 + q * 32 + lane;
+    const bool rok = row < p.m;
+    double* s_cf = reinterpret_cast<double*>(smem + MX_COL_OFF);
+    const double2* Cin = p.t.cin ? p.t.cin + (long long)b * p.t.scin : C;
+    const double2* Cin2 = NX == 2 ? p.t.cin2 + (long long)b * p.t.scin2 : C;
+    // undo the power-of-two scaling of the operands: 2^-(exponents of row and column)
+    if (threadIdx.x - 64 < MX_BN) {
+      const int col = n0 + (int)threadIdx.x - 64;
+      s_cf[threadIdx.x - 64] = col < p.n ? ldexp(1.0, -p.eb[(long long)b * p.n + col]) : 0.0;
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(32 * MX_EPI_WARPS) : "memory");
+    const double sc = (p.scale ? p.scale[b] : 1.0) *
+                      (rok ? ldexp(1.0, -p.ea[(long long)b * p.m + row]) : 0.0);
+    const cplx alpha = mk(p.alpha.x * sc, p.alpha.y * sc);
+    cplx beta = mk(p.beta.x, p.beta.y), beta2 = mk(0.0, 0.0);
+    if (NX >= 1 && p.t.beta_b) beta = beta * mk(p.t.beta_b[b].x, p.t.beta_b[b].y);
+    if (NX == 2) beta2 = mk(p.t.beta2.x, p.t.beta2.y) * mk(p.t.beta2_b[b].x, p.t.beta2_b[b].y);
+    const cplx dg = mk(p.diag.x, p.diag.y);
+    if (NX >= 1) {
+      // four lanes per column, one 128-byte line each
+#pragma unroll
+      for (int c = lane >> 2; c < MX_BN / 2; c += 8) {
+        const int r = m0 + q * 32 + (lane & 3) * 8, col = cb + c;
+        if (r < p.m && col < p.n) {
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(Cin + r + (long long)col * p.ldc));
+          if (NX == 2)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(Cin2 + r + (long long)col * p.ldc));
+        }
+      }
+    }
+    // NX = 2: one buffer (registers), each chunk's reads with its own TMEM loads
+    constexpr int NB = NX == 2 ? 1 : 2;
+    double2 o1[NB][EC], o2[NB][EC];
+    auto fetch = [&](int ch, double2(&x1)[EC], double2(&x2)[EC]) {
+#pragma unroll
+      for (int j = 0; j < EC; ++j) {
+        const int col = cb + ch * EC + j;
+        const bool in = rok && col < p.n;
+        const long long at = row + (long long)col * p.ldc;
+        if (NX >= 1) x1[j] = in ? Cin[at] : make_double2(0.0, 0.0);
+        if (NX == 2) x2[j] = in ? Cin2[at] : make_double2(0.0, 0.0);
+      }
+    };
+    if (NX >= 1) fetch(0, o1[0], o2[0]);
     const bool waited = mbar_wait(accum, 0u, abort_flag, p.err) && !*abort_flag && nkb > 0;
     const bool ok = __all_sync(0xffffffffu, waited);  // tcgen05.ld below is warp-collective
     tc_fence_after();
-    const int row = m0 + q * 32 + lane;
-    const double sc = p.scale ? p.scale[b] : 1.0;
-    const cplx alpha = mk(p.alpha.x * sc, p.alpha.y * sc);
-    cplx beta = mk(p.beta.x, p.beta.y);
-    if (p.t.beta_b) beta = beta * mk(p.t.beta_b[b].x, p.t.beta_b[b].y);
-    const bool use_beta = (p.beta.x != 0.0 || p.beta.y != 0.0);
-    const double2* Cin = p.t.cin ? p.t.cin + (long long)b * p.t.scin : C;
-    const bool use_2 = p.t.cin2 != nullptr;
-    const double2* Cin2 = use_2 ? p.t.cin2 + (long long)b * p.t.scin2 : C;
-    const cplx beta2 = use_2 ? mk(p.t.beta2.x, p.t.beta2.y) * mk(p.t.beta2_b[b].x, p.t.beta2_b[b].y)
-                             : mk(0.0, 0.0);
-    const cplx dg = mk(p.diag.x, p.diag.y);
-    const int* eB = p.eb + (long long)b * p.n;
-    // undo the power-of-two scaling of the operands: 2^-(row exponent of A)
-    const double row_unscale = row < p.m ? ldexp(1.0, -p.ea[(long long)b * p.m + row]) : 1.0;
     if (ok) {
-      for (int c0 = 0; c0 < MX_BN; c0 += 16) {
-        if (n0 + c0 >= p.n) break;  // warp-uniform
-        uint32_t vr[16], vi[16], cr[16], ci[16];
-        const uint32_t lane_addr = ((uint32_t)(q * 32) << 16);
-        tmem_ld16(tmem + lane_addr + (uint32_t)c0, vr);
-        tmem_ld16(tmem + lane_addr + (uint32_t)(MX_BN + c0), vi);
-        tmem_ld16(tmem + lane_addr + (uint32_t)(2 * MX_BN + c0), cr);
-        tmem_ld16(tmem + lane_addr + (uint32_t)(3 * MX_BN + c0), ci);
+      const uint32_t t0 = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * (MX_BN / 2));
+#pragma unroll
+      for (int ch = 0; ch < NCH; ++ch) {
+        if (cb + ch * EC >= p.n) break;  // warp-uniform
+        uint32_t vr[EC], vi[EC], cr[EC], ci[EC];
+        tmem_ld8(t0 + (uint32_t)(ch * EC), vr);
+        tmem_ld8(t0 + (uint32_t)(MX_BN + ch * EC), vi);
+        tmem_ld8(t0 + (uint32_t)(2 * MX_BN + ch * EC), cr);
+        tmem_ld8(t0 + (uint32_t)(3 * MX_BN + ch * EC), ci);
+        // the next chunk's reads before this chunk's stores: a load after a
+        // store through the same pointer type would otherwise wait for it
+        if (NX == 1 && ch + 1 < NCH) fetch(ch + 1, o1[(ch + 1) % NB], o2[(ch + 1) % NB]);
+        if (NX == 2 && ch > 0) fetch(ch, o1[0], o2[0]);
         tmem_ld_wait();
-        if (row < p.m) {
-          // all 16 reads of C are issued before the first store: a load after
-          // a store through the same pointer type would otherwise wait for it
-          double2 old[16], old2[16];
-          if (use_beta) {
+        if (rok) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int col = n0 + c0 + j;
-              old[j] = col < p.n ? Cin[row + (long long)col * p.ldc] : make_double2(0.0, 0.0);
-            }
-          }
-          if (use_2) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int col = n0 + c0 + j;
-              old2[j] = col < p.n ? Cin2[row + (long long)col * p.ldc] : make_double2(0.0, 0.0);
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int col = n0 + c0 + j;
+          for (int j = 0; j < EC; ++j) {
+            const int col = cb + ch * EC + j;
             if (col < p.n) {
               // K halves: set 0 at columns [0, 2BN), set 1 (empty if nkb == 1) at [2BN, 4BN)
               const double s1r = nkb > 1 ? (double)__uint_as_float(cr[j]) : 0.0;
               const double s1i = nkb > 1 ? (double)__uint_as_float(ci[j]) : 0.0;
-              const double f = row_unscale * ldexp(1.0, -eB[col]);
+              const double f = s_cf[col - n0];
               cplx v = alpha * mk(f * ((double)__uint_as_float(vr[j]) + s1r),
                                   f * ((double)__uint_as_float(vi[j]) + s1i));
-              if (use_beta) v = v + beta * mk(old[j].x, old[j].y);
-              if (use_2) v = v + beta2 * mk(old2[j].x, old2[j].y);
+              if (NX >= 1) v = v + beta * mk(o1[ch % NB][j].x, o1[ch % NB][j].y);
+              if (NX == 2) v = v + beta2 * mk(o2[ch % NB][j].x, o2[ch % NB][j].y);
               if (row == col) v = v + dg;
               C[row + (long long)col * p.ldc] = make_double2(v.x, v.y);
             }
@@ -770,20 +800,22 @@ int gemm_mixed(int m, int n, int k, cplx alpha, const double* scale, const doubl
   // workspace are already those of the operand (the caller's previous call
   // split the same unchanged matrix in the same role and shape; for A the
   // column count n may differ), so the split is skipped
+  // entries the product leaves alone (GemmTerms::need) need no planes of B either
+  // (A's are kept whole for a caller that reuses them)
+  const int* sk = terms.need ? terms.need : steps;
+  const int sk_at = terms.need ? terms.need_above : step;
   int rc;
   if (!(reuse & 1) &&
       (rc = split_operand(true, m, k, kp, a, lda, sa, pa, ea, batch, steps, step, stream)))
     return rc;
   if (!(reuse & 2) &&
-      (rc = split_operand(false, n, k, kp, b, ldb, sb, pb, eb, batch, steps, step, stream)))
+      (rc = split_operand(false, n, k, kp, b, ldb, sb, pb, eb, batch, sk, sk_at, stream)))
     return rc;
   CUtensorMap ta, tb;
   rc = make_map(&ta, pa, m, kp, batch * MX_PLANES, MX_BM);
   if (rc) return rc;
   rc = make_map(&tb, pb, n, kp, batch * MX_PLANES, MX_BN);
   if (rc) return rc;
-  static int smem_done[64];
-  EUV_CUDA_TRY(ensure_smem(gemm_split3_kernel, (int)MX_SMEM, smem_done));
   MixedArgs p;
   p.m = m;
   p.n = n;
@@ -805,9 +837,17 @@ int gemm_mixed(int m, int n, int k, cplx alpha, const double* scale, const doubl
   p.ea = ea;
   p.eb = eb;
   dim3 grid((m + MX_BM - 1) / MX_BM, (n + MX_BN - 1) / MX_BN, batch);
-  gemm_split3_kernel<<<grid, MX_THREADS, MX_SMEM, stream>>>(ta, tb, p);
-  EUV_LAUNCH_CHECK();
-  return EUV_OK;
+  const int nx = terms.cin2 ? 2 : (beta.x != 0.0 || beta.y != 0.0) ? 1 : 0;
+  static int smem_done[3][64];
+  auto launch = [&](auto kernel, int* done) -> int {
+    EUV_CUDA_TRY(ensure_smem(kernel, (int)MX_SMEM, done));
+    kernel<<<grid, MX_THREADS, MX_SMEM, stream>>>(ta, tb, p);
+    EUV_LAUNCH_CHECK();
+    return EUV_OK;
+  };
+  if (nx == 0) return launch(gemm_split3_kernel<0>, smem_done[0]);
+  if (nx == 1) return launch(gemm_split3_kernel<1>, smem_done[1]);
+  return launch(gemm_split3_kernel<2>, smem_done[2]);
 }
 
 }  // namespace euv

@@ -627,7 +627,7 @@ __host__ __device__ inline long long poly_id_at(int n_units, int slice, int t, i
 __global__ void __launch_bounds__(PF_SAMPLES)
     poly_coef_kernel(PolySlices p, const int* lidx, const int* midx, const double* kx0,
                      const double* ky0, const int* polar, double2* coef, double2* ident,
-                     double2* shift, double* radius, int* steps, int* status) {
+                     double2* shift, double* radius, int* steps, int* blocks, int* status) {
   const int u = blockIdx.x, sl = blockIdx.y, tid = threadIdx.x;
   __shared__ double s_lo[2], s_hi[2], s_km[2];
   __shared__ cplx s_f[2][PF_SAMPLES], s_w[PF_SAMPLES], s_a[2][PF_K + 1];
@@ -727,6 +727,7 @@ __global__ void __launch_bounds__(PF_SAMPLES)
     shift[t] = make_double2(ia.x, ia.y);
     radius[t] = g.r;
     steps[t] = m;
+    blocks[t] = jb;
     cplx c = s_a[0][0], sn = s_a[1][0];
     for (int i = 0; i <= p.m[sl]; ++i) {
       ident[poly_id_at(p.n_units, sl, i, 0) + u] = make_double2(c.x, c.y);
@@ -1078,7 +1079,7 @@ struct AmpWork {
   double2 *pw, *pair[3];  // per unit: 6 powers, three pairs of N^2 matrices
   double2 *adm, *V2, *W2, *coef, *ident, *shift;
   double *klm, *radius;
-  int *steps, *ipiv, *info, *capped;
+  int *steps, *blocks, *ipiv, *info, *capped;
   void* mwork;
   size_t mbytes;
 };
@@ -1097,6 +1098,7 @@ static bool carve(const euv_amp_desc* d, Bump& bp, AmpWork& w) {
   w.klm = bp.take<double>(U * N);
   w.radius = bp.take<double>(NS * U);
   w.steps = bp.take<int>(NS * U);
+  w.blocks = bp.take<int>(NS * U);
   w.ipiv = bp.take<int>(U * N);
   w.info = bp.take<int>(U);
   w.capped = bp.take<int>(1);
@@ -1248,7 +1250,7 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
   }
   poly_coef_kernel<<<dim3(U, NS), PF_SAMPLES, 0, stream>>>(ps, d->d_lindex, d->d_mindex, d->d_kx0,
                                                            d->d_ky0, d->d_polar, w.coef, w.ident, w.shift,
-                                                           w.radius, w.steps, status);
+                                                           w.radius, w.steps, w.blocks, status);
   EUV_LAUNCH_CHECK();
 
   // Mixed form: G^-1 by the Euler product (I - E)^-1 = prod_f (I + E^(2^f)),
@@ -1280,6 +1282,8 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
     const Mat* cin2 = nullptr;
     const double2* beta2_b = nullptr;
     cplx beta2 = mk(1.0, 0.0);
+    const int* need = nullptr;
+    int need_above = 0;
   };
   auto mul = [&](cplx alpha, const double* scale, const Mat& A, const Mat& B, cplx beta,
                  const Mat& C, int reuse, const Term& x = Term{}, int n = 0) -> int {
@@ -1291,6 +1295,8 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
     t.scin2 = x.cin2 ? x.cin2->s : 0;
     t.beta2 = make_double2(x.beta2.x, x.beta2.y);
     t.beta2_b = x.beta2_b;
+    t.need = x.need;
+    t.need_above = x.need_above;
     return gemm(N, n > 0 ? n : N, N, alpha, scale, A.p, N, A.s, B.p, N, B.s, beta, C.p, N, C.s,
                 zero, U, nullptr, 0, reuse, t);
   };
@@ -1321,8 +1327,11 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
       if (b < J - 2 &&
           (r2 = poly_blocks<1>(q, N, pb, 6 * nn, w.coef, U, n, b, cs[1].p, nullptr, 2 * nn, stream)))
         return r2;
-      if ((r2 = mul(one, nullptr, pw[q - 1], cs[0], one, cs[1], b < J - 2 ? kReuseA : 0, Term{},
-                    2 * N)))
+      // units whose ellipse needs no block above b hold B_b already
+      Term x;
+      x.need = w.blocks + (size_t)n * U;
+      x.need_above = b + 1;
+      if ((r2 = mul(one, nullptr, pw[q - 1], cs[0], one, cs[1], b < J - 2 ? kReuseA : 0, x, 2 * N)))
         return r2;
       swap(cs[0], cs[1]);
     }

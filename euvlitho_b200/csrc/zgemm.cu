@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(GTHREADS, MI == 2 ? 4 : 2) zgemm_kernel(GemmAr
   double2* C = p.c + (long long)bz * p.sc;
   const int tid = threadIdx.x;
 
+  if (!UPD && p.t.need != nullptr && p.t.need[bz] <= p.t.need_above) return;
   if (p.steps != nullptr && p.step >= p.steps[bz]) {
     // inactive double-angle step for this batch entry: C = A
     // eight loads in flight per thread before their stores
