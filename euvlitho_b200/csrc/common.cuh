@@ -60,6 +60,8 @@ struct GemmTerms {
   // entries with need[b] <= need_above are left as they are (C untouched)
   const int* need = nullptr;
   int need_above = 0;
+  // FP64 form: three real products per complex one (zgemm.cu)
+  bool three = false;
 };
 
 // exp(z) for complex z.

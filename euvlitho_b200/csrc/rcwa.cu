@@ -1297,6 +1297,7 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
     t.beta2_b = x.beta2_b;
     t.need = x.need;
     t.need_above = x.need_above;
+    t.three = true;
     return gemm(N, n > 0 ? n : N, N, alpha, scale, A.p, N, A.s, B.p, N, B.s, beta, C.p, N, C.s,
                 zero, U, nullptr, 0, reuse, t);
   };
@@ -1344,6 +1345,7 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
       GemmTerms t;
       t.cin = s;
       t.scin = t.scin2 = 2 * nn;
+      t.three = true;
       t.beta_b = w.ident + poly_id_at(U, n, step, 0);
       t.cin2 = c;
       t.beta2 = make_double2(2.0, 0.0);
