@@ -60,9 +60,18 @@ struct GemmTerms {
   // entries with need[b] <= need_above are left as they are (C untouched)
   const int* need = nullptr;
   int need_above = 0;
+  // steps come in pairs (0, 1), (2, 3) ... that end in the buffer they began in: an
+  // entry inactive in both is left alone, one active in the first only is copied
+  // back by the second
+  bool paired = false;
   // FP64 form: three real products per complex one (zgemm.cu)
   bool three = false;
 };
+
+// Whether an inactive entry (step >= steps) of a step-predicated GEMM copies A to C.
+__host__ __device__ __forceinline__ bool step_copies(bool paired, int steps, int step) {
+  return !paired || ((step & 1) && steps == step);
+}
 
 // exp(z) for complex z.
 __host__ __device__ __forceinline__ cplx cexp_(cplx z) {

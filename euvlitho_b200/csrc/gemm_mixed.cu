@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(MX_THREADS, 1)
 
   if (p.t.need != nullptr && p.t.need[b] <= p.t.need_above) return;
   if (p.steps != nullptr && p.step >= p.steps[b]) {
+    if (!step_copies(p.t.paired, p.steps[b], p.step)) return;
     // inactive double-angle step of this batch entry: C = A on this tile
     // (eight loads in flight per thread before their stores: the CTA holds a
     // whole SM's shared memory, so the copy must not wait on each element)

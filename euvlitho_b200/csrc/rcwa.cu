@@ -481,15 +481,15 @@ __global__ void taylor_prep_kernel(int n, int batch, const double2* D, const dou
 // sum at every step; with the identity inside the operands the 2048 nm
 // eight-slice image was 1.6e-5 off, 7e-6 for the expansion about 0).  Products: q - 1 for the powers and
 // 2 (J - 1) for the two functions; q and J from poly_plan, a double-angle step
-// only where degree q * jcap is not enough (clips of a few hundred nm with
-// orders near grazing).  With the row recursion of euv_amp (no G^-1, no product
+// only where degree q * jcap is not enough (orders near grazing): a step is two
+// products, as many as one more block, and each doubles the error.  With the row recursion of euv_amp (no G^-1, no product
 // with the solved columns) the call takes 8 N^3 products instead of 25 for a 60
 // nm slab in the mixed form.  B200, whole image calls: four 1024 nm clips at N =
 // 625 (24 units, mixed) 11.64 -> 8.15 ms and 1.1e-5 -> 1.5e-6 of the exact image;
 // N = 961, 6 units, FP64 46.9 -> 27.2 ms; M3D at N = 2177, FP64 94.1 -> 53.5 ms.
-constexpr int PF_K = 24;       // largest degree
+constexpr int PF_K = 30;       // largest degree (one per lane of a warp)
 constexpr int PF_Q = 6;        // largest q
-constexpr int PF_J = 6;        // largest block count (q = 4)
+constexpr int PF_J = 5;        // largest block count
 constexpr int PF_SAMPLES = 64; // points on the ellipse
 constexpr double kPolyTolFp64 = 1e-16;
 constexpr double kPolyTolMixed = 5e-8;  // the split products carry ~1e-6
@@ -570,10 +570,10 @@ __host__ __device__ inline void poly_shape(int precision, double k, cplx eps_m1,
   const double tau0 = 0.25 * d * k * cabs(eps_m1);
   if (precision == EUV_PREC_MIXED) {
     *q = tau0 < 0.16 ? 3 : (tau0 < 0.5 ? 4 : 5);
-    *jcap = *q == 5 ? 3 : 4;
+    *jcap = 4;
   } else {
     *q = tau0 < 0.2 ? 5 : 6;
-    *jcap = 4;
+    *jcap = 5;
   }
 }
 
@@ -606,7 +606,9 @@ struct PolySlices {
   cplx eps_m1[EUV_MAX_SLICES];
   double leps[EUV_MAX_SLICES];  // |log eps|
   double d[EUV_MAX_SLICES];
+  // blocks and steps launched (an even number) and the steps a unit may take
   int q[EUV_MAX_SLICES], jcap[EUV_MAX_SLICES], j[EUV_MAX_SLICES], m[EUV_MAX_SLICES];
+  int m_limit[EUV_MAX_SLICES];
 };
 
 // Coefficients of block b, function f of (unit, slice): PF_Q complex values, the
@@ -616,7 +618,7 @@ __host__ __device__ inline long long poly_coef_at(int n_units, int slice, int un
 }
 // Identity parts [unit] of function f of a slice after t double-angle steps.
 __host__ __device__ inline long long poly_id_at(int n_units, int slice, int t, int f) {
-  return (((long long)slice * (kMaxSteps + 1) + t) * 2 + f) * n_units;
+  return (((long long)slice * (kMaxSteps + 2) + t) * 2 + f) * n_units;
 }
 
 // One CTA of 64 threads per (unit, slice): the ellipse from the unit's own
@@ -662,7 +664,7 @@ __global__ void __launch_bounds__(PF_SAMPLES)
   const PolyRegion g = poly_region(p.k, p.eps_m1[sl], lo, hi, w);
   const int q = p.q[sl], jl = p.j[sl];
   int jb, m;
-  bool ok = poly_pick(g, p.d[sl], p.tol, q, p.jcap[sl], p.m[sl], &jb, &m);
+  bool ok = poly_pick(g, p.d[sl], p.tol, q, p.jcap[sl], p.m_limit[sl], &jb, &m);
   if (jb > jl) {  // more blocks than launched
     jb = jl;
     ok = poly_degree(g, ldexp(p.d[sl], -m), 100.0 * p.tol) <= q * jb;
@@ -687,6 +689,7 @@ __global__ void __launch_bounds__(PF_SAMPLES)
   }
   __syncthreads();
   const int deg = q * jb;
+  static_assert(2 * (PF_K + 1) <= PF_SAMPLES && PF_K < 32, "one thread per coefficient");
   if (tid < 2 * (PF_K + 1)) {
     const int f = tid / (PF_K + 1), n = tid % (PF_K + 1);
     cplx s = mk(0.0, 0.0);
@@ -1042,6 +1045,7 @@ static PolyPlan poly_plan(const euv_amp_desc* d, int slice, double tol) {
   const int limit = d->m_max > 0 && d->m_max < kMaxSteps ? d->m_max : kMaxSteps;
   poly_pick(g, d->dabs[slice], tol, r.q, r.jcap, limit, &r.j, &r.m);
   if (r.m > 0) r.j = r.jcap;  // a unit that needs fewer steps may need all the blocks
+  r.m += r.m & 1;             // steps are launched in pairs (GemmTerms::paired)
   return r;
 }
 
@@ -1093,7 +1097,7 @@ static bool carve(const euv_amp_desc* d, Bump& bp, AmpWork& w) {
   w.V2 = bp.take<double2>(cols);
   w.W2 = bp.take<double2>(cols);
   w.coef = bp.take<double2>(NS * U * 2 * PF_J * PF_Q);
-  w.ident = bp.take<double2>(NS * U * 2 * (kMaxSteps + 1));
+  w.ident = bp.take<double2>(NS * U * 2 * (kMaxSteps + 2));
   w.shift = bp.take<double2>(NS * U);
   w.klm = bp.take<double>(U * N);
   w.radius = bp.take<double>(NS * U);
@@ -1247,6 +1251,7 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
     ps.jcap[n] = r.jcap;
     ps.j[n] = r.j;
     ps.m[n] = r.m;
+    ps.m_limit[n] = d->m_max > 0 && d->m_max < r.m ? d->m_max : r.m;
   }
   poly_coef_kernel<<<dim3(U, NS), PF_SAMPLES, 0, stream>>>(ps, d->d_lindex, d->d_mindex, d->d_kx0,
                                                            d->d_ky0, d->d_polar, w.coef, w.ident, w.shift,
@@ -1345,7 +1350,7 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
       GemmTerms t;
       t.cin = s;
       t.scin = t.scin2 = 2 * nn;
-      t.three = true;
+      t.three = t.paired = true;
       t.beta_b = w.ident + poly_id_at(U, n, step, 0);
       t.cin2 = c;
       t.beta2 = make_double2(2.0, 0.0);

@@ -244,6 +244,7 @@ __global__ void __launch_bounds__(GTHREADS, 3) zgemm_kernel(GemmArgs p) {
 
   if (p.t.need != nullptr && p.t.need[bz] <= p.t.need_above) return;
   if (p.steps != nullptr && p.step >= p.steps[bz]) {
+    if (!step_copies(p.t.paired, p.steps[bz], p.step)) return;
     // inactive double-angle step for this batch entry: C = A
     // eight loads in flight per thread before their stores
     constexpr int U = 8;
