@@ -14,6 +14,8 @@
 //      registers.
 // Only the DFT of the non-zero pupil box is evaluated (the reference FFTs the
 // whole zero-padded grid).  Partial images are added with FP64 atomics.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace euv {
@@ -92,6 +94,7 @@ struct AbbeParams {
   int xdiv, ydiv, lpx, lpy, bx, by, ncut, n_src, n_order, nsplit;
   const double2* coef;
   const int* nidx;
+  const int* px;
   const int* py;
   const int* row_start;
   const int* tab_of_unit;
@@ -321,9 +324,358 @@ __global__ void __launch_bounds__(AB_THREADS) abbe_kernel(AbbeParams p, const do
   }
 }
 
+// ------------------------------------------------------- band-limited form
+// A source's field holds orders l0..l0+Wx, m0..m0+Wy (the pupil disc seen from
+// that source), so |E|^2 holds -Wx..Wx, -Wy..Wy only: it is known from GX x GY
+// samples, GX >= 2 Wx + 1, and a sum over sources has to be carried to the XDIV x
+// YDIV image only once.  At NA 0.33 and 1024 nm that is 28 x 28 samples per source
+// instead of 256 x 256.  The kernel above is bound by its field evaluations; here
+// what remains is the load of the E factors and a few microseconds of set-up and
+// interpolation, so it serves the calls with enough sources x pixels (band_form).
+// B200: linear model, 1024 nm, two clips of 916 sources, FP64, per launch 4930 ->
+// 129 us; 24 units of 1024 nm, 67 sources each, FP32 1215 -> 191 us; four units of
+// 2048 nm, 380 sources, FP32 7.3 -> 0.80 ms.  What bounds it now is latency: three
+// block barriers and one round of gathered loads per source.
+//
+// A cluster of 8 CTAs takes a share of one unit's sources: per source the E
+// factors (as above) in a box that starts at the support (a common phase of a
+// source's field does not matter), both DFT stages on the coarse grid as four-way
+// splits, |E|^2 added to the CTA's samples in shared
+// memory.  Then the eight partial sums are added through distributed shared memory
+// and each CTA interpolates an eighth of the image columns,
+//   I(x, y) = sum_uv Kx(x, u) S(u, v) Ky(y, v),
+//   K(x, u) = D_W(x / X - u / G) / G,  D_W the Dirichlet kernel of degree W,
+// added to the image by FP64 atomics.  W is read off the sources' index tables
+// (nidx >= 0) by the cluster itself, so it holds for any tables; a grid that does not
+// fit shared memory is taken in several passes over rows.
+constexpr int BD_CL = 8;
+constexpr size_t BD_SMEM_MAX = 220 * 1024;
+
+__host__ __device__ inline int up4(int n) { return (n + 3) / 4 * 4; }
+
+// Shared memory for supports of width wx, wy with 4 yc coarse rows per pass and
+// nloc sources per CTA.
+template <typename R>
+__host__ __device__ inline size_t band_bytes(int nloc, int wx, int wy, int yc) {
+  const size_t v = 2 * sizeof(R), ex = up4(wx + 1), ey = up4(wy + 1), gx = up4(2 * wx + 1);
+  size_t b = (((size_t)nloc * sizeof(int2)) + 15) & ~(size_t)15;  // origins
+  b += 2 * gx * 4 * yc * sizeof(double);                          // samples, their sum
+  b += ex * ey * 3 * v;                                           // E
+  b += ex * 4 * yc * 3 * v;                                       // G
+  b += gx * v + (size_t)yc * ey * v;                              // twiddles
+  return b;
+}
+
+// D_w(n / d) / g = sin(pi (2w+1) n/d) / (g sin(pi n/d)); both angles reduced as
+// integers to a quarter turn, so that no digit is lost near multiples of pi.
+// Needs |n| < 2^31 / (2w + 1), d < 2^30.
+__device__ __forceinline__ double dirichlet(int n, int d, int w, int g) {
+  n %= d;
+  if (n < 0) n += d;
+  if (2 * n > d) n = d - n;  // even in n, period d
+  if (n == 0) return (2.0 * w + 1.0) / g;
+  unsigned m = (unsigned)n * (unsigned)(2 * w + 1) % (2u * (unsigned)d);
+  double sg = 1.0;
+  if (m > (unsigned)d) {
+    m = 2u * d - m;
+    sg = -1.0;
+  }
+  if (2 * m > (unsigned)d) m = d - m;
+  const double q = 1.0 / (double)d;
+  return sg * sinpi((double)m * q) / (g * sinpi((double)n * q));
+}
+
+constexpr int BD_PT = 8;  // pupil points per thread whose indices are loaded ahead
+
+template <typename R>
+__global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(512)
+    abbe_band_kernel(AbbeParams p, size_t cap, const double2* ax, double* image) {
+  namespace cg = cooperative_groups;
+  using V2 = typename vec2<R>::type;
+  using C = cx<R>;
+  cg::cluster_group cluster = cg::this_cluster();
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  __shared__ int s_w[2], s_all[2];
+  const int rank = (int)cluster.block_rank();
+  const int u = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
+  const int nsrc_u = p.nsrc_of_unit[u], img = p.img_of_unit[u];
+  const int s_first = blockIdx.x, s_step = gridDim.x;
+  const long long tab = (long long)p.tab_of_unit[u] * p.n_src;
+  const int nloc = (p.n_src + s_step - 1) / s_step;
+  int2* org = reinterpret_cast<int2*>(sm_raw);  // first order of each source's support
+
+  // origins and widths of the supports: a warp per source
+  if (tid < 2) s_w[tid] = 0;
+  __syncthreads();
+  for (int ls = tid >> 5; s_first + ls * s_step < nsrc_u; ls += nt >> 5) {
+    const int* idx = p.nidx + (tab + s_first + ls * s_step) * p.ncut;
+    int lo = 1 << 30, hi = -(1 << 30), mo = 1 << 30, mi = -(1 << 30);
+    for (int i = tid & 31; i < p.ncut; i += 32)
+      if (idx[i] >= 0) {
+        lo = min(lo, p.px[i]);
+        hi = max(hi, p.px[i]);
+        mo = min(mo, p.py[i]);
+        mi = max(mi, p.py[i]);
+      }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+      hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+      mo = min(mo, __shfl_xor_sync(0xffffffffu, mo, off));
+      mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, off));
+    }
+    if ((tid & 31) == 0) {
+      org[ls] = make_int2(lo, mo);
+      if (hi >= lo) {
+        atomicMax(&s_w[0], hi - lo);
+        atomicMax(&s_w[1], mi - mo);
+      }
+    }
+  }
+  __syncthreads();
+  if (tid < 2) s_all[tid] = s_w[tid];
+  cluster.sync();
+  if (tid < 2) {
+    int w = 0;
+    for (int t = 0; t < BD_CL; ++t) w = max(w, *cluster.map_shared_rank(&s_all[tid], t));
+    s_w[tid] = w;
+  }
+  __syncthreads();
+  // (orders lie in the pupil box, which bounds the grid the host made room for)
+  const int wx = min(s_w[0], 2 * p.lpx), wy = min(s_w[1], 2 * p.lpy);
+  const int gx = up4(2 * wx + 1), gy = up4(2 * wy + 1), gx4 = gx / 4, gy4 = gy / 4;
+  const int ex = up4(wx + 1), ey = up4(wy + 1);  // box of E, zero outside the support
+  // rows of the coarse grid per pass: y0 in [ya, ya + yc), each with its three
+  // partners y0 + q gy / 4 (the host has checked that one fits)
+  int yc = gy4;
+  while (yc > 1 && band_bytes<R>(nloc, wx, wy, yc) > cap) --yc;
+  const int rows = 4 * yc;
+  double* acc = reinterpret_cast<double*>(sm_raw + (((size_t)nloc * sizeof(int2) + 15) & ~(size_t)15));
+  double* sum = acc + (size_t)gx * rows;
+  double* work = sum + (size_t)gx * rows;  // E, G, twiddles; the kernels when the sources are done
+  const size_t work_n = (cap - (reinterpret_cast<unsigned char*>(work) - sm_raw)) / sizeof(double);
+  V2* E = reinterpret_cast<V2*>(work);          // [ex][ey][3]
+  V2* G = E + (size_t)ex * ey * 3;              // [ex][rows][3]
+  V2* twx = G + (size_t)ex * rows * 3;          // [gx]
+  V2* twy = twx + gx;                           // [yc][ey]
+  const double wgt = p.inv_weight[img];
+  double* im = image + (size_t)img * p.xdiv * p.ydiv;
+  for (int ya = 0; ya < gy4; ya += yc) {
+    const int ny = min(yc, gy4 - ya), nrow = 4 * ny;
+    for (int j = tid; j < gx; j += nt) {
+      double sn, cs;
+      sincospi(2.0 * j / gx, &sn, &cs);
+      twx[j] = V2{(R)cs, (R)sn};
+    }
+    for (int j = tid; j < ny * ey; j += nt) {
+      double sn, cs;
+      sincospi(2.0 * (double)((j % ey) * (ya + j / ey) % gy) / gy, &sn, &cs);
+      twy[j] = V2{(R)cs, (R)sn};
+    }
+    for (int j = tid; j < gx * nrow; j += nt) acc[j] = 0.0;
+    for (int j = tid; j < ex * ey * 3; j += nt) E[j] = V2{(R)0, (R)0};
+    // order indices of the first source, then of the next one while this one runs
+    int nx[BD_PT];
+    auto indices = [&](int s) {
+#pragma unroll
+      for (int k = 0; k < BD_PT; ++k) {
+        const int i = tid + k * nt;
+        nx[k] = (s < nsrc_u && i < p.ncut) ? p.nidx[(tab + s) * p.ncut + i] : -1;
+      }
+    };
+    indices(s_first);
+    __syncthreads();
+    int ls = 0;
+    for (int s = s_first; s < nsrc_u; s += s_step, ++ls) {
+      const int2 o0 = org[ls];
+      const double2* axs = ax + ((long long)u * p.n_src + s) * p.n_order;
+      const double2* cfs = p.coef + (tab + s) * p.ncut * 3;
+      auto place = [&](int i, int n) {
+        const double2 a = axs[n];
+        V2* e = E + ((size_t)(p.px[i] - o0.x) * ey + (p.py[i] - o0.y)) * 3;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double2 f = cfs[(size_t)i * 3 + c];
+          const cplx v = mk(f.x, f.y) * mk(a.x, a.y);
+          e[c] = V2{(R)v.x, (R)v.y};
+        }
+      };
+#pragma unroll
+      for (int k = 0; k < BD_PT; ++k)
+        if (nx[k] >= 0) place(tid + k * nt, nx[k]);
+      for (int i = tid + BD_PT * nt; i < p.ncut; i += nt) {
+        const int n = p.nidx[(tab + s) * p.ncut + i];
+        if (n >= 0) place(i, n);
+      }
+      __syncthreads();
+      indices(s + s_step);
+      // stage y: four rows per sum (radix 4 in the order mod 4)
+      for (int o = tid; o < ny * ex * 3; o += nt) {
+        const int c = o % 3, lx = (o / 3) % ex, yy = o / (3 * ex);
+        const V2* ty = twy + yy * ey;
+        const V2* e = E + (size_t)lx * ey * 3 + c;
+        C g[4] = {{(R)0, (R)0}, {(R)0, (R)0}, {(R)0, (R)0}, {(R)0, (R)0}};
+        for (int m = 0; m < ey; m += 4)
+#pragma unroll
+          for (int k = 0; k < 4; ++k, e += 3) g[k] = g[k] + C{e[0].x, e[0].y} * C{ty[m + k].x, ty[m + k].y};
+        const C A = g[0] + g[2], B{g[0].x - g[2].x, g[0].y - g[2].y};
+        const C S = g[1] + g[3], D{g[1].x - g[3].x, g[1].y - g[3].y};
+        V2* out = G + ((size_t)lx * nrow + yy) * 3 + c;
+        out[0] = V2{A.x + S.x, A.y + S.y};
+        out[(size_t)ny * 3] = V2{B.x - D.y, B.y + D.x};
+        out[(size_t)2 * ny * 3] = V2{A.x - S.x, A.y - S.y};
+        out[(size_t)3 * ny * 3] = V2{B.x + D.y, B.y - D.x};
+      }
+      __syncthreads();
+      // E back to zero for the next source; stage x and |f|^2: four columns per
+      // pass over the rows of G
+      for (int j = tid; j < ex * ey * 3; j += nt) E[j] = V2{(R)0, (R)0};
+      for (int o = tid; o < gx4 * nrow; o += nt) {
+        const int x0 = o / nrow, yl = o - x0 * nrow;
+        C P[4][3];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) P[k][0] = P[k][1] = P[k][2] = C{(R)0, (R)0};
+        const V2* gp = G + (size_t)yl * 3;
+        int at = 0;  // lx x0 mod gx
+        for (int lx = 0; lx < ex; lx += 4) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k, gp += (size_t)nrow * 3) {
+            const V2 t = twx[at];
+            const C w{t.x, t.y};
+#pragma unroll
+            for (int c = 0; c < 3; ++c) P[k][c] = P[k][c] + C{gp[c].x, gp[c].y} * w;
+            at += x0;
+            if (at >= gx) at -= gx;
+          }
+        }
+        double e[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const C A = P[0][c] + P[2][c], B{P[0][c].x - P[2][c].x, P[0][c].y - P[2][c].y};
+          const C S = P[1][c] + P[3][c], D{P[1][c].x - P[3][c].x, P[1][c].y - P[3][c].y};
+          const C f[4] = {{A.x + S.x, A.y + S.y}, {B.x - D.y, B.y + D.x},
+                          {A.x - S.x, A.y - S.y}, {B.x + D.y, B.y - D.x}};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) e[q] += (double)(f[q].x * f[q].x + f[q].y * f[q].y);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[(x0 + q * gx4) * nrow + yl] += e[q];
+      }
+      __syncthreads();
+    }
+    __syncthreads();
+    cluster.sync();
+    // sum of the cluster's samples: each CTA adds an eighth and hands it to all
+    const int total = gx * nrow, share = (total + BD_CL - 1) / BD_CL;
+    for (int j = rank * share + tid; j < min(total, (rank + 1) * share); j += nt) {
+      double v = 0.0;
+#pragma unroll
+      for (int t = 0; t < BD_CL; ++t) v += cluster.map_shared_rank(acc, t)[j];
+#pragma unroll
+      for (int t = 0; t < BD_CL; ++t) cluster.map_shared_rank(sum, t)[j] = v;
+    }
+    cluster.sync();
+    // interpolation of the columns x in [xa, xb): in strips of columns and rows
+    // whose kernels fit the shared memory of E and G
+    const int xs = (p.xdiv + BD_CL - 1) / BD_CL, xa = rank * xs, xb = min(p.xdiv, xa + xs);
+    const int xt = max(1, min(xs, (int)(work_n / 2 / (size_t)(gx + nrow))));
+    const int yt = max(1, min(p.ydiv, (int)(work_n / 2 / (size_t)nrow)));
+    double* T = work;                    // [xt][nrow]
+    double* Kx = work + (size_t)xt * nrow;  // [xt][gx]
+    double* Ky = work + work_n / 2;      // [nrow][yt]
+    for (int y0 = 0; y0 < p.ydiv; y0 += yt) {
+      const int yn = min(yt, p.ydiv - y0);
+      __syncthreads();
+      for (int j = tid; j < yn * nrow; j += nt) {
+        const int v = j / yn, y = y0 + j % yn, row = ya + v % ny + (v / ny) * gy4;
+        Ky[j] = wgt * dirichlet(y * gy - row * p.ydiv, gy * p.ydiv, wy, gy);
+      }
+      for (int x0 = xa; x0 < xb; x0 += xt) {
+        const int xn = min(xt, xb - x0);
+        __syncthreads();
+        for (int j = tid; j < xn * gx; j += nt) {
+          const int x = x0 + j / gx, c = j % gx;
+          Kx[j] = dirichlet(x * gx - c * p.xdiv, gx * p.xdiv, wx, gx);
+        }
+        __syncthreads();
+        for (int j = tid; j < xn * nrow; j += nt) {
+          const int xx = j / nrow, v = j - xx * nrow;
+          double t = 0.0;
+          for (int c = 0; c < gx; ++c) t = fma(Kx[xx * gx + c], sum[c * nrow + v], t);
+          T[j] = t;
+        }
+        __syncthreads();
+        // lanes take consecutive y; four columns share each Ky value
+        const int xg = (xn + 3) / 4;
+        for (int j = tid; j < xg * yn; j += nt) {
+          const int g = j / yn, y = j - g * yn, left = xn - 4 * g;
+          double v[4] = {0.0, 0.0, 0.0, 0.0};
+          const double* t = T + (size_t)4 * g * nrow;
+          for (int r = 0; r < nrow; ++r) {
+            const double ky = Ky[r * yn + y];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (q < left) v[q] = fma(t[q * nrow + r], ky, v[q]);
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (q < left) atomicAdd(&im[(size_t)(x0 + 4 * g + q) * p.ydiv + y0 + y], v[q]);
+        }
+      }
+    }
+    __syncthreads();
+    // a peer may still read this CTA's samples or write its sum
+    cluster.sync();
+  }
+}
+
 }  // namespace euv
 
 using namespace euv;
+
+// The band-limited form pays from 2e7 field evaluations (sources x pixels x pupil
+// rows) per launch on, below that its set-up costs more than it saves, and where
+// one row pass of the widest possible support fits shared memory.
+static size_t band_least(const euv_abbe_desc* d) {
+  return d->precision == EUV_PREC_MIXED ? band_bytes<float>(d->n_src, 2 * d->lpx, 2 * d->lpy, 1)
+                                        : band_bytes<double>(d->n_src, 2 * d->lpx, 2 * d->lpy, 1);
+}
+static bool band_form(const euv_abbe_desc* d) {
+  const double work = (double)d->n_units * d->n_src * d->xdiv * d->ydiv * (2 * d->lpx + 1);
+  return work >= 2e7 && band_least(d) <= BD_SMEM_MAX &&
+         (double)(4 * d->lpx + 8) * d->xdiv * (4 * d->lpx + 1) < 2e9 &&
+         (double)(4 * d->lpy + 8) * d->ydiv * (4 * d->lpy + 1) < 2e9;  // dirichlet's range
+}
+
+template <typename R>
+static int launch_band(const euv_abbe_desc* d, const AbbeParams& p, const double2* ax, double* image,
+                       cudaStream_t stream) {
+  // clusters per unit: one CTA per SM, two where more sources than that wait, no
+  // more clusters than groups of eight sources
+  int dev = 0, sms = 148;
+  EUV_CUDA_TRY(cudaGetDevice(&dev));
+  EUV_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  int nc = (2 * sms - 4 * BD_CL) / (BD_CL * d->n_units);
+  const int most = (d->n_src + BD_CL - 1) / BD_CL;
+  nc = nc < 1 ? 1 : nc > most ? most : nc;
+  const int nloc = (d->n_src + BD_CL * nc - 1) / (BD_CL * nc);
+  // shared memory for the supports of a pupil disc (width lp) in one pass, at
+  // least one row of the widest possible
+  const int gx = up4(2 * d->lpx + 1), gy = up4(2 * d->lpy + 1);
+  size_t smem = band_bytes<R>(nloc, d->lpx, d->lpy, gy / 4);
+  const size_t least = band_least(d);
+  if (smem > BD_SMEM_MAX) smem = BD_SMEM_MAX;
+  if (smem < least) smem = least;
+  static int done[64];
+  EUV_CUDA_TRY(ensure_smem(abbe_band_kernel<R>, (int)BD_SMEM_MAX, done));
+  // threads: the fewest rounds of stage x's (column group, row) items
+  const int items = gx / 4 * gy, rounds = (items + 511) / 512;
+  int threads = ((items + rounds - 1) / rounds + 31) / 32 * 32;
+  if (threads < 128) threads = 128;
+  abbe_band_kernel<R><<<dim3(BD_CL * nc, d->n_units), threads, smem, stream>>>(p, smem, ax, image);
+  EUV_LAUNCH_CHECK();
+  return EUV_OK;
+}
 
 extern "C" int euv_abbe(const euv_abbe_desc* d, const euv_c64* d_ax, double* d_image,
                         void* stream_) {
@@ -349,6 +701,7 @@ extern "C" int euv_abbe(const euv_abbe_desc* d, const euv_c64* d_ax, double* d_i
   p.n_order = d->n_order;
   p.coef = reinterpret_cast<const double2*>(d->d_coef);
   p.nidx = d->d_nidx;
+  p.px = d->d_px;
   p.py = d->d_py;
   p.row_start = d->d_row_start;
   p.tab_of_unit = d->d_tab_of_unit;
@@ -365,6 +718,10 @@ extern "C" int euv_abbe(const euv_abbe_desc* d, const euv_c64* d_ax, double* d_i
   if (smem > 227 * 1024) {
     euv_set_error("euv_abbe: pupil too large for one CTA (%zu bytes of shared memory)", smem);
     return EUV_ERR_BAD_ARG;
+  }
+  if (band_form(d)) {
+    if (fp32) return launch_band<float>(d, p, reinterpret_cast<const double2*>(d_ax), d_image, stream);
+    return launch_band<double>(d, p, reinterpret_cast<const double2*>(d_ax), d_image, stream);
   }
   using Kern = void (*)(AbbeParams, const double2*, double*);
   static const Kern kerns[4] = {abbe_kernel<double, false>, abbe_kernel<double, true>,
