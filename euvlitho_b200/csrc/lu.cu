@@ -14,8 +14,9 @@
 //   update : A22 -= L21 U12 with the batched DMMA zgemm;
 //   look-ahead: the next panel is factored on a high-priority side stream while
 //            the rest of the update runs (the panel alone fills only `batch` SMs).
-// Solve: the row swaps on B, then one launch that keeps 8 (or fewer, for large
-// n) columns of X in shared memory per CTA through both substitutions.
+// Solve: the row swaps on B, then one launch that keeps 8 or 12 columns of X in
+// shared memory per CTA through both substitutions, or blocks of 32 rows (two
+// launches each) where fewer columns fit.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -132,8 +133,9 @@ __global__ void __launch_bounds__(LU_PANEL_THREADS) lu_panel_kernel(int n, int j
 // with the block's columns at compile-time register indices v[0..LC_BLK); the
 // register row is rotated by LC_BLK after each block (one block's code for the
 // whole panel, no runtime register indexing).  One cluster barrier per column
-// jj: before it, every CTA finds its candidate (first max of |re|+|im| in its
-// rows >= jj, as izamax; every warp reduces the warp maxima itself) and sends
+// jj (a block barrier for one CTA): before it, every CTA finds its candidate (first
+// max of |re|+|im| in its rows >= jj, as izamax; every warp reduces the warp maxima
+// itself) and sends
 // the candidate's value, index and row to every CTA through distributed shared
 // memory, one column per lane of the warp that holds the row, and rank 0 sends
 // row jj the same way; after it, every thread reduces the LC candidates in
@@ -153,25 +155,52 @@ constexpr int LC_BLK = 4;
 static_assert(LU_NB == 32, "one panel column per lane");
 static_assert(LU_NB % LC_BLK == 0, "whole blocks");
 
-__device__ __forceinline__ void argmax_step(double& v, int& i, double ov, int oi) {
-  if (ov > v || (ov == v && oi < i)) {
-    v = ov;
-    i = oi;
-  }
+// A panel column costs about 1.5 us at 256 rows (1.8 before the three reductions in
+// hardware, the reciprocal with one division and the search under the update); what
+// is left is a chain of two barriers, the reductions, the division and 31 updates of
+// a row by every thread.
+// Candidates compare as the bits of |re|+|im| (order of non-negative doubles), ties
+// to the smallest row: three warp reductions in hardware.  Lanes without a row hold
+// key 0 and row n.
+struct Cand {
+  unsigned long long key;
+  int row;
+};
+__device__ __forceinline__ Cand warp_argmax(unsigned long long key, int row) {
+  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  const int r = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? row : 0x7fffffff);
+  return Cand{((unsigned long long)mh << 32) | ml, r};
+}
+__device__ __forceinline__ unsigned long long abs_key(cplx v) {
+  return (unsigned long long)__double_as_longlong(cabs1(v));
+}
+
+// 1 / d: one real division, d scaled by a power of two so that |d|^2 neither
+// over- nor underflows (the exponents at the ends of the range divide as cdiv)
+__device__ __forceinline__ cplx crecip(cplx d) {
+  const double m = fmax(fabs(d.x), fabs(d.y));
+  const int e = (__double2hiint(m) >> 20) & 0x7ff;
+  if (e < 2 || e > 2044) return cdiv(mk(1.0, 0.0), d);
+  const double s = __hiloint2double((2046 - e) << 20, 0);
+  const double x = d.x * s, y = d.y * s;
+  const double r = s / (x * x + y * y);
+  return mk(x * r, -y * r);
 }
 
 template <int LC>
-__global__ void __cluster_dims__(LC, 1, 1) __launch_bounds__(LC_THREADS, 1)
+__global__ void __launch_bounds__(LC_THREADS, 1)
     lu_panel_cluster_kernel(int n, int j0, int jb, double2* A, long long lda, long long sa,
                             int* ipiv, int* info) {
   cg::cluster_group cluster = cg::this_cluster();
-  const int q = (int)cluster.block_rank();
+  const int q = LC == 1 ? 0 : (int)cluster.block_rank();
   const int mat = blockIdx.x / LC;
   A += (long long)mat * sa;
   ipiv += (long long)mat * n;
-  __shared__ double s_wv[LU_NB][LC_WARPS];
+  __shared__ unsigned long long s_wk[LU_NB][LC_WARPS];
   __shared__ int s_wi[LU_NB][LC_WARPS];
-  __shared__ double s_cv[LU_NB][LC];
+  __shared__ unsigned long long s_ck[LU_NB][LC];
   __shared__ int s_ci[LU_NB][LC];
   __shared__ double2 s_crow[2][LC][LU_NB];  // candidate rows, by rank
   __shared__ double2 s_rjj[2][LU_NB];       // row jj
@@ -184,6 +213,9 @@ __global__ void __cluster_dims__(LC, 1, 1) __launch_bounds__(LC_THREADS, 1)
 #pragma unroll
   for (int k = 0; k < LU_NB; ++k)
     v[k] = (own && k < jb) ? ld2(&A[r + (long long)(j0 + k) * lda]) : mk(0.0, 0.0);
+  // this warp's candidate of the first column; later ones are found as soon as
+  // their column is updated, under the rest of the rank-1 update
+  Cand w = warp_argmax(own ? abs_key(v[0]) : 0ull, own ? r : n);
 #pragma unroll 1
   for (int c0 = 0; c0 < jb; c0 += LC_BLK) {  // jb is the same for every thread
 #pragma unroll
@@ -191,33 +223,21 @@ __global__ void __cluster_dims__(LC, 1, 1) __launch_bounds__(LC_THREADS, 1)
       const int c = c0 + i;
       if (c >= jb) break;
       const int jj = j0 + c, buf = c & 1;
-      double best = (own && r >= jj) ? cabs1(v[i]) : -1.0;
-      int bidx = (own && r >= jj) ? r : n;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1)
-        argmax_step(best, bidx, __shfl_xor_sync(0xffffffffu, best, off),
-                    __shfl_xor_sync(0xffffffffu, bidx, off));
       if (lane == 0) {
-        s_wv[c][warp] = best;
-        s_wi[c][warp] = bidx;
+        s_wk[c][warp] = w.key;
+        s_wi[c][warp] = w.row;
       }
       __syncthreads();
       {
-        double bv = lane < LC_WARPS ? s_wv[c][lane] : -1.0;
-        int bi = lane < LC_WARPS ? s_wi[c][lane] : n;
-#pragma unroll
-        for (int off = LC_WARPS / 2; off > 0; off >>= 1)
-          argmax_step(bv, bi, __shfl_xor_sync(0xffffffffu, bv, off),
-                      __shfl_xor_sync(0xffffffffu, bi, off));
-        // lane 0 decides (the lanes agree unless a NaN breaks the order)
-        bv = __shfl_sync(0xffffffffu, bv, 0);
-        bi = __shfl_sync(0xffffffffu, bi, 0);
+        const Cand b = warp_argmax(lane < LC_WARPS ? s_wk[c][lane] : 0ull,
+                                   lane < LC_WARPS ? s_wi[c][lane] : n);
+        const int bi = b.row;
         if (bi < n && (bi - j0 - q * LC_THREADS) >> 5 == warp) {
           if (r == bi)
 #pragma unroll
             for (int k = i; k < LU_NB; ++k) s_crow[buf][q][k] = make_double2(v[k].x, v[k].y);
           __syncwarp();
-          if (lane >= i) {
+          if (LC > 1 && lane >= i) {
             const double2 x = s_crow[buf][q][lane];
 #pragma unroll
             for (int t = 0; t < LC; ++t)
@@ -225,8 +245,13 @@ __global__ void __cluster_dims__(LC, 1, 1) __launch_bounds__(LC_THREADS, 1)
           }
         }
         if (warp == 0 && lane < LC) {
-          *cluster.map_shared_rank(&s_cv[c][q], lane) = bv;
-          *cluster.map_shared_rank(&s_ci[c][q], lane) = bi;
+          if (LC == 1) {
+            s_ck[c][0] = b.key;
+            s_ci[c][0] = bi;
+          } else {
+            *cluster.map_shared_rank(&s_ck[c][q], lane) = b.key;
+            *cluster.map_shared_rank(&s_ci[c][q], lane) = bi;
+          }
         }
       }
       if (q == 0 && warp == 0) {
@@ -234,21 +259,24 @@ __global__ void __cluster_dims__(LC, 1, 1) __launch_bounds__(LC_THREADS, 1)
 #pragma unroll
           for (int k = i; k < LU_NB; ++k) s_rjj[buf][k] = make_double2(v[k].x, v[k].y);
         __syncwarp();
-        if (lane >= i) {
+        if (LC > 1 && lane >= i) {
           const double2 x = s_rjj[buf][lane];
 #pragma unroll
           for (int t = 1; t < LC; ++t) *cluster.map_shared_rank(&s_rjj[buf][lane], t) = x;
         }
       }
-      cluster.sync();
-      double bv = s_cv[c][0];
+      if (LC == 1)
+        __syncthreads();
+      else
+        cluster.sync();
+      unsigned long long bk = s_ck[c][0];
       int bi = s_ci[c][0], qw = 0;
 #pragma unroll
       for (int t = 1; t < LC; ++t) {
-        const double ov = s_cv[c][t];
+        const unsigned long long ok = s_ck[c][t];
         const int oi = s_ci[c][t];
-        if (ov > bv || (ov == bv && oi < bi)) {
-          bv = ov;
+        if (ok > bk || (ok == bk && oi < bi)) {
+          bk = ok;
           bi = oi;
           qw = t;
         }
@@ -262,18 +290,27 @@ __global__ void __cluster_dims__(LC, 1, 1) __launch_bounds__(LC_THREADS, 1)
         for (int k = i; k < LU_NB; ++k) v[k] = mk(src[k].x, src[k].y);
       }
       const double2 dd = prow[i];
-      if (dd.x == 0.0 && dd.y == 0.0) {
-        if (zero_col == 0) zero_col = jj + 1;
-      } else if (own && r > jj) {
-        const cplx l = v[i] * cdiv(mk(1.0, 0.0), mk(dd.x, dd.y));
+      const bool zero = dd.x == 0.0 && dd.y == 0.0;
+      if (zero && zero_col == 0) zero_col = jj + 1;
+      const bool below = own && r > jj;
+      cplx l = mk(0.0, 0.0);
+      if (!zero && below) {
+        l = v[i] * crecip(mk(dd.x, dd.y));
         v[i] = l;
-        // columns c+1 .. jb-1 are v[i+1 .. jb-1-c0]; blocks of 8 past them are skipped
+      }
+      // column c + 1 first: its candidates are sought while the others are updated
+      if (i + 1 < LU_NB) {
+        if (!zero && below) v[i + 1] = v[i + 1] - l * mk(prow[i + 1].x, prow[i + 1].y);
+        w = warp_argmax(below ? abs_key(v[i + 1]) : 0ull, below ? r : n);
+      }
+      if (!zero && below) {
+        // columns c+2 .. jb-1 are v[i+2 .. jb-1-c0]; blocks of 8 past them are skipped
 #pragma unroll
         for (int k0 = 0; k0 < LU_NB; k0 += 8) {
-          if (k0 + 8 > i + 1 && k0 < jb - c0) {
+          if (k0 + 8 > i + 2 && k0 < jb - c0) {
 #pragma unroll
             for (int k = k0; k < k0 + 8; ++k)
-              if (k > i) v[k] = v[k] - l * mk(prow[k].x, prow[k].y);
+              if (k > i + 1) v[k] = v[k] - l * mk(prow[k].x, prow[k].y);
           }
         }
       }
@@ -290,6 +327,56 @@ __global__ void __cluster_dims__(LC, 1, 1) __launch_bounds__(LC_THREADS, 1)
     if (tid < jb) ipiv[j0 + tid] = s_piv[tid];
     if (tid == 0 && zero_col != 0 && info[mat] == 0) info[mat] = zero_col;
   }
+}
+
+template <int LC>
+static void panel_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int batch,
+                         cudaStream_t st) {
+  cfg = {};
+  cfg.gridDim = dim3(LC * batch);
+  cfg.blockDim = dim3(LC_THREADS);
+  cfg.stream = st;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = LC;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = LC > 1 ? 1 : 0;
+}
+
+template <int LC>
+static int launch_panel(int n, int j0, int jb, double2* A, long long lda, long long sa, int* ipiv,
+                        int* info, int batch, cudaStream_t st) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[1];
+  panel_config<LC>(cfg, at, batch, st);
+  EUV_CUDA_TRY(cudaLaunchKernelEx(&cfg, lu_panel_cluster_kernel<LC>, n, j0, jb, A, lda, sa, ipiv,
+                                  info));
+  EUV_LAUNCH_CHECK();
+  return EUV_OK;
+}
+
+// Whether this device runs clusters of 16 (beyond the portable size), asked once.
+static bool panel16() {
+  static int state[64];  // 0 unknown, 1 yes, 2 no
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  int st = __atomic_load_n(&state[dev], __ATOMIC_ACQUIRE);
+  if (st == 0) {
+    int clusters = 0;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    panel_config<16>(cfg, at, 1, nullptr);
+    const bool ok = cudaFuncSetAttribute(lu_panel_cluster_kernel<16>,
+                                         cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                         1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&clusters, lu_panel_cluster_kernel<16>, &cfg) ==
+                        cudaSuccess &&
+                    clusters > 0;
+    if (!ok) (void)cudaGetLastError();
+    st = ok ? 1 : 2;
+    __atomic_store_n(&state[dev], st, __ATOMIC_RELEASE);
+  }
+  return st == 1;
 }
 
 // Row swaps ipiv[j0..j0+jb) applied to every column outside [skip0, skip1).
@@ -321,55 +408,8 @@ __global__ void lu_laswp_kernel(int n, int ncols, int j0, int jb, int skip0, int
 }
 
 // X = T^-1 X for a jb x jb triangular block T of the factor (unit lower when
-// lower != 0, non-unit upper otherwise) and the jb-row slab X of `ncols`
-// columns.  One thread per column; T staged in shared memory.
-__global__ void lu_trsm_block_kernel(int jb, int ncols, int lower, const double2* T,
-                                     long long ldt, long long st, double2* X, long long ldx,
-                                     long long sx) {
-  __shared__ double2 Ts[LU_NB][LU_NB + 1];
-  const int b = blockIdx.y;
-  T += (long long)b * st;
-  X += (long long)b * sx;
-  for (int idx = threadIdx.x; idx < jb * jb; idx += blockDim.x) {
-    int r = idx % jb, c = idx / jb;
-    Ts[r][c] = T[r + (long long)c * ldt];
-  }
-  __syncthreads();
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= ncols) return;
-  cplx x[LU_NB];
-#pragma unroll
-  for (int r = 0; r < LU_NB; ++r)
-    if (r < jb) x[r] = ld2(&X[r + (long long)col * ldx]);
-  if (lower) {
-#pragma unroll
-    for (int r = 0; r < LU_NB; ++r) {
-      if (r < jb) {
-        cplx s = x[r];
-#pragma unroll
-        for (int q = 0; q < LU_NB; ++q)
-          if (q < r) s = s - mk(Ts[r][q].x, Ts[r][q].y) * x[q];
-        x[r] = s;
-      }
-    }
-  } else {
-#pragma unroll
-    for (int r = LU_NB - 1; r >= 0; --r) {
-      if (r < jb) {
-        cplx s = x[r];
-#pragma unroll
-        for (int q = 0; q < LU_NB; ++q)
-          if (q > r && q < jb) s = s - mk(Ts[r][q].x, Ts[r][q].y) * x[q];
-        x[r] = cdiv(s, mk(Ts[r][r].x, Ts[r][r].y));
-      }
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < LU_NB; ++r)
-    if (r < jb) st2(&X[r + (long long)col * ldx], x[r]);
-}
-
-// The same solve with one warp per column: lane r holds row r of X; step q
+// lower != 0, non-unit upper otherwise) and the jb-row slab X of `ncols` columns,
+// one warp per column, T staged in shared memory: lane r holds row r of X; step q
 // broadcasts the finished x_q by shuffle and every later (lower) or earlier
 // (upper) lane subtracts its term, so a column takes jb short steps instead of
 // one thread's chain of jb^2/2 dependent products.  8 columns per CTA.
@@ -397,8 +437,10 @@ __global__ void __launch_bounds__(32 * LU_TRSM_WARPS)
       if (lane > q && lane < jb) x = x - mk(Ts[lane][q].x, Ts[lane][q].y) * xq;
     }
   } else {
+    // each lane's reciprocal pivot, off the serial chain
+    const cplx rinv = lane < jb ? crecip(mk(Ts[lane][lane].x, Ts[lane][lane].y)) : mk(0.0, 0.0);
     for (int q = jb - 1; q >= 0; --q) {
-      if (lane == q) x = cdiv(x, mk(Ts[q][q].x, Ts[q][q].y));
+      if (lane == q) x = x * rinv;
       const cplx xq = mk(__shfl_sync(0xffffffffu, x.x, q), __shfl_sync(0xffffffffu, x.y, q));
       if (lane < q) x = x - mk(Ts[lane][q].x, Ts[lane][q].y) * xq;
     }
@@ -443,7 +485,9 @@ static cudaError_t lu_side(LuSide** out) {
 // Row-swap granularity the laswp after panel j0 applies to the panel's own
 // columns: 1 after the cluster kernel (column c lacks the swaps of pivots
 // c+1..), 0 after lu_panel_kernel (the panel's columns are complete).
-static int panel_sub(int n, int j0) { return n - j0 <= 8 * LC_THREADS ? 1 : 0; }
+static int panel_sub(int n, int j0) {
+  return n - j0 <= 8 * LC_THREADS || (n - j0 <= 16 * LC_THREADS && panel16()) ? 1 : 0;
+}
 
 static int lu_panel(int n, int j0, int jb, double2* A, long long lda, long long sa, int* ipiv,
                     int* info, int batch, cudaStream_t st) {
@@ -451,15 +495,15 @@ static int lu_panel(int n, int j0, int jb, double2* A, long long lda, long long 
   // the tuning table may spread a panel's rows over more CTAs than they need
   const int lc_min = tune_lookup(EUV_KNOB_LU_CLUSTER, n, batch);
   if (rows <= LC_THREADS && lc_min <= 1)
-    lu_panel_cluster_kernel<1><<<batch, LC_THREADS, 0, st>>>(n, j0, jb, A, lda, sa, ipiv, info);
-  else if (rows <= 2 * LC_THREADS && lc_min <= 2)
-    lu_panel_cluster_kernel<2><<<2 * batch, LC_THREADS, 0, st>>>(n, j0, jb, A, lda, sa, ipiv, info);
-  else if (rows <= 4 * LC_THREADS && lc_min <= 4)
-    lu_panel_cluster_kernel<4><<<4 * batch, LC_THREADS, 0, st>>>(n, j0, jb, A, lda, sa, ipiv, info);
-  else if (rows <= 8 * LC_THREADS)
-    lu_panel_cluster_kernel<8><<<8 * batch, LC_THREADS, 0, st>>>(n, j0, jb, A, lda, sa, ipiv, info);
-  else
-    lu_panel_kernel<<<batch, LU_PANEL_THREADS, 0, st>>>(n, j0, jb, A, lda, sa, ipiv, info);
+    return launch_panel<1>(n, j0, jb, A, lda, sa, ipiv, info, batch, st);
+  if (rows <= 2 * LC_THREADS && lc_min <= 2)
+    return launch_panel<2>(n, j0, jb, A, lda, sa, ipiv, info, batch, st);
+  if (rows <= 4 * LC_THREADS && lc_min <= 4)
+    return launch_panel<4>(n, j0, jb, A, lda, sa, ipiv, info, batch, st);
+  if (rows <= 8 * LC_THREADS) return launch_panel<8>(n, j0, jb, A, lda, sa, ipiv, info, batch, st);
+  if (rows <= 16 * LC_THREADS && panel16())
+    return launch_panel<16>(n, j0, jb, A, lda, sa, ipiv, info, batch, st);
+  lu_panel_kernel<<<batch, LU_PANEL_THREADS, 0, st>>>(n, j0, jb, A, lda, sa, ipiv, info);
   EUV_LAUNCH_CHECK();
   return EUV_OK;
 }
@@ -473,6 +517,7 @@ static int lu_update(int n, int j0, int jb, int c0, int nc, double2* A, long lon
       jb, nc, 1, A + j0 + (long long)j0 * lda, lda, sa, A + j0 + (long long)c0 * lda, lda, sa);
   EUV_LAUNCH_CHECK();
   const int rest = n - j0 - jb;
+  if (rest <= 0) return EUV_OK;
   return zgemm_sub(rest, nc, jb, A + (j0 + jb) + (long long)j0 * lda, lda, sa,
                    A + j0 + (long long)c0 * lda, lda, sa, A + (j0 + jb) + (long long)c0 * lda,
                    lda, sa, batch, st);
@@ -483,8 +528,14 @@ static int lu_update(int n, int j0, int jb, int c0, int nc, double2* A, long lon
 // high-priority side stream (its batch CTAs take SMs as soon as any frees up)
 // while the update of the remaining columns runs on the caller's stream.  The
 // column sets are disjoint; the laswp of the next panel waits for both.
+// extra: columns n .. n + extra - 1 of A are right-hand sides, which every step
+// swaps and updates with the trailing columns: they end as L^-1 P B (lu_back
+// finishes them).  The forward substitution so rides in launches that are there
+// anyway, most of it under the panel chain (B200, image calls, with the blocked
+// backward pass above N = 1562: 2048 nm, eight slices, 61.7 -> 53.4 ms; M3D at N =
+// 2121 44.0 -> 38.1 ms; 24 units of N = 625 6.50 -> 6.23 ms).
 int lu_factor(int n, double2* A, long long lda, long long sa, int* ipiv, int* info, int batch,
-              cudaStream_t stream) {
+              cudaStream_t stream, int extra) {
   if (n <= 0 || batch <= 0) return EUV_OK;
   LuSide* side = nullptr;
   EUV_CUDA_TRY(lu_side(&side));
@@ -494,12 +545,15 @@ int lu_factor(int n, double2* A, long long lda, long long sa, int* ipiv, int* in
   int rc = lu_panel(n, j0, jb, A, lda, sa, ipiv, info, batch, stream);
   if (rc) return rc;
   for (;;) {
-    dim3 gs((n + 127) / 128, batch);
-    lu_laswp_kernel<<<gs, 128, 0, stream>>>(n, n, j0, jb, j0, j0 + jb, A, lda, sa, ipiv, n, panel_sub(n, j0));
+    dim3 gs((n + extra + 127) / 128, batch);
+    lu_laswp_kernel<<<gs, 128, 0, stream>>>(n, n + extra, j0, jb, j0, j0 + jb, A, lda, sa, ipiv, n, panel_sub(n, j0));
     EUV_LAUNCH_CHECK();
     const int rest = n - j0 - jb;
-    if (rest <= 0) break;
-    const int j1 = j0 + jb, nb2 = rest < LU_NB ? rest : LU_NB, rem = rest - nb2;
+    if (rest <= 0) {
+      if ((rc = lu_update(n, j0, jb, n, extra, A, lda, sa, batch, stream))) return rc;
+      break;
+    }
+    const int j1 = j0 + jb, nb2 = rest < LU_NB ? rest : LU_NB, rem = rest - nb2 + extra;
     if ((rc = lu_update(n, j0, jb, j1, nb2, A, lda, sa, batch, stream))) return rc;
     if (rem > 0) {
       EUV_CUDA_TRY(cudaEventRecord(side->fork, stream));
@@ -638,7 +692,8 @@ __device__ __forceinline__ void update_rows(double2* xs, int n, const double2* L
   }
 }
 
-template <int RC>
+// BACK: the forward half is done (lu_factor's extra columns), U x = y only.
+template <int RC, bool BACK>
 __global__ void __launch_bounds__(LS_THREADS) lu_subst_kernel(int n, int nrhs, const double2* LU,
                                                               long long lda, long long sa,
                                                               double2* B, long long ldb,
@@ -659,7 +714,8 @@ __global__ void __launch_bounds__(LS_THREADS) lu_subst_kernel(int n, int nrhs, c
   B += (long long)b * sb;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   DiagPrefetch pf;
-  pf.load(LU, lda, 0, n < LS_BLK ? n : LS_BLK, tid);
+  const int jl = ((n - 1) / LS_BLK) * LS_BLK;  // last diagonal block
+  pf.load(LU, lda, BACK ? jl : 0, BACK ? n - jl : (n < LS_BLK ? n : LS_BLK), tid);
   for (int i = tid; i < RC * n; i += LS_THREADS) {
     const int c = i / n, r = i - c * n;
     xs[i] = c < nc ? B[r + (long long)(c0 + c) * ldb] : make_double2(0.0, 0.0);
@@ -667,7 +723,7 @@ __global__ void __launch_bounds__(LS_THREADS) lu_subst_kernel(int n, int nrhs, c
   pf.store(ds, tid);
   __syncthreads();
   // ---- forward: L y = b
-  for (int j0 = 0; j0 < n; j0 += LS_BLK) {
+  for (int j0 = 0; !BACK && j0 < n; j0 += LS_BLK) {
     const int jb = (n - j0) < LS_BLK ? (n - j0) : LS_BLK;
     if (warp < nc) {
       double2* xc = xs + (long long)warp * n + j0;
@@ -681,20 +737,20 @@ __global__ void __launch_bounds__(LS_THREADS) lu_subst_kernel(int n, int nrhs, c
     }
     __syncthreads();
     // next diagonal block: the forward pass's successor, or the backward pass's first
-    const int jn = j0 + LS_BLK < n ? j0 + LS_BLK : ((n - 1) / LS_BLK) * LS_BLK;
+    const int jn = j0 + LS_BLK < n ? j0 + LS_BLK : jl;
     pf.load(LU, lda, jn, (n - jn) < LS_BLK ? (n - jn) : LS_BLK, tid);
     update_rows<RC>(xs, n, LU, lda, j0, jb, j0 + jb, n, tid);
     pf.store(ds, tid);
     __syncthreads();
   }
   // ---- backward: U x = y
-  for (int j0 = ((n - 1) / LS_BLK) * LS_BLK; j0 >= 0; j0 -= LS_BLK) {
+  for (int j0 = jl; j0 >= 0; j0 -= LS_BLK) {
     const int jb = (n - j0) < LS_BLK ? (n - j0) : LS_BLK;
     if (warp < nc) {
       double2* xc = xs + (long long)warp * n + j0;
       cplx x = lane < jb ? ld2(&xc[lane]) : mk(0.0, 0.0);
       // each lane's reciprocal pivot, off the serial chain below
-      const cplx rinv = lane < jb ? cdiv(mk(1.0, 0.0), ld2(&ds[lane][lane])) : mk(0.0, 0.0);
+      const cplx rinv = lane < jb ? crecip(ld2(&ds[lane][lane])) : mk(0.0, 0.0);
 #pragma unroll
       for (int q = LS_BLK - 1; q >= 0; --q) {
         if (q < jb) {  // warp-uniform
@@ -717,17 +773,90 @@ __global__ void __launch_bounds__(LS_THREADS) lu_subst_kernel(int n, int nrhs, c
   }
 }
 
-template <int RC>
+template <int RC, bool BACK>
 static int launch_subst(int n, int nrhs, const double2* LU, long long lda, long long sa,
                         double2* B, long long ldb, long long sb, int batch, const int* order,
                         long long ostride, cudaStream_t stream) {
   static int smem_done[64];
   const int smem = (int)((size_t)RC * n * sizeof(double2));
-  EUV_CUDA_TRY(ensure_smem(lu_subst_kernel<RC>, smem, smem_done));
+  EUV_CUDA_TRY(ensure_smem(lu_subst_kernel<RC, BACK>, smem, smem_done));
   dim3 grid((nrhs + RC - 1) / RC, batch);
-  lu_subst_kernel<RC><<<grid, LS_THREADS, smem, stream>>>(n, nrhs, LU, lda, sa, B, ldb, sb, order,
+  lu_subst_kernel<RC, BACK><<<grid, LS_THREADS, smem, stream>>>(n, nrhs, LU, lda, sa, B, ldb, sb, order,
                                                           ostride);
   EUV_LAUNCH_CHECK();
+  return EUV_OK;
+}
+
+// Right-hand sides per CTA of the one-launch solve, 0 where one column of X does
+// not fit shared memory (or the batch the grid).  12 instead of 8 where that takes
+// fewer waves (one CTA per SM either way: the resident columns fill its shared
+// memory), or where the tuning table says so.
+static int subst_columns(int n, int nrhs, int batch, bool slots, int* rc) {
+  *rc = 0;
+  if (batch > 65535) return EUV_OK;
+  const size_t col = (size_t)n * sizeof(double2);
+  if (12 * col <= LS_SMEM_MAX && nrhs >= 12) {
+    const int tuned = tune_lookup(EUV_KNOB_LU_SUBST_COLS, n, batch);
+    bool twelve = tuned == 12;
+    if (tuned == 0) {
+      int sms = 0, dev = 0;
+      EUV_CUDA_TRY(cudaGetDevice(&dev));
+      EUV_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      const long long w8 = ((long long)((nrhs + 7) / 8) * batch + sms - 1) / sms;
+      const long long w12 = ((long long)((nrhs + 11) / 12) * batch + sms - 1) / sms;
+      // with empty source slots skipped the launch holds fewer live CTAs than
+      // its grid, so a tie in waves goes to 12 (measured: 24 units of N = 961,
+      // 96 slots for families of 96, 92 and 12 sources, step 25.35 -> 24.97 ms)
+      twelve = sms > 0 && (w12 < w8 || (slots && w12 == w8));
+    }
+    if (twelve) {
+      *rc = 12;
+      return EUV_OK;
+    }
+  }
+  for (int r = 8; r >= 1; r >>= 1)
+    if (r * col <= LS_SMEM_MAX && nrhs >= r) {
+      *rc = r;
+      return EUV_OK;
+    }
+  return EUV_OK;
+}
+
+// The one-launch solve needs eight columns per CTA to run on the FP64 tensor path;
+// above N = 1562 fewer fit, and every CTA streams the factor for four or two columns
+// (B200, four units of N = 1681, 380 columns: 10.5 -> 3.8 ms).  A handful of
+// columns takes one launch anyway.
+static bool subst_pays(int cols, int nrhs) { return cols >= 8 || (cols > 0 && nrhs <= 8); }
+
+template <bool BACK>
+static int subst(int rc, int n, int nrhs, const double2* LU, long long lda, long long sa, double2* B,
+                 long long ldb, long long sb, int batch, const int* order, long long ostride,
+                 cudaStream_t stream) {
+  switch (rc) {
+    case 12: return launch_subst<12, BACK>(n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
+    case 8: return launch_subst<8, BACK>(n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
+    case 4: return launch_subst<4, BACK>(n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
+    case 2: return launch_subst<2, BACK>(n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
+    default: return launch_subst<1, BACK>(n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
+  }
+}
+
+// U X = Y or (lower) L Y = B by blocks of LU_NB rows, two launches each.
+static int blocked_solve(bool lower, int n, int nrhs, const double2* LU, long long lda, long long sa,
+                         double2* B, long long ldb, long long sb, int batch, cudaStream_t stream) {
+  const int nblk = (n + LU_NB - 1) / LU_NB;
+  for (int k = 0; k < nblk; ++k) {
+    const int j0 = (lower ? k : nblk - 1 - k) * LU_NB, jb = (n - j0) < LU_NB ? (n - j0) : LU_NB;
+    lu_trsm_warp_kernel<<<trsm_grid(nrhs, batch), 32 * LU_TRSM_WARPS, 0, stream>>>(
+        jb, nrhs, lower ? 1 : 0, LU + j0 + (long long)j0 * lda, lda, sa, B + j0, ldb, sb);
+    EUV_LAUNCH_CHECK();
+    const int r0 = lower ? j0 + jb : 0, rows = lower ? n - r0 : j0;
+    if (rows > 0) {
+      const int rc = zgemm_sub(rows, nrhs, jb, LU + r0 + (long long)j0 * lda, lda, sa, B + j0, ldb, sb,
+                               B + r0, ldb, sb, batch, stream);
+      if (rc != EUV_OK) return rc;
+    }
+  }
   return EUV_OK;
 }
 
@@ -738,66 +867,26 @@ int lu_solve(int n, int nrhs, const double2* LU, long long lda, long long sa, co
   dim3 gs((nrhs + 127) / 128, batch);
   lu_laswp_kernel<<<gs, 128, 0, stream>>>(n, nrhs, 0, n, 0, 0, B, ldb, sb, ipiv, n, 0);
   EUV_LAUNCH_CHECK();
-  if (batch <= 65535) {
-    const size_t col = (size_t)n * sizeof(double2);
-    // 12 right-hand sides per CTA where that takes fewer waves than 8 (one CTA
-    // per SM either way: the resident columns fill its shared memory), or where
-    // the tuning table says so
-    if (12 * col <= LS_SMEM_MAX && nrhs >= 12) {
-      const int tuned = tune_lookup(EUV_KNOB_LU_SUBST_COLS, n, batch);
-      bool twelve = tuned == 12;
-      if (tuned == 0) {
-        int sms = 0, dev = 0;
-        EUV_CUDA_TRY(cudaGetDevice(&dev));
-        EUV_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const long long w8 = ((long long)((nrhs + 7) / 8) * batch + sms - 1) / sms;
-        const long long w12 = ((long long)((nrhs + 11) / 12) * batch + sms - 1) / sms;
-        // with empty source slots skipped the launch holds fewer live CTAs than
-        // its grid, so a tie in waves goes to 12 (measured: 24 units of N = 961,
-        // 96 slots for families of 96, 92 and 12 sources, step 25.35 -> 24.97 ms)
-        twelve = sms > 0 && (w12 < w8 || (order != nullptr && w12 == w8));
-      }
-      if (twelve)
-        return launch_subst<12>(n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
-    }
-    if (8 * col <= LS_SMEM_MAX && nrhs >= 8)
-      return launch_subst<8>(n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
-    if (4 * col <= LS_SMEM_MAX && nrhs >= 4)
-      return launch_subst<4>(n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
-    if (2 * col <= LS_SMEM_MAX && nrhs >= 2)
-      return launch_subst<2>(n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
-    if (col <= LS_SMEM_MAX)
-      return launch_subst<1>(n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
-  }
-  // n too large for one column of X in shared memory: blocked trsm + GEMM
-  // forward: L y = b (unit lower)
-  for (int j0 = 0; j0 < n; j0 += LU_NB) {
-    const int jb = (n - j0) < LU_NB ? (n - j0) : LU_NB;
-    lu_trsm_block_kernel<<<gs, 128, 0, stream>>>(jb, nrhs, 1, LU + j0 + (long long)j0 * lda, lda,
-                                                  sa, B + j0, ldb, sb);
-    EUV_LAUNCH_CHECK();
-    const int rest = n - j0 - jb;
-    if (rest > 0) {
-      int rc = zgemm_sub(rest, nrhs, jb, LU + (j0 + jb) + (long long)j0 * lda, lda, sa, B + j0,
-                         ldb, sb, B + j0 + jb, ldb, sb, batch, stream);
-      if (rc != EUV_OK) return rc;
-    }
-  }
-  // backward: U x = y
-  const int nblk = (n + LU_NB - 1) / LU_NB;
-  for (int bi = nblk - 1; bi >= 0; --bi) {
-    const int j0 = bi * LU_NB;
-    const int jb = (n - j0) < LU_NB ? (n - j0) : LU_NB;
-    lu_trsm_block_kernel<<<gs, 128, 0, stream>>>(jb, nrhs, 0, LU + j0 + (long long)j0 * lda, lda,
-                                                  sa, B + j0, ldb, sb);
-    EUV_LAUNCH_CHECK();
-    if (j0 > 0) {
-      int rc = zgemm_sub(j0, nrhs, jb, LU + (long long)j0 * lda, lda, sa, B + j0, ldb, sb, B,
-                         ldb, sb, batch, stream);
-      if (rc != EUV_OK) return rc;
-    }
-  }
-  return EUV_OK;
+  int cols = 0;
+  int rc = subst_columns(n, nrhs, batch, order != nullptr, &cols);
+  if (rc) return rc;
+  if (subst_pays(cols, nrhs))
+    return subst<false>(cols, n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
+  if ((rc = blocked_solve(true, n, nrhs, LU, lda, sa, B, ldb, sb, batch, stream))) return rc;
+  return blocked_solve(false, n, nrhs, LU, lda, sa, B, ldb, sb, batch, stream);
+}
+
+// U X = Y for columns that lu_factor carried along.
+int lu_back(int n, int nrhs, const double2* LU, long long lda, long long sa, double2* B,
+            long long ldb, long long sb, int batch, cudaStream_t stream, const int* order,
+            long long ostride) {
+  if (n <= 0 || nrhs <= 0 || batch <= 0) return EUV_OK;
+  int cols = 0;
+  const int rc = subst_columns(n, nrhs, batch, order != nullptr, &cols);
+  if (rc) return rc;
+  if (subst_pays(cols, nrhs))
+    return subst<true>(cols, n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
+  return blocked_solve(false, n, nrhs, LU, lda, sa, B, ldb, sb, batch, stream);
 }
 
 }  // namespace euv
@@ -815,7 +904,7 @@ extern "C" int euv_lu_factor(int n, euv_c64* d_a, int lda, long long stride_a, i
     return EUV_ERR_BAD_ARG;
   }
   return euv::lu_factor(n, reinterpret_cast<double2*>(d_a), lda, stride_a, d_ipiv, d_info, batch,
-                        (cudaStream_t)stream);
+                        (cudaStream_t)stream, 0);
 }
 
 extern "C" int euv_lu_solve(int n, int nrhs, const euv_c64* d_lu, int lda, long long stride_a,

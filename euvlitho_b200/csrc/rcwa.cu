@@ -32,8 +32,12 @@ int zgemm(int m, int n, int k, cplx alpha, const double* scale, const double2* a
           long long sa, const double2* b, long long ldb, long long sb, cplx beta, double2* c,
           long long ldc, long long sc, cplx diag, int batch, const int* steps, int step,
           cudaStream_t stream, const GemmTerms& terms = GemmTerms{});
+// extra: right-hand sides in the columns after A's (L^-1 P B on return, for lu_back)
 int lu_factor(int n, double2* A, long long lda, long long sa, int* ipiv, int* info, int batch,
-              cudaStream_t stream);
+              cudaStream_t stream, int extra = 0);
+int lu_back(int n, int nrhs, const double2* LU, long long lda, long long sa, double2* B,
+            long long ldb, long long sb, int batch, cudaStream_t stream, const int* order,
+            long long ostride);
 // order (optional): per batch entry, ostride ints whose first nrhs mark the
 // right-hand sides; a CTA whose columns are all < 0 (zero columns) is skipped
 int lu_solve(int n, int nrhs, const double2* LU, long long lda, long long sa, const int* ipiv,
@@ -836,14 +840,15 @@ __global__ void source_rows_kernel(int n, int nsrc, const int* src_order, const 
                                    const double2* C, const double2* S, long long sc,
                                    const double2* V, const double2* W, long long sw,
                                    const double2* P, const double2* Q, long long sp, double2* V2,
-                                   double2* W2, double2* rhs) {
+                                   double2* W2, double2* rhs, long long sr) {
   const int b = blockIdx.z, s = blockIdx.x;
   const int i = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int o = src_order[(long long)b * nsrc + s];
   const long long t = ((long long)b * nsrc + s) * n + i;
+  double2* r_out = rhs + b * sr + (long long)s * n + i;
   if (o < 0) {
-    V2[t] = W2[t] = rhs[t] = make_double2(0.0, 0.0);
+    V2[t] = W2[t] = *r_out = make_double2(0.0, 0.0);
     return;
   }
   const long long e = (long long)o * n + i;
@@ -863,7 +868,7 @@ __global__ void source_rows_kernel(int n, int nsrc, const int* src_order, const 
   }
   V2[t] = make_double2(vv.x - 2.0 * kl * sv.y, vv.y + 2.0 * kl * sv.x);
   W2[t] = make_double2(w2.x, w2.y);
-  rhs[t] = make_double2(-r.x, -r.y);
+  *r_out = make_double2(-r.x, -r.y);
 }
 
 // Bottom of several slices (Q = I): what of P c + i D s and c + i P s is not a
@@ -893,9 +898,9 @@ __global__ void bottom_rows_kernel(int n, const double2* shift, const double* ra
 
 // Ax[b](i,s) = r x + (1 - r) [i == src_order], r = src_2kz / (2 klm): x is the
 // reflected amplitude of a unit wave in order src_order, the caller's 2 kz its
-// weight (header.h:1394-1465); zero for empty slots.  In place.
+// weight (header.h:1394-1465); zero for empty slots.
 __global__ void ax_out_kernel(int n, int nsrc, const int* src_order, const double* src_2kz,
-                              const double* klm, double2* ax) {
+                              const double* klm, const double2* x, long long sx, double2* ax) {
   const int b = blockIdx.z, s = blockIdx.x;
   const int i = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -906,7 +911,7 @@ __global__ void ax_out_kernel(int n, int nsrc, const int* src_order, const doubl
     return;
   }
   const double r = src_2kz[bs] / (2.0 * klm[(long long)b * n + o]);
-  double2 v = ax[bs * n + i];
+  double2 v = x[b * sx + (long long)s * n + i];
   v.x = r * v.x + (i == o ? 1.0 - r : 0.0);
   v.y = r * v.y;
   ax[bs * n + i] = v;
@@ -1423,7 +1428,11 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
       const int ns = d->n_src;
       const Mat V = pw[1], W = pw[2], M = pw[3];  // the powers above E are free now
       const long long sn = (long long)N * ns;
-      const Mat V2{w.V2, sn}, W2{w.W2, sn}, ax{reinterpret_cast<double2*>(d_ax), sn};
+      // the right-hand sides stand behind M's columns (in the next two buffers), so
+      // that the factorisation carries them along; more than fit are solved apart
+      const bool behind = ns <= 2 * N;
+      const Mat V2{w.V2, sn}, W2{w.W2, sn};
+      const Mat ax = behind ? pw[4] : Mat{reinterpret_cast<double2*>(d_ax), sn};
       const double2* Qp = bottom ? nullptr : Q.p;
       if ((rc = mul(pi_, rad, E, S, zero, W, 0))) return rc;
       top_rows_kernel<<<gdg, bs, 0, stream>>>(N, w.klm, ia, rad, c0, s0, C.p, S.p, C.s, E.p, V.p,
@@ -1433,7 +1442,7 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
       if (ns > 0) {
         source_rows_kernel<<<gs, bs, 0, stream>>>(N, ns, d->d_src_order, w.klm, ia, c0, s0, C.p, S.p,
                                                   C.s, V.p, W.p, V.s, P.p, Qp, P.s, V2.p, W2.p,
-                                                  ax.p);
+                                                  ax.p, ax.s);
         EUV_LAUNCH_CHECK();
       }
       if ((rc = mul(one, nullptr, P, V, one, M, 0))) return rc;
@@ -1442,14 +1451,17 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
         if ((rc = mul(one, nullptr, Q, W, one, M, 0))) return rc;
         if (ns > 0 && (rc = mul(m1, nullptr, Q, W2, one, ax, kReuseA, Term{}, ns))) return rc;
       }
-      if ((rc = lu_factor(N, M.p, N, M.s, w.ipiv, w.info, U, stream))) return rc;
+      if ((rc = lu_factor(N, M.p, N, M.s, w.ipiv, w.info, U, stream, behind ? ns : 0))) return rc;
       flag_singular_kernel<<<grid1(U, 256), 256, 0, stream>>>(w.info, U, status);
       EUV_LAUNCH_CHECK();
       if (ns > 0) {
         // empty source slots (order < 0, zero columns) skip their CTAs
-        if ((rc = lu_solve(N, ns, M.p, N, M.s, w.ipiv, ax.p, N, sn, U, stream, d->d_src_order, ns)))
+        if ((rc = behind ? lu_back(N, ns, M.p, N, M.s, ax.p, N, ax.s, U, stream, d->d_src_order, ns)
+                         : lu_solve(N, ns, M.p, N, M.s, w.ipiv, ax.p, N, ax.s, U, stream,
+                                    d->d_src_order, ns)))
           return rc;
-        ax_out_kernel<<<gs, bs, 0, stream>>>(N, ns, d->d_src_order, d->d_src_2kz, w.klm, ax.p);
+        ax_out_kernel<<<gs, bs, 0, stream>>>(N, ns, d->d_src_order, d->d_src_2kz, w.klm, ax.p, ax.s,
+                                             reinterpret_cast<double2*>(d_ax));
         EUV_LAUNCH_CHECK();
       }
       return EUV_OK;
