@@ -24,6 +24,9 @@
 #include <stdio.h>
 #include <string.h>
 #include <math.h>
+
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace euv {
@@ -62,144 +65,200 @@ inline double theta_for(int precision) {
 constexpr int kMaxSteps = 40;
 
 // ---------------------------------------------------------------- mask DFT
-// The indicator of pattern pixel (x, y), x < FX, y < FY (header.h:1153-1166):
-// the mask bit of column x / meshx and row NDIVY-1 - y / meshy + y_offset
-// (rows outside the mask read as absorber), inverted unless select_vacuum.
-__device__ __forceinline__ double mask_indicator(const uint8_t* bits, int ndivx, int ndivy,
-                                                 int meshx, int meshy, int select_vacuum,
-                                                 int y_offset, int x, int y) {
-  const int ii = x / meshx;
-  const int jj = ndivy - 1 - y / meshy + y_offset;
-  int b = 0;
-  if (jj >= 0 && jj < ndivy) {
-    const long long bit = (long long)ndivx * jj + ii;
-    b = (bits[bit >> 3] >> (7 - (int)(bit & 7))) & 1;
+// Separable DFT of the vacuum indicator V (the mask bits; the absorber's is
+// delta - F_V), frequencies l in [-lh, lh], m in [-mh, mh].  V is real, so only
+// l >= 0 is summed and F(-l, -m) = conj F(l, m).  Mask row jj carries the pattern
+// rows y = meshy (ndivy - 1 - jj + y_offset) + r (header.h:1153-1166; rows outside
+// the mask read as absorber, rows past the grid drop out), so both stages run
+// over mask pixels:
+//   T(l, jj) = sum_ii V(ii, jj) Wx(ii, l),   F(l, m) = sum_jj T(l, jj) Wy(jj, m),
+// Wx, Wy the twiddles summed over a pixel's mesh.
+// Stage 1 multiplies the bits on the FP64 tensor path: the A fragments of 16 mask
+// rows are decoded from the packed bits in registers, the columns are Re and Im of
+// the l's.  It is bound by the FP64 pipe; the masked adds it replaces waited on
+// shared memory and summed both signs of the frequency (B200, this stage: two 1024
+// nm masks, 25 x 25 frequencies, 170 -> 23 us; sixteen 2048 nm masks, 81 x 81, 2.92
+// -> 0.74 ms).
+constexpr int SP_ROWS = 128, SP_K = 32, SP_CL = 8;
+
+// Wx[ii][2 (lh + 1)]: Re, Im of sum_r exp(-2 pi i l (meshx ii + r) / fx) / (fx fy)
+__global__ void spectrum_wx_kernel(int ndivx, int meshx, int fx, double scale, int lh, double* W) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= ndivx * (lh + 1)) return;
+  const int l = t % (lh + 1), ii = t / (lh + 1);
+  double re = 0.0, im = 0.0;
+  for (int r = 0; r < meshx; ++r) {
+    const long long q = ((long long)l * (meshx * ii + r)) % fx;
+    double s, c;
+    sincospi(-2.0 * (double)q / (double)fx, &s, &c);
+    re += c;
+    im += s;
   }
-  return select_vacuum ? (double)b : (double)(1 - b);
+  W[2 * t] = scale * re;
+  W[2 * t + 1] = scale * im;
+}
+// Wy[m' + mr jj] = sum over the pattern rows of mask row jj of exp(-2 pi i m y / fy)
+__global__ void spectrum_wy_kernel(int ndivy, int meshy, int fy, int y_offset, int mh, double2* W) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, mr = 2 * mh + 1;
+  if (t >= ndivy * mr) return;
+  const int m = t % mr - mh, jj = t / mr;
+  double re = 0.0, im = 0.0;
+  for (int r = 0; r < meshy; ++r) {
+    const int y = meshy * (ndivy - 1 - jj + y_offset) + r;
+    if (y < 0 || y >= fy) continue;
+    long long q = ((long long)m * y) % fy;
+    if (q < 0) q += fy;
+    double s, c;
+    sincospi(-2.0 * (double)q / (double)fy, &s, &c);
+    re += c;
+    im += s;
+  }
+  W[t] = make_double2(re, im);
 }
 
-// Stage 1 of the separable DFT, straight from the packed bits:
-//   T[g][m'][x] = sum_y IND_g(x, y) Wy[y + FY m']        (x contiguous)
-// CTA tile: 32 x-columns (lanes) x 64 frequencies (8 warps x 8) for one mask,
-// y streamed through shared memory in chunks of 32.  The indicator is 0/1, so
-// each term is a masked add of a twiddle; one CTA per (x tile, m' tile, mask).
-constexpr int SP_X = 32, SP_M = 64, SP_Y = 32;
-__global__ void __launch_bounds__(256) spectrum_rows_kernel(
-    const uint8_t* bits, long long mask_bytes, int ndivx, int ndivy, int fx, int fy, int mr,
-    int select_vacuum, int y_offset, const double2* Wy, double2* T) {
-  __shared__ double2 ws[SP_Y][SP_M + 1];
-  __shared__ double vs[SP_Y][SP_X];
-  const int g = blockIdx.z;
-  const int x0 = blockIdx.x * SP_X, m0 = blockIdx.y * SP_M;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint8_t* mb = bits + (long long)g * mask_bytes;
-  const int meshx = fx / ndivx, meshy = fy / ndivy;
-  double ar[8], ai[8];
+// The 32 bits from bit `at` on (MSB first, the first bit in bit 31), zero past `end`
+__device__ __forceinline__ unsigned bits32(const uint8_t* mask, long long at, long long end) {
+  if (at >= end) return 0u;
+  const long long b = at >> 3, last = (end + 7) >> 3;
+  unsigned long long v = 0;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) ar[j] = ai[j] = 0.0;
-  for (int y0 = 0; y0 < fy; y0 += SP_Y) {
-    for (int i = threadIdx.x; i < SP_Y * SP_M; i += 256) {
-      const int yy = i % SP_Y, mm = i / SP_Y, y = y0 + yy, m = m0 + mm;
-      ws[yy][mm] = (y < fy && m < mr) ? Wy[y + (long long)fy * m] : make_double2(0.0, 0.0);
+  for (int k = 0; k < 5; ++k) v = (v << 8) | (b + k < last ? mask[b + k] : 0);
+  unsigned w = (unsigned)(v >> (8 - (int)(at & 7)));
+  if (end - at < 32) w &= ~0u << (32 - (int)(end - at));
+  return w;
+}
+
+// Stage 1.  A cluster of 8 CTAs takes 128 rows of one mask and one tile of 8 NB
+// columns; CTA q sums its eighth of the pixels ii, 8 warps with 16 rows each, W
+// staged by 32 pixels; the eight partial sums meet in distributed shared memory.
+template <int NB>
+__global__ void __cluster_dims__(SP_CL, 1, 1) __launch_bounds__(256)
+    spectrum_rows_kernel(const uint8_t* bits, long long mask_bytes, int ndivx, int ndivy, int lh,
+                         const double* W, double2* T) {
+  namespace cg = cooperative_groups;
+  constexpr int ST = NB * 8 + 4;  // doubles per staged pixel: conflict-free fragments
+  cg::cluster_group cluster = cg::this_cluster();
+  const int q = (int)cluster.block_rank();
+  extern __shared__ double2 sm_spec[];
+  double* ws = reinterpret_cast<double*>(sm_spec);  // [2][SP_K][ST], then [SP_ROWS][NB * 8]
+  const int g = blockIdx.z, row0 = (blockIdx.x / SP_CL) * SP_ROWS, c0 = blockIdx.y * NB * 8;
+  const int cols = 2 * (lh + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, fg = lane >> 2, ft = lane & 3;
+  const uint8_t* mask = bits + (long long)g * mask_bytes;
+  // pixels [xa, xb) of this CTA, whole steps of SP_K
+  const int share = ((ndivx + SP_CL - 1) / SP_CL + SP_K - 1) / SP_K * SP_K;
+  const int xa = q * share, xb = min(ndivx, xa + share);
+  const int steps = xb > xa ? (xb - xa + SP_K - 1) / SP_K : 0;
+  auto stage = [&](int k) {
+    double* w = ws + (k & 1) * SP_K * ST;
+    for (int i = tid; i < SP_K * NB * 4; i += 256) {  // pairs of columns: 16-byte copies
+      const int c = 2 * (i % (NB * 4)), x = xa + k * SP_K + i / (NB * 4);
+      const bool ok = x < ndivx && c0 + c < cols;
+      const double* src = ok ? W + (long long)x * cols + c0 + c : W;
+      const unsigned sa = (unsigned)__cvta_generic_to_shared(&w[(i / (NB * 4)) * ST + c]);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(src),
+                   "r"(ok ? 16 : 0)
+                   : "memory");
     }
-    for (int i = threadIdx.x; i < SP_Y * SP_X; i += 256) {
-      const int xx = i % SP_X, yy = i / SP_X, x = x0 + xx, y = y0 + yy;
-      vs[yy][xx] = (x < fx && y < fy)
-                       ? mask_indicator(mb, ndivx, ndivy, meshx, meshy, select_vacuum, y_offset, x, y)
-                       : 0.0;
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  double acc[NB][4];
+#pragma unroll
+  for (int j = 0; j < NB; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[j][e] = 0.0;
+  const int ra = row0 + warp * 16 + fg, rb = ra + 8;
+  if (steps > 0) stage(0);
+  for (int k = 0; k < steps; ++k) {
+    const int x = xa + k * SP_K;
+    const long long at = (long long)ndivx * ra + x, bt = (long long)ndivx * rb + x;
+    const unsigned wa = ra < ndivy ? bits32(mask, at, (long long)ndivx * (ra + 1)) : 0u;
+    const unsigned wb = rb < ndivy ? bits32(mask, bt, (long long)ndivx * (rb + 1)) : 0u;
+    if (k + 1 < steps) {
+      stage(k + 1);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
     __syncthreads();
-#pragma unroll 4
-    for (int yy = 0; yy < SP_Y; ++yy) {
-      const double a = vs[yy][lane];
+    const double* w = ws + (k & 1) * SP_K * ST;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const double2 wv = ws[yy][w + 8 * j];
-        ar[j] = fma(a, wv.x, ar[j]);
-        ai[j] = fma(a, wv.y, ai[j]);
+    for (int s = 0; s < SP_K / 4; ++s) {
+      const int sh = 31 - (4 * s + ft);
+      const double a0 = __hiloint2double((int)((wa >> sh) & 1u) * 0x3ff00000, 0);
+      const double a1 = __hiloint2double((int)((wb >> sh) & 1u) * 0x3ff00000, 0);
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        const double b = w[(4 * s + ft) * ST + 8 * j + fg];
+        asm volatile(
+            "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+            "{%0,%1,%2,%3};\n"
+            : "+d"(acc[j][0]), "+d"(acc[j][1]), "+d"(acc[j][2]), "+d"(acc[j][3])
+            : "d"(a0), "d"(a1), "d"(b));
       }
     }
     __syncthreads();
   }
-  const int x = x0 + lane;
-  if (x >= fx) return;
+  double* red = ws;  // [SP_ROWS][NB * 8]
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int m = m0 + w + 8 * j;
-    if (m < mr) T[((long long)g * mr + m) * fx + x] = make_double2(ar[j], ai[j]);
-  }
-}
-
-// Stage 2:  out[g][l' + LR m'] = sum_x Wx[l' + LR x] T[g][m'][x]
-// One CTA per (m', mask); the T row is staged in shared memory, threads own l'.
-constexpr int SC_THREADS = 64, SC_X = 256;
-__global__ void __launch_bounds__(SC_THREADS) spectrum_cols_kernel(int fx, int lr, int mr,
-                                                                   const double2* Wx,
-                                                                   const double2* T,
-                                                                   double2* out) {
-  __shared__ double2 ts[SC_X];
-  const int m = blockIdx.x, g = blockIdx.y;
-  const double2* t = T + ((long long)g * mr + m) * fx;
-  for (int l0 = 0; l0 < lr; l0 += SC_THREADS) {
-    const int l = l0 + threadIdx.x;
-    double sr = 0.0, si = 0.0;
-    for (int x0 = 0; x0 < fx; x0 += SC_X) {
-      __syncthreads();
-      for (int i = threadIdx.x; i < SC_X; i += SC_THREADS)
-        ts[i] = x0 + i < fx ? t[x0 + i] : make_double2(0.0, 0.0);
-      __syncthreads();
-      if (l < lr) {
-        const int xe = fx - x0 < SC_X ? fx - x0 : SC_X;
-        const double2* wx = Wx + l + (long long)lr * x0;
-#pragma unroll 8
-        for (int xx = 0; xx < xe; ++xx) {
-          const double2 a = wx[(long long)lr * xx], b = ts[xx];
-          sr = fma(a.x, b.x, fma(-a.y, b.y, sr));
-          si = fma(a.x, b.y, fma(a.y, b.x, si));
-        }
-      }
+  for (int j = 0; j < NB; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      red[(warp * 16 + fg + 8 * (e >> 1)) * (NB * 8) + 8 * j + 2 * ft + (e & 1)] = acc[j][e];
+  cluster.sync();
+  // rows 16 q .. 16 q + 15: lanes take consecutive rows
+  for (int i = tid; i < 16 * NB * 4; i += 256) {
+    const int r = 16 * q + i % 16, c = 2 * (i / 16), jj = row0 + r;
+    double2 v = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int t = 0; t < SP_CL; ++t) {
+      const double* p = cluster.map_shared_rank(red, t) + r * (NB * 8) + c;
+      v.x += p[0];
+      v.y += p[1];
     }
-    if (l < lr) out[(long long)g * lr * mr + l + (long long)lr * m] = make_double2(sr, si);
+    if (jj < ndivy && c0 + c < cols)
+      T[((long long)g * (lh + 1) + (c0 + c) / 2) * ndivy + jj] = v;
   }
+  cluster.sync();  // a peer may still read this CTA's sums
+}
+template <int NB>
+constexpr size_t spectrum_smem() {
+  const size_t a = 2 * (size_t)SP_K * (NB * 8 + 4) * sizeof(double);
+  const size_t b = (size_t)SP_ROWS * NB * 8 * sizeof(double);
+  return a > b ? a : b;
 }
 
-// Stage 2 as a split-K DMMA GEMM (out = Wx T^T, K = x in `parts` chunks, one
-// batch entry per chunk): the chunk partial sums, added here.
-__global__ void spectrum_reduce_kernel(const double2* part, int parts, long long total,
-                                       double2* out) {
+// F(l, m) from the K chunks' partial sums P[part][g][l >= 0][m'], both signs of l and,
+// unless select_vacuum, the absorber's spectrum delta - F
+__global__ void spectrum_reduce_kernel(const double2* part, int parts, int masks, int lh, int mh,
+                                       int select_vacuum, double2* out) {
+  const int lr = 2 * lh + 1, mr = 2 * mh + 1;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= total) return;
-  double2 s = part[t];
-  for (int p = 1; p < parts; ++p) {
-    const double2 v = part[(long long)p * total + t];
+  if (t >= (long long)masks * lr * mr) return;
+  const int l = (int)(t % lr) - lh, m = (int)(t / lr % mr) - mh, g = (int)(t / ((long long)lr * mr));
+  const long long total = (long long)masks * (lh + 1) * mr;
+  const bool neg = l < 0;
+  const double2* p = part + ((long long)g * (lh + 1) + (neg ? -l : l)) * mr + (neg ? mh - m : mh + m);
+  double2 s = p[0];
+  for (int k = 1; k < parts; ++k) {
+    const double2 v = p[k * total];
     s.x += v.x;
     s.y += v.y;
+  }
+  if (neg) s.y = -s.y;
+  if (!select_vacuum) {
+    s.x = (l == 0 && m == 0 ? 1.0 : 0.0) - s.x;
+    s.y = -s.y;
   }
   out[t] = s;
 }
 
-// K chunks of stage 2 (0: the per-column kernel): fx / parts a multiple of 64
-static int spectrum_parts(int fx) {
-  if (fx % 64) return 0;
-  int parts = fx / 64 < 16 ? fx / 64 : 16;
-  while ((fx / 64) % parts) --parts;
+// K chunks of stage 2: ndivy / parts a multiple of 64 where that is possible
+static int spectrum_parts(int ndivy) {
+  if (ndivy % 64) return 1;
+  int parts = ndivy / 64 < 16 ? ndivy / 64 : 16;
+  while ((ndivy / 64) % parts) --parts;
   return parts;
-}
-
-// W[r + rows*c] = scale * exp(-2 pi i ((f*g) mod fdiv)/fdiv) with f = r - roff
-// (frequency) and g = c - coff (sample), or transposed roles when `freq_rows`==0.
-__global__ void twiddle_kernel(int rows, int cols, int roff, int coff, int fdiv, int freq_rows,
-                               double scale, double2* W) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)rows * cols) return;
-  int r = (int)(t % rows), c = (int)(t / rows);
-  long long f = freq_rows ? (r - roff) : (c - coff);
-  long long g = freq_rows ? c : r;
-  long long q = (f * g) % fdiv;
-  if (q < 0) q += fdiv;
-  double s, co;
-  sincospi(-2.0 * (double)q / (double)fdiv, &s, &co);
-  W[t] = make_double2(scale * co, scale * s);
 }
 
 // ---------------------------------------------------------------- D and G
@@ -1492,21 +1551,34 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
 // ------------------------------------------------------------------ spectrum
 extern "C" size_t euv_mask_spectrum_workspace_bytes(int n_masks, int ndivx, int ndivy, int fdivx,
                                                     int fdivy, int lh, int mh) {
-  (void)ndivx;
-  (void)ndivy;
-  const size_t lr = 2 * (size_t)lh + 1, mr = 2 * (size_t)mh + 1;
+  (void)fdivx;
+  (void)fdivy;
+  const size_t mr = 2 * (size_t)mh + 1, lp = (size_t)lh + 1;
   Bump bp{nullptr, (size_t)-1, 0, true};
-  bp.take<double2>((size_t)fdivy * mr);
-  bp.take<double2>(lr * (size_t)fdivx);
+  bp.take<double>((size_t)ndivx * 2 * lp);
+  bp.take<double2>((size_t)ndivy * mr);
   const size_t nm = n_masks > 1 ? n_masks : 1;
-  bp.take<double2>(nm * mr * fdivx);
-  bp.take<double2>(nm * (size_t)spectrum_parts(fdivx) * lr * mr);
+  bp.take<double2>(nm * lp * ndivy);
+  bp.take<double2>(nm * (size_t)spectrum_parts(ndivy) * lp * mr);
   bp.take<char>(256);  // the run's alignment slack between the two arrays
   return bp.off;
 }
 
+template <int NB>
+static int launch_spectrum_rows(const uint8_t* bits, long long mask_bytes, int ndivx, int ndivy,
+                                int lh, int tiles, int masks, const double* W, double2* T,
+                                cudaStream_t stream) {
+  static int done[64];
+  constexpr size_t sm = spectrum_smem<NB>();
+  EUV_CUDA_TRY(ensure_smem(spectrum_rows_kernel<NB>, (int)sm, done));
+  const dim3 g(SP_CL * ((ndivy + SP_ROWS - 1) / SP_ROWS), tiles, masks);
+  spectrum_rows_kernel<NB><<<g, 256, sm, stream>>>(bits, mask_bytes, ndivx, ndivy, lh, W, T);
+  EUV_LAUNCH_CHECK();
+  return EUV_OK;
+}
+
 // Masks are transformed in groups that fit the workspace (all of them when it
-// was sized by euv_mask_spectrum_workspace_bytes for n_masks): two launches per
+// was sized by euv_mask_spectrum_workspace_bytes for n_masks): three launches per
 // group after the two twiddle tables.
 extern "C" int euv_mask_spectrum(const uint8_t* d_bits, int n_masks, int ndivx, int ndivy,
                                  int fdivx, int fdivy, int lh, int mh, int select_vacuum,
@@ -1518,52 +1590,60 @@ extern "C" int euv_mask_spectrum(const uint8_t* d_bits, int n_masks, int ndivx, 
     return EUV_ERR_BAD_ARG;
   }
   cudaStream_t stream = (cudaStream_t)stream_;
-  const int lr = 2 * lh + 1, mr = 2 * mh + 1;
+  const int lp = lh + 1, lr = 2 * lh + 1, mr = 2 * mh + 1;
+  const int meshx = fdivx / ndivx, meshy = fdivy / ndivy;
   Bump bp{reinterpret_cast<char*>(d_work), work_bytes, 0, true};
-  double2* Wy = bp.take<double2>((size_t)fdivy * mr);
-  double2* Wx = bp.take<double2>((size_t)lr * fdivx);
-  const int parts = spectrum_parts(fdivx);
-  const size_t t_bytes = (size_t)mr * fdivx * sizeof(double2);
-  const size_t p_bytes = (size_t)parts * lr * mr * sizeof(double2);
+  double* Wx = bp.take<double>((size_t)ndivx * 2 * lp);
+  double2* Wy = bp.take<double2>((size_t)ndivy * mr);
+  const int parts = spectrum_parts(ndivy);
+  const size_t t_bytes = (size_t)lp * ndivy * sizeof(double2);
+  const size_t p_bytes = (size_t)parts * lp * mr * sizeof(double2);
   const size_t left = bp.ok && work_bytes > bp.off + 256 ? work_bytes - bp.off - 256 : 0;
   long long group = (long long)(left / (t_bytes + p_bytes));
-  if (group > 65535) group = 65535;  // grid z / y limit
+  if (group > 65535) group = 65535;  // grid z limit
   if (!d_work || !bp.ok || group < 1) {
     euv_set_error("euv_mask_spectrum: workspace too small");
     return EUV_ERR_WORKSPACE;
   }
   double2* T = reinterpret_cast<double2*>(reinterpret_cast<char*>(d_work) + bp.off);
-  // Wy[y + FY m'] = exp(-2 pi i m y / FY) ; Wx[l' + LR x] = exp(-2 pi i l x/FX)/(FX FY)
-  twiddle_kernel<<<grid1((long long)fdivy * mr, 256), 256, 0, stream>>>(fdivy, mr, 0, mh, fdivy, 0,
-                                                                        1.0, Wy);
+  spectrum_wx_kernel<<<grid1((long long)ndivx * lp, 256), 256, 0, stream>>>(
+      ndivx, meshx, fdivx, 1.0 / ((double)fdivx * (double)fdivy), lh, Wx);
   EUV_LAUNCH_CHECK();
-  twiddle_kernel<<<grid1((long long)lr * fdivx, 256), 256, 0, stream>>>(
-      lr, fdivx, lh, 0, fdivx, 1, 1.0 / ((double)fdivx * (double)fdivy), Wx);
+  spectrum_wy_kernel<<<grid1((long long)ndivy * mr, 256), 256, 0, stream>>>(ndivy, meshy, fdivy,
+                                                                           y_offset, mh, Wy);
   EUV_LAUNCH_CHECK();
   const long long mask_bytes = (long long)ndivx * ndivy / 8;
+  // column tiles of at most eight blocks of 8, as even as they come
+  const int blocks = (2 * lp + 7) / 8, tiles = (blocks + 7) / 8, nb = (blocks + tiles - 1) / tiles;
   for (long long g0 = 0; g0 < n_masks; g0 += group) {
     const int ng = (int)(n_masks - g0 < group ? n_masks - g0 : group);
-    dim3 g1((fdivx + SP_X - 1) / SP_X, (mr + SP_M - 1) / SP_M, ng);
-    spectrum_rows_kernel<<<g1, 256, 0, stream>>>(d_bits + g0 * mask_bytes, mask_bytes, ndivx,
-                                                  ndivy, fdivx, fdivy, mr, select_vacuum,
-                                                  y_offset, Wy, T);
-    EUV_LAUNCH_CHECK();
-    double2* out = reinterpret_cast<double2*>(d_out) + g0 * lr * mr;
-    if (parts > 0) {
-      // out (lr x ng mr) = Wx (lr x FX) T^T (FX x ng mr), K split in `parts` chunks
-      const int kc = fdivx / parts;
-      const long long cols = (long long)ng * mr;
-      double2* P = reinterpret_cast<double2*>(
-          reinterpret_cast<char*>(T) + ((ng * t_bytes + 255) & ~(size_t)255));
-      int rc = zgemm(lr, (int)cols, kc, mk(1.0, 0.0), nullptr, Wx, lr, (long long)kc * lr, T,
-                     fdivx, kc, mk(0.0, 0.0), P, lr, (long long)lr * cols, mk(0.0, 0.0), parts,
-                     nullptr, 0, stream);
-      if (rc) return rc;
-      const long long total = (long long)lr * cols;
-      spectrum_reduce_kernel<<<grid1(total, 256), 256, 0, stream>>>(P, parts, total, out);
-    } else {
-      spectrum_cols_kernel<<<dim3(mr, ng), SC_THREADS, 0, stream>>>(fdivx, lr, mr, Wx, T, out);
+    const uint8_t* b = d_bits + g0 * mask_bytes;
+    int rc = EUV_OK;
+#define EUV_SPECTRUM_CASE(NB) \
+  case NB: rc = launch_spectrum_rows<NB>(b, mask_bytes, ndivx, ndivy, lh, tiles, ng, Wx, T, stream); break
+    switch (nb) {
+      EUV_SPECTRUM_CASE(1);
+      EUV_SPECTRUM_CASE(2);
+      EUV_SPECTRUM_CASE(3);
+      EUV_SPECTRUM_CASE(4);
+      EUV_SPECTRUM_CASE(5);
+      EUV_SPECTRUM_CASE(6);
+      EUV_SPECTRUM_CASE(7);
+      default: rc = launch_spectrum_rows<8>(b, mask_bytes, ndivx, ndivy, lh, tiles, ng, Wx, T, stream);
     }
+#undef EUV_SPECTRUM_CASE
+    if (rc) return rc;
+    // P (mr x ng lp) = Wy (mr x ndivy) T (ndivy x ng lp), K split in `parts` chunks
+    const int kc = ndivy / parts;
+    const long long cols = (long long)ng * lp;
+    double2* P = reinterpret_cast<double2*>(
+        reinterpret_cast<char*>(T) + ((ng * t_bytes + 255) & ~(size_t)255));
+    rc = zgemm(mr, (int)cols, kc, mk(1.0, 0.0), nullptr, Wy, mr, (long long)kc * mr, T, ndivy, kc,
+               mk(0.0, 0.0), P, mr, (long long)mr * cols, mk(0.0, 0.0), parts, nullptr, 0, stream);
+    if (rc) return rc;
+    const long long total = (long long)ng * lr * mr;
+    spectrum_reduce_kernel<<<grid1(total, 256), 256, 0, stream>>>(
+        P, parts, ng, lh, mh, select_vacuum, reinterpret_cast<double2*>(d_out) + g0 * lr * mr);
     EUV_LAUNCH_CHECK();
   }
   return EUV_OK;
