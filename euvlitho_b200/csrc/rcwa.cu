@@ -554,7 +554,7 @@ constexpr int PF_K = 30;       // largest degree (one per lane of a warp)
 constexpr int PF_Q = 6;        // largest q
 constexpr int PF_J = 5;        // largest block count
 constexpr int PF_SAMPLES = 64; // points on the ellipse
-constexpr double kPolyTolFp64 = 1e-16;
+constexpr double kPolyTolFp64 = 1e-15;  // first dropped term; the ones after it fall factorially
 constexpr double kPolyTolMixed = 5e-8;  // the split products carry ~1e-6
 
 struct PolyRegion {
@@ -622,22 +622,35 @@ struct PolyPlan {
   int q, jcap, j, m;  // powers, block limit; blocks and double-angle steps launched
 };
 
-// q from the slab alone (not from the orders or periods, so that clips of
-// different periods share a launch and a unit's arithmetic does not depend on
-// the others): the q with the fewest products at the degrees such slabs need.
-// tau0 = d k |eps - 1| / 4 is the pattern's part of tau.  Mixed (tol 5e-8):
-// 7.5 nm slices take degree 5-6 (q = 3: 4 products), 20-30 nm 7-8 (q = 4: 5),
-// 60 nm 10-11 (q = 5, J = 2..3: 6-8); FP64: 10-12 (q = 5) and 18-20 (q = 6).
-__host__ __device__ inline void poly_shape(int precision, double k, cplx eps_m1, double d, int* q,
-                                           int* jcap) {
-  const double tau0 = 0.25 * d * k * cabs(eps_m1);
-  if (precision == EUV_PREC_MIXED) {
-    *q = tau0 < 0.16 ? 3 : (tau0 < 0.5 ? 4 : 5);
-    *jcap = 4;
-  } else {
-    *q = tau0 < 0.2 ? 5 : 6;
-    *jcap = 5;
+// q, and the block limit.  deg > 0: an estimate of the degree the launch's units
+// need (they share their period), q is the one with the fewest products, then the
+// fewest blocks: degree 11-12 (60 nm slabs of 1 um clips, mixed) takes q = 6, J = 2, 7
+// products, 19 (the same, FP64) q = 5, J = 4, 10.  deg = 0, clips of several periods
+// in one launch: q from the slab alone, so that a unit's arithmetic does not
+// depend on the others; tau0 = d k |eps - 1| / 4 is the pattern's part of tau.  Mixed:
+// 7.5 nm slices need degree 5-6 (q = 3: 4 products), 20-30 nm 7-8 (q = 4: 5), 60 nm
+// 10-12 (q = 5, J = 2..3: 6-8); FP64: 10-12 (q = 5) and 18-20 (q = 6).
+__host__ __device__ inline void poly_shape(int precision, double k, cplx eps_m1, double d, int deg,
+                                           int* q, int* jcap) {
+  *jcap = precision == EUV_PREC_MIXED ? 4 : 5;
+  if (deg > 0) {
+    int best = 1 << 30;
+    for (int c = 3; c <= PF_Q; ++c) {
+      const int j = (deg + c - 1) / c, cost = 8 * (c - 1 + 2 * (j - 1)) + j;
+      if (j <= *jcap && cost < best) {
+        best = cost;
+        *q = c;
+      }
+    }
+    if (best < (1 << 30)) return;
+    *q = PF_Q;  // beyond every q's reach: the longest blocks
+    return;
   }
+  const double tau0 = 0.25 * d * k * cabs(eps_m1);
+  if (precision == EUV_PREC_MIXED)
+    *q = tau0 < 0.16 ? 3 : (tau0 < 0.5 ? 4 : 5);
+  else
+    *q = tau0 < 0.2 ? 5 : 6;
 }
 
 // Blocks and double-angle steps of one unit: the fewest steps with which jcap
@@ -1105,7 +1118,18 @@ static PolyPlan poly_plan(const euv_amp_desc* d, int slice, double tol) {
   const double wx = gx * d->lmax * kx, wy = gy * d->mmax * ky;
   const PolyRegion g = poly_region(d->k, em1, 0.0, kx * kx + ky * ky, leps * (wx > wy ? wx : wy));
   PolyPlan r;
-  poly_shape(d->precision, d->k, em1, d->dabs[slice], &r.q, &r.jcap);
+  int deg = 0;
+  if (!d->d_dx && !d->d_dy) {
+    // degree of a typical unit: incidence along one axis only, and the corners of
+    // the order box only if the set holds them
+    const double lx = gx * d->lmax, ly = gy * d->mmax;
+    const bool box = d->n_orders == (2 * d->lmax + 1) * (2 * d->mmax + 1);
+    const double ax = kx * kx + (box ? ly * ly : 0.0), ay = ky * ky + (box ? lx * lx : 0.0);
+    deg = poly_degree(poly_region(d->k, em1, 0.0, ax > ay ? ax : ay, leps * (wx > wy ? wx : wy)),
+                      d->dabs[slice], tol);
+    if (deg > PF_K) deg = 0;
+  }
+  poly_shape(d->precision, d->k, em1, d->dabs[slice], deg, &r.q, &r.jcap);
   const int limit = d->m_max > 0 && d->m_max < kMaxSteps ? d->m_max : kMaxSteps;
   poly_pick(g, d->dabs[slice], tol, r.q, r.jcap, limit, &r.j, &r.m);
   if (r.m > 0) r.j = r.jcap;  // a unit that needs fewer steps may need all the blocks
