@@ -1025,6 +1025,16 @@ __global__ void flag_singular_kernel(const int* info, int n, int* status) {
 constexpr int kReuseA = 1;
 constexpr int kReuseB = 2;
 
+// Order count up to which the mixed form multiplies in FP64: a product of split
+// planes is three launches of which the two splits and the product's prologue and
+// epilogue are latency (22 us at N = 121), the FP64 one 7-9 us.  By N alone, so that
+// a unit's arithmetic does not depend on the batch: B200, 256 nm clips at N = 121,
+// eight slices, 4 units 2.44 -> 1.34 ms, 16 units 2.53 -> 1.66 ms, 64 units 3.79 ->
+// 4.69 ms; at N = 169 4 units gain as much and 48 lose a third, so the line is drawn
+// below.  Launches of several periods (the served form) are batches by purpose and
+// keep the split planes.
+constexpr int kMixedFp64Orders = 128;
+
 struct Gemm {
   int precision;
   void* mwork;
@@ -1265,7 +1275,8 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
   // device-detected conditions go to the caller's status word, else to a
   // workspace word nobody reads
   int* status = d->d_status ? d->d_status : w.capped;
-  Gemm gemm{d->precision, w.mwork, w.mbytes, stream, status};
+  const bool small = N <= kMixedFp64Orders && !d->d_dx && !d->d_dy;
+  Gemm gemm{small ? EUV_PREC_FP64 : d->precision, w.mwork, w.mbytes, stream, status};
   int rc;
 
   if (!d->d_status) EUV_CUDA_TRY(cudaMemsetAsync(w.capped, 0, sizeof(int), stream));
