@@ -262,29 +262,29 @@ __global__ void cnn_conv1_kernel(int B, const float* x0, const float* w, const f
 
 // ------------------------------------------------------------------ tcgen05 GEMM
 
-// Shared-memory ring of a TF32x3 GEMM: per stage A (hi, lo) 128 x 16 fp32 and
-// B (hi, lo) bn x 16 fp32, 64-byte swizzled K-major.
+// Shared-memory ring of the dense layers' TF32x3 GEMM: per stage the fp32 weight
+// tile 128 x 16 and B (hi, lo) bn x 16 fp32, 64-byte swizzled K-major.
 struct CnnRing {
   uint8_t* base;
   int stage_bytes, b_bytes;
-  __device__ uint8_t* a(int s, int pl) const { return base + s * stage_bytes + pl * CNN_A_TILE; }
+  __device__ uint8_t* a(int s) const { return base + s * stage_bytes; }
   __device__ uint8_t* b(int s, int pl) const {
-    return base + s * stage_bytes + 2 * CNN_A_TILE + pl * b_bytes;
+    return base + s * stage_bytes + CNN_A_TILE + pl * b_bytes;
   }
 };
 
-// hi*hi + hi*lo + lo*hi of one 16-wide K block into the accumulator at tmem
-__device__ __forceinline__ void cnn_mma_block(const CnnRing& r, int s, uint32_t tmem,
+// hi*hi + hi*lo + lo*hi of one 16-wide K block into the accumulator at tmem; the
+// weights' (hi, lo) parts are 16 TMEM columns each at ta
+__device__ __forceinline__ void cnn_mma_block(const CnnRing& r, int s, uint32_t tmem, uint32_t ta,
                                               uint32_t idesc, bool first) {
 #pragma unroll
   for (int k8 = 0; k8 < CNN_BK / 8; ++k8) {
-    const uint64_t ah = umma_desc_sw64(r.a(s, 0) + k8 * 32);
-    const uint64_t al = umma_desc_sw64(r.a(s, 1) + k8 * 32);
+    const uint32_t ah = ta + 8 * k8, al = ah + CNN_BK;
     const uint64_t bh = umma_desc_sw64(r.b(s, 0) + k8 * 32);
     const uint64_t bl = umma_desc_sw64(r.b(s, 1) + k8 * 32);
-    umma_tf32(tmem, ah, bh, idesc, (first && k8 == 0) ? 0u : 1u);
-    umma_tf32(tmem, ah, bl, idesc, 1u);
-    umma_tf32(tmem, al, bh, idesc, 1u);
+    umma_tf32_ta(tmem, ah, bh, idesc, (first && k8 == 0) ? 0u : 1u);
+    umma_tf32_ta(tmem, ah, bl, idesc, 1u);
+    umma_tf32_ta(tmem, al, bh, idesc, 1u);
   }
 }
 
@@ -420,62 +420,64 @@ __global__ void __launch_bounds__(CNN_THREADS) cnn_conv_kernel(
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = idesc_tf32_mn(false, 128, bn);
-      int ia = 0, ib = 0, local = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < p.total_tiles && ok; t += gridDim.x, ++local) {
-        const int ab = local % p.nbuf, use = local / p.nbuf;
-        if (!mbar_wait_bounded(&tempty[ab], (uint32_t)((use & 1) ^ 1), abort_flag, p.err,
-                               CNN_TIMEOUT_NS)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t acc = tmem + (uint32_t)(ab * mt * bn);
-        for (int kx = 0; kx < 3 && ok; ++kx)
-          for (int cc = 0; cc < cchunks && ok; ++cc, ++ia) {
-            const int sa = ia % p.a_stages;
-            if (!mbar_wait_bounded(&afull[sa], (uint32_t)((ia / p.a_stages) & 1), abort_flag,
-                                   p.err, CNN_TIMEOUT_NS)) {
+    const uint32_t idesc = idesc_tf32_mn(false, 128, bn);
+    const bool leader = elect_one();
+    int ia = 0, ib = 0, local = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < p.total_tiles && ok; t += gridDim.x, ++local) {
+      const int ab = local % p.nbuf, use = local / p.nbuf;
+      if (!__all_sync(0xffffffffu,
+                      mbar_wait_bounded(&tempty[ab], (uint32_t)((use & 1) ^ 1), abort_flag,
+                                        p.err, CNN_TIMEOUT_NS))) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      const uint32_t acc = tmem + (uint32_t)(ab * mt * bn);
+      for (int kx = 0; kx < 3 && ok; ++kx)
+        for (int cc = 0; cc < cchunks && ok; ++cc, ++ia) {
+          const int sa = ia % p.a_stages;
+          if (!__all_sync(0xffffffffu,
+                          mbar_wait_bounded(&afull[sa], (uint32_t)((ia / p.a_stages) & 1),
+                                            abort_flag, p.err, CNN_TIMEOUT_NS))) {
+            ok = false;
+            break;
+          }
+          for (int ky = 0; ky < 3; ++ky, ++ib) {
+            const int sb = ib % p.b_stages;
+            if (!__all_sync(0xffffffffu,
+                            mbar_wait_bounded(&bfull[sb], (uint32_t)((ib / p.b_stages) & 1),
+                                              abort_flag, p.err, CNN_TIMEOUT_NS))) {
               ok = false;
               break;
             }
-            for (int ky = 0; ky < 3; ++ky, ++ib) {
-              const int sb = ib % p.b_stages;
-              if (!mbar_wait_bounded(&bfull[sb], (uint32_t)((ib / p.b_stages) & 1), abort_flag,
-                                     p.err, CNN_TIMEOUT_NS)) {
-                ok = false;
-                break;
-              }
-              tc_fence_after();
-              const bool first = kx == 0 && cc == 0 && ky == 0;
-              const uint8_t* bh = b_ring + (sb * 2) * b_plane;
-              const uint8_t* bl = bh + b_plane;
-              for (int m = 0; m < mt; ++m) {
-                // rows (8 m + ky) * 16 .. + 127 of the halo block
-                const uint8_t* ah = a_ring + (sa * 2) * a_plane + (8 * m + ky) * 16 * 64;
-                const uint8_t* al = ah + a_plane;
-                const uint32_t d = acc + (uint32_t)(m * bn);
+            tc_fence_after();
+            const bool first = kx == 0 && cc == 0 && ky == 0;
+            const uint8_t* bh = b_ring + (sb * 2) * b_plane;
+            const uint8_t* bl = bh + b_plane;
+            for (int m = 0; leader && m < mt; ++m) {
+              // rows (8 m + ky) * 16 .. + 127 of the halo block
+              const uint8_t* ah = a_ring + (sa * 2) * a_plane + (8 * m + ky) * 16 * 64;
+              const uint8_t* al = ah + a_plane;
+              const uint32_t d = acc + (uint32_t)(m * bn);
 #pragma unroll
-                for (int k8 = 0; k8 < CNN_BK / 8; ++k8) {
-                  const uint64_t dah = umma_desc_sw64(ah + k8 * 32);
-                  const uint64_t dal = umma_desc_sw64(al + k8 * 32);
-                  const uint64_t dbh = umma_desc_sw64(bh + k8 * 32);
-                  const uint64_t dbl = umma_desc_sw64(bl + k8 * 32);
-                  umma_tf32(d, dah, dbh, idesc, (first && k8 == 0) ? 0u : 1u);
-                  umma_tf32(d, dah, dbl, idesc, 1u);
-                  umma_tf32(d, dal, dbh, idesc, 1u);
-                }
+              for (int k8 = 0; k8 < CNN_BK / 8; ++k8) {
+                const uint64_t dah = umma_desc_sw64(ah + k8 * 32);
+                const uint64_t dal = umma_desc_sw64(al + k8 * 32);
+                const uint64_t dbh = umma_desc_sw64(bh + k8 * 32);
+                const uint64_t dbl = umma_desc_sw64(bl + k8 * 32);
+                umma_tf32(d, dah, dbh, idesc, (first && k8 == 0) ? 0u : 1u);
+                umma_tf32(d, dah, dbl, idesc, 1u);
+                umma_tf32(d, dal, dbh, idesc, 1u);
               }
-              umma_commit(&bempty[sb]);
             }
-            umma_commit(&aempty[sa]);
+            if (leader) umma_commit(&bempty[sb]);
           }
-        if (ok) umma_commit(&tfull[ab]);
-      }
-      umma_commit(done);  // always: teardown waits for the MMAs in flight
+          if (leader) umma_commit(&aempty[sa]);
+        }
+      if (ok && leader) umma_commit(&tfull[ab]);
     }
+    if (leader) umma_commit(done);  // always: teardown waits for the MMAs in flight
   } else {
     const int q = warp & 3;
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
@@ -559,6 +561,14 @@ static CnnConvPlan cnn_conv_plan(int cout, int models) {
   return c;
 }
 
+// TMEM columns of a dense layer: the accumulator's, and all of them
+__host__ __device__ __forceinline__ int cnn_fc_acols(int bn) { return (bn + 31) / 32 * 32; }
+__host__ __device__ __forceinline__ int cnn_fc_tcols(int bn, int stages) {
+  int t = 32;
+  while (t < cnn_fc_acols(bn) + 2 * CNN_BK * stages) t <<= 1;
+  return t;
+}
+
 struct CnnFcArgs {
   int models, batch;
   int bn, nkb, stages;
@@ -570,18 +580,22 @@ struct CnnFcArgs {
 // Split-K fully connected layer: A = fp32 weights [M][rows][K] (128 rows per
 // CTA), B = activation planes [2M][batch][K] (bn masks per CTA), K range
 // split blockIdx.y % nsplit; FP32 partial sums to part[split][model][mask][row].
-// The TMA writes the fp32 weight tile into the stage's hi tile; warps 2..5
-// split it in place (hi) and into the lo tile (same swizzled positions:
-// the transform is elementwise), fence the generic-proxy writes for the
-// tensor core and arrive on conv[s]; the MMA warp waits on conv[s].  After
-// the K loop the same warps run the epilogue.
+// The TMA writes the fp32 weight tile; warps 2..5 split it and store the (hi, lo)
+// parts to the stage's TMEM columns, from where the tensor core reads A.
+// The weights stream from HBM once, which bounds the layer up to about 32 masks.
+// What kept it from that, six networks and one mask (6.9 GB, 1.06 ms at the copy
+// rate): 1.69 ms with the split written back to shared memory, a lane == 0 branch
+// around the issue loop and two CTAs per SM.  A CTA's MMA thread is then a serial
+// chain of about 700 cycles per 8 KB, at any number of stages; the issue loop under
+// elect_one and four CTAs per SM give 1.34 ms, and the split in integer operations
+// (split_tf32f) 1.07.
 __global__ void __launch_bounds__(CNN_THREADS) cnn_fc_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     CnnFcArgs p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  CnnRing ring{smem, 2 * CNN_A_TILE + 2 * p.bn * CNN_BK * 4, p.bn * CNN_BK * 4};
+  CnnRing ring{smem, CNN_A_TILE + 2 * p.bn * CNN_BK * 4, p.bn * CNN_BK * 4};
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.stages * ring.stage_bytes);
   uint64_t* conv = full + p.stages;
   uint64_t* empty = conv + p.stages;
@@ -593,13 +607,12 @@ __global__ void __launch_bounds__(CNN_THREADS) cnn_fc_kernel(
   const int m0 = 128 * blockIdx.x;
   const int split = blockIdx.y % p.nsplit;
   const int n0 = p.bn * (blockIdx.y / p.nsplit);
-  uint32_t tcols = 32;
-  while ((int)tcols < p.bn) tcols <<= 1;
+  const uint32_t tcols = (uint32_t)cnn_fc_tcols(p.bn, p.stages);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&conv[s], 2);
+      mbar_init(&conv[s], 4);
       mbar_init(&empty[s], 1);
     }
     mbar_init(accum, 1);
@@ -611,7 +624,8 @@ __global__ void __launch_bounds__(CNN_THREADS) cnn_fc_kernel(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = *tmem_slot;                        // accumulator, bn columns
+  const uint32_t ta0 = tmem + (uint32_t)cnn_fc_acols(p.bn);  // split weights, 32 per stage
   const int nkb = p.nkb;
 
   if (warp == 0) {
@@ -623,7 +637,7 @@ __global__ void __launch_bounds__(CNN_THREADS) cnn_fc_kernel(
         if (!mbar_wait_bounded(&empty[s], ph ^ 1u, abort_flag, p.err, CNN_TIMEOUT_NS)) break;
         mbar_expect_tx(&full[s], (uint32_t)(CNN_A_TILE + 2 * ring.b_bytes));
         const int k0 = (split * nkb + kb) * CNN_BK;
-        tma_load_3d(ring.a(s, 0), &tmA, k0, m0, model, &full[s]);
+        tma_load_3d(ring.a(s), &tmA, k0, m0, model, &full[s]);
         for (int pl = 0; pl < 2; ++pl)
           tma_load_3d(ring.b(s, pl), &tmB, k0, n0, 2 * model + pl, &full[s]);
         issued = kb + 1;
@@ -634,56 +648,65 @@ __global__ void __launch_bounds__(CNN_THREADS) cnn_fc_kernel(
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = idesc_tf32_mn(false, 128, p.bn);
-      for (int kb = 0; kb < nkb; ++kb) {
-        const int s = kb % p.stages;
-        const uint32_t ph = (uint32_t)((kb / p.stages) & 1);
-        if (!mbar_wait_bounded(&conv[s], ph, abort_flag, p.err, CNN_TIMEOUT_NS)) break;
-        tc_fence_after();
-        cnn_mma_block(ring, s, tmem, idesc, kb == 0);
+    const uint32_t idesc = idesc_tf32_mn(false, 128, p.bn);
+    const bool leader = elect_one();
+    int s = 0;
+    uint32_t ph = 0;
+    for (int kb = 0; kb < nkb; ++kb) {
+      const bool got = mbar_wait_bounded(&conv[s], ph, abort_flag, p.err, CNN_TIMEOUT_NS);
+      if (!__all_sync(0xffffffffu, got)) break;
+      tc_fence_after();
+      if (leader) {
+        cnn_mma_block(ring, s, tmem, ta0 + 2 * CNN_BK * s, idesc, kb == 0);
         umma_commit(&empty[s]);
       }
-      umma_commit(accum);
+      if (++s == p.stages) {
+        s = 0;
+        ph ^= 1u;
+      }
     }
+    if (leader) umma_commit(accum);
   } else {
-    // weight split, 2048 fp32 of a stage's A tile: warps 2-3 take the even K
-    // blocks, warps 4-5 the odd ones (two stages converting at once), 32 per thread
-    const int grp = (warp - 2) >> 1;
-    const int et = threadIdx.x - 64 - 64 * grp;  // 0..63
-    for (int kb = grp; kb < nkb; kb += 2) {
+    // weight split: a row per thread, in the TMEM lanes that the warp can reach
+    const int q = warp & 3;
+    const int r = q * 32 + lane;
+    const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+    for (int kb = 0; kb < nkb; ++kb) {
       const int s = kb % p.stages;
       const uint32_t ph = (uint32_t)((kb / p.stages) & 1);
       const bool got = mbar_wait_bounded(&full[s], ph, abort_flag, p.err, CNN_TIMEOUT_NS);
       if (!__all_sync(0xffffffffu, got)) break;
-      float4* hi = reinterpret_cast<float4*>(ring.a(s, 0));
-      float4* lo = reinterpret_cast<float4*>(ring.a(s, 1));
+      tc_fence_after();
+      const float4* a = reinterpret_cast<const float4*>(ring.a(s)) + 4 * r;
+      uint32_t hi[16], lo[16];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int i = et + 64 * u;
-        const float4 x = hi[i];
-        float4 h, l;
-        split_tf32f(x.x, h.x, l.x);
-        split_tf32f(x.y, h.y, l.y);
-        split_tf32f(x.z, h.z, l.z);
-        split_tf32f(x.w, h.w, l.w);
-        hi[i] = h;
-        lo[i] = l;
+      for (int c = 0; c < 4; ++c) {
+        const float4 x = a[c ^ ((r >> 1) & 3)];  // 64-byte swizzle
+        const float v[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float h, l;
+          split_tf32f(v[e], h, l);
+          hi[4 * c + e] = __float_as_uint(h);
+          lo[4 * c + e] = __float_as_uint(l);
+        }
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      const uint32_t ta = ta0 + lane_addr + 2 * CNN_BK * s;
+      tmem_st16(ta, hi);
+      tmem_st16(ta + CNN_BK, lo);
+      tmem_st_wait();
+      tc_fence_before();
       __syncwarp();
       if (lane == 0)
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&conv[s]))
                      : "memory");
     }
-    const int q = warp & 3;
     const bool waited =
         mbar_wait_bounded(accum, 0u, abort_flag, p.err, CNN_TIMEOUT_NS) && !*abort_flag;
     const bool ok = __all_sync(0xffffffffu, waited);
     tc_fence_after();
-    const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     if (ok) {
-      const int row = m0 + q * 32 + lane;
+      const int row = m0 + r;
       float* part = p.part + ((long long)split * p.models + model) * p.batch * p.rows;
       for (int c0 = 0; c0 < p.bn; c0 += 16) {
         if (n0 + c0 >= p.batch) break;  // warp-uniform
@@ -753,21 +776,31 @@ __global__ void cnn_fc2_finish_kernel(int M, int B, int op, int max_out, CnnOutA
 
 // ------------------------------------------------------------------ host
 
+// CTAs per SM of a dense layer, and the stages that its share of shared memory and
+// TMEM holds.
+// Up to 32 masks four: more issuing warps (one, two, four CTAs: 2.87, 1.72, 1.34 ms for
+// the case above); above that the products bind and the ring needs the columns
+// (one network, 64 masks: 1.93 -> 1.66 ms with two, 256 masks 6.62 -> 5.59 with one).
+static int cnn_fc_ctas(int bn) { return bn <= 32 ? 4 : bn <= 128 ? 2 : 1; }
 static int cnn_stages(int bn) {
-  const int stage = 2 * CNN_A_TILE + 2 * bn * CNN_BK * 4;
-  const int budget = stage <= 24 * 1024 ? 110 * 1024 : 200 * 1024;  // two CTAs / SM when small
-  int s = budget / stage;
-  return s < 2 ? 2 : (s > 6 ? 6 : s);
+  const int n = cnn_fc_ctas(bn);
+  const int m = (224 / n - 3) * 1024 / (CNN_A_TILE + 2 * bn * CNN_BK * 4);
+  const int t = (512 / n - cnn_fc_acols(bn)) / (2 * CNN_BK);
+  return m < t ? m : t;
 }
+// No more CTAs on an SM than its 512 TMEM columns serve: the request is at least the
+// share of 227 KB that excludes one more.
 static size_t cnn_smem(int bn, int stages) {
-  return (size_t)stages * (2 * CNN_A_TILE + 2 * bn * CNN_BK * 4) + 1024 + 256;
+  const size_t ring = (size_t)stages * (CNN_A_TILE + 2 * bn * CNN_BK * 4) + 1024 + 256;
+  const size_t least = (size_t)228 * 1024 / (512 / cnn_fc_tcols(bn, stages) + 1) + 1024;
+  return ring > least ? ring : least;
 }
 
-template <class Kern, class Args>
-static int cnn_launch(Kern kernel, dim3 grid, size_t smem, const CUtensorMap& ta,
-                      const CUtensorMap& tb, const Args& p, cudaStream_t stream, int* done) {
-  EUV_CUDA_TRY(ensure_smem(kernel, (int)smem, done));
-  kernel<<<grid, CNN_THREADS, smem, stream>>>(ta, tb, p);
+static int cnn_fc_launch(dim3 grid, size_t smem, const CUtensorMap& ta, const CUtensorMap& tb,
+                         const CnnFcArgs& p, cudaStream_t stream) {
+  static int done[64];
+  EUV_CUDA_TRY(ensure_smem(cnn_fc_kernel, (int)smem, done));
+  cnn_fc_kernel<<<grid, CNN_THREADS, smem, stream>>>(ta, tb, p);
   EUV_LAUNCH_CHECK();
   return EUV_OK;
 }
@@ -1015,10 +1048,7 @@ extern "C" int euv_cnn_predict(const euv_cnn_desc* d, const uint8_t* d_bits, con
     p.part = work + (f == 0 ? W.part1 : W.part2);
     p.err = err;
     dim3 grid(rows / 128, ntiles * nsplit, M);
-    static int fc_done[64];
-    if ((rc = cnn_launch(cnn_fc_kernel, grid, cnn_smem(bn, p.stages), ta, tb, p, stream,
-                         fc_done)))
-      return rc;
+    if ((rc = cnn_fc_launch(grid, cnn_smem(bn, p.stages), ta, tb, p, stream))) return rc;
     if (f == 0) {
       const long long n = (long long)M * B * CNN_FC1_N;
       cnn_fc1_finish_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(

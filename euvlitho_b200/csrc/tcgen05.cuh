@@ -3,7 +3,7 @@
 // mbarriers with bounded waits, TMA tensor loads, UMMA shared-memory
 // descriptors for 64-byte-swizzled K-major tiles, tcgen05.mma of kind tf32
 // (the CNN; the mixed GEMM issues kind::f16 itself), TMEM loads, the
-// FP64/FP32 -> (hi, lo) TF32 split and the driver's tensor-map encoder.
+// FP32 -> (hi, lo) TF32 split and the driver's tensor-map encoder.
 #pragma once
 #include <cuda.h>
 #include "common.cuh"
@@ -70,6 +70,19 @@ __device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, i
       "r"(smem_u32(bar))
       : "memory");
 }
+// One lane of a converged warp.  An issue loop that all lanes run, with only its
+// tcgen05 instructions under this predicate, keeps descriptors and addresses in
+// uniform registers; under a lane == 0 branch each one is moved there for every
+// instruction, about 70 cycles per tcgen05.mma measured.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
 // K-major operand, 64-byte swizzle: 8-row atoms of 512 B (SBO), version 1.
 __device__ __forceinline__ uint64_t umma_desc_sw64(const void* tile) {
   const uint64_t addr = smem_u32(tile);
@@ -96,6 +109,16 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t da, uint64_t
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
       "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// The same with A in TMEM: 128 lanes x 8 columns at ta.
+__device__ __forceinline__ void umma_tf32_ta(uint32_t tmem_d, uint32_t ta, uint64_t db,
+                                             uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(ta), "l"(db), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -136,6 +159,18 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
         "=r"(r[7])
       : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
+      "%13,%14,%15};" ::"r"(r[0]),
+      "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+      "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+      "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -143,18 +178,16 @@ __device__ __forceinline__ void tmem_ld_wait() {
 // x = hi + lo with hi = x rounded to TF32 (nearest, ties away) and lo the
 // remainder rounded to TF32: hi*hi + hi*lo + lo*hi then carries about 22
 // significant bits of each product.
-__device__ __forceinline__ float tf32_round(float f) {
-  uint32_t h;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(f));
-  return __uint_as_float(h);
-}
-__device__ __forceinline__ void split_tf32(double x, float& hi, float& lo) {
-  hi = tf32_round((float)x);
-  lo = (float)(x - (double)hi);
-}
+// In integer operations: cvt.rna.tf32.f32 costs several of them, which shows where
+// the dense layers split 8 KB of weights in the time that HBM needs to deliver them
+// (one mask, six networks: 1.61 -> 1.33 ms for the whole prediction).
 __device__ __forceinline__ void split_tf32f(float x, float& hi, float& lo) {
-  hi = tf32_round(x);
-  lo = tf32_round(x - hi);  // x - hi is exact in fp32
+  // a carry out of the fraction is the next exponent; what it makes of a NaN is
+  // undone by hi = x - d
+  const float h = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+  const float d = __fsub_rn(x, h);  // exact
+  hi = __fsub_rn(x, d);             // h
+  lo = __uint_as_float((__float_as_uint(d) + 0x1000u) & 0xffffe000u);
 }
 
 // ------------------------------------------------------------------ host

@@ -129,3 +129,44 @@ def test_predict_more_masks_than_one_tile(cuda, models):
     for i in (0, 7, 256, 259):
         err = _rel(got[i], ref[i % 10])
         assert err < TOL, (i, err)
+
+
+@pytest.mark.parametrize("n", [16, 17, 32, 33, 128, 129, 256])
+def test_predict_at_the_edges_of_the_dense_layers_tiles(cuda, models, n):
+    """The dense layers' CTAs per SM change at 32 and 128 masks, their stages and the
+    padding of the mask tile in between: every mask against the FP32 oracle."""
+    facs = O.seeded_factors()
+    pred = cnn.CnnPredictor(O.state_dicts(models[:1]), [facs[0]], cuda)
+    base = rasters(5, 12)
+    got = pred.predict(np.concatenate([base] * (n // 5 + 1))[:n])[0]
+    x = torch.from_numpy(np.stack([O.compmask_bits(r) for r in base])).reshape(-1, 1, 512, 512)
+    prev = (torch.backends.cuda.matmul.allow_tf32, torch.backends.cudnn.allow_tf32)
+    torch.backends.cuda.matmul.allow_tf32 = False
+    torch.backends.cudnn.allow_tf32 = False
+    try:
+        m = models[0].to(cuda)
+        with torch.no_grad():
+            ref = m(x.to(cuda)).double().cpu().numpy() / facs[0]
+        models[0].to("cpu")
+    finally:
+        torch.backends.cuda.matmul.allow_tf32, torch.backends.cudnn.allow_tf32 = prev
+    assert got.shape == (n, O.NCUT)
+    for i in range(n):
+        assert _rel(got[i], ref[i % 5]) < TOL, i
+
+
+@pytest.mark.parametrize("bits", [0x7FC00000, 0x7FFFFFFF, 0xFFFFFFFF - (1 << 32), 0x7F800000])
+def test_weights_that_are_not_numbers(cuda, models, bits):
+    """A NaN (either sign, any payload) or an infinity among the dense weights reaches
+    its own output and no other."""
+    facs = O.seeded_factors()
+    sd = dict(O.state_dicts(models[:1])[0])
+    raw = rasters(2, 13)
+    ref = cnn.CnnPredictor([sd], [facs[0]], cuda).predict(raw)[0]
+    w = sd["fc2.weight"].clone()
+    w[7, 100] = torch.tensor([bits], dtype=torch.int32).view(torch.float32)[0]
+    sd["fc2.weight"] = w
+    got = cnn.CnnPredictor([sd], [facs[0]], cuda).predict(raw)[0]
+    assert not np.isfinite(got[:, 7]).any()
+    rest = np.arange(O.NCUT) != 7
+    np.testing.assert_array_equal(got[:, rest], ref[:, rest])
