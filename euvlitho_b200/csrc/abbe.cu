@@ -390,6 +390,7 @@ constexpr int BD_PT = 8;  // pupil points per thread whose indices are loaded ah
 template <typename R>
 __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(512)
     abbe_band_kernel(AbbeParams p, size_t cap, const double2* ax, double* image) {
+  dependent_begin();
   namespace cg = cooperative_groups;
   using V2 = typename vec2<R>::type;
   using C = cx<R>;
@@ -672,7 +673,8 @@ static int launch_band(const euv_abbe_desc* d, const AbbeParams& p, const double
   const int items = gx / 4 * gy, rounds = (items + 511) / 512;
   int threads = ((items + rounds - 1) / rounds + 31) / 32 * 32;
   if (threads < 128) threads = 128;
-  abbe_band_kernel<R><<<dim3(BD_CL * nc, d->n_units), threads, smem, stream>>>(p, smem, ax, image);
+  EUV_CUDA_TRY(launch_dependent(abbe_band_kernel<R>, dim3(BD_CL * nc, d->n_units), dim3(threads),
+                                smem, stream, p, smem, ax, image));
   EUV_LAUNCH_CHECK();
   return EUV_OK;
 }

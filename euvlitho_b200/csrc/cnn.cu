@@ -216,6 +216,7 @@ __device__ __forceinline__ void cnn_store16(float* hi_base, long long plane, int
 // pixel (py, px) of image blockIdx.y, model blockIdx.z.
 __global__ void cnn_conv1_kernel(int B, const float* x0, const float* w, const float* bias,
                                  const float* scale, const float* shift, float* out) {
+  dependent_begin();
   __shared__ float sw[144], sb[16], ss[16], sh[16];
   const int m = blockIdx.z, img = blockIdx.y;
   for (int i = threadIdx.x; i < 144; i += blockDim.x) sw[i] = w[m * 144 + i];
@@ -316,6 +317,7 @@ __host__ __device__ constexpr int cnn_conv_a_plane(int mt) { return (8 * mt + 2)
 __global__ void __launch_bounds__(CNN_THREADS) cnn_conv_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     CnnConvArgs p) {
+  dependent_begin();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -592,6 +594,7 @@ struct CnnFcArgs {
 __global__ void __launch_bounds__(CNN_THREADS) cnn_fc_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     CnnFcArgs p) {
+  dependent_begin();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -733,6 +736,7 @@ __global__ void __launch_bounds__(CNN_THREADS) cnn_fc_kernel(
 // h = ReLU(sum of fc1 partials + bias) as (hi, lo) planes [M][2][B][4096]
 __global__ void cnn_fc1_finish_kernel(int M, int B, const float* part, const float* bias,
                                       float* h) {
+  dependent_begin();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long n = (long long)M * B * CNN_FC1_N;
   if (t >= n) return;
@@ -757,6 +761,7 @@ struct CnnOutArgs {
 __global__ void cnn_fc2_finish_kernel(int M, int B, int op, int max_out, CnnOutArgs no,
                                       const float* part, const float* bias,
                                       const double* factors, double* out) {
+  dependent_begin();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long n = (long long)M * B * max_out;
   if (t >= n) return;
@@ -800,7 +805,7 @@ static int cnn_fc_launch(dim3 grid, size_t smem, const CUtensorMap& ta, const CU
                          const CnnFcArgs& p, cudaStream_t stream) {
   static int done[64];
   EUV_CUDA_TRY(ensure_smem(cnn_fc_kernel, (int)smem, done));
-  cnn_fc_kernel<<<grid, CNN_THREADS, smem, stream>>>(ta, tb, p);
+  EUV_CUDA_TRY(launch_dependent(cnn_fc_kernel, grid, dim3(CNN_THREADS), smem, stream, ta, tb, p));
   EUV_LAUNCH_CHECK();
   return EUV_OK;
 }
@@ -961,9 +966,9 @@ extern "C" int euv_cnn_predict(const euv_cnn_desc* d, const uint8_t* d_bits, con
     cnn_input_kernel<<<g, 256, 0, stream>>>(d_bits, work + W.x0);
     EUV_LAUNCH_CHECK();
     dim3 g1((CNN_IN / 2) * (CNN_IN / 2) / 256, B, M);
-    cnn_conv1_kernel<<<g1, 256, 0, stream>>>(B, work + W.x0, blob + L.w[0], blob + L.bias[0],
-                                             blob + L.scale[0], blob + L.shift[0],
-                                             work + W.act[0]);
+    EUV_CUDA_TRY(launch_dependent(cnn_conv1_kernel, g1, dim3(256), 0, stream, B, work + W.x0,
+                                  blob + L.w[0], blob + L.bias[0], blob + L.scale[0],
+                                  blob + L.shift[0], work + W.act[0]));
     EUV_LAUNCH_CHECK();
   }
   // conv2..conv5
@@ -1014,7 +1019,8 @@ extern "C" int euv_cnn_predict(const euv_cnn_desc* d, const uint8_t* d_bits, con
       euv_set_error("euv_cnn_predict: conv kernel setup failed");
       return EUV_ERR_CUDA;
     }
-    cnn_conv_kernel<<<grid, CNN_THREADS, smem, stream>>>(ta, tb, p);
+    EUV_CUDA_TRY(launch_dependent(cnn_conv_kernel, grid, dim3(CNN_THREADS), smem, stream, ta, tb,
+                                  p));
     EUV_LAUNCH_CHECK();
   }
   // fc1, fc2: A = weight planes [M*2][rows][K], B = activation planes [M*2][B][K]
@@ -1051,14 +1057,16 @@ extern "C" int euv_cnn_predict(const euv_cnn_desc* d, const uint8_t* d_bits, con
     if ((rc = cnn_fc_launch(grid, cnn_smem(bn, p.stages), ta, tb, p, stream))) return rc;
     if (f == 0) {
       const long long n = (long long)M * B * CNN_FC1_N;
-      cnn_fc1_finish_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(
-          M, B, work + W.part1, blob + L.fc1_b, work + W.h);
+      EUV_CUDA_TRY(launch_dependent(cnn_fc1_finish_kernel, dim3((unsigned)((n + 255) / 256)),
+                                    dim3(256), 0, stream, M, B, work + W.part1, blob + L.fc1_b,
+                                    work + W.h));
     } else {
       CnnOutArgs no;
       for (int m = 0; m < EUV_CNN_MAX_MODELS; ++m) no.n_out[m] = m < M ? d->n_out[m] : 0;
       const long long n = (long long)M * B * d->max_out;
-      cnn_fc2_finish_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(
-          M, B, L.op, d->max_out, no, work + W.part2, blob + L.fc2_b, d->d_factors, d_out);
+      EUV_CUDA_TRY(launch_dependent(cnn_fc2_finish_kernel, dim3((unsigned)((n + 255) / 256)),
+                                    dim3(256), 0, stream, M, B, L.op, d->max_out, no,
+                                    work + W.part2, blob + L.fc2_b, d->d_factors, d_out));
     }
     EUV_LAUNCH_CHECK();
   }

@@ -156,6 +156,7 @@ template <int NX>
 __global__ void __launch_bounds__(MX_THREADS, 1)
     gemm_split3_kernel(const __grid_constant__ CUtensorMap tmA,
                        const __grid_constant__ CUtensorMap tmB, MixedArgs p) {
+  dependent_begin();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -564,6 +565,7 @@ template <int R>
 __global__ void __launch_bounds__(MX_SLAB_THREADS)
     split_a_slab_kernel(int M, int K, int Kp, const double2* A, long long lda, long long sa,
                         __half* out, int* ea, const int* steps, int step) {
+  dependent_begin();
   extern __shared__ double2 slab[];  // [R][Ks]: element (row r, column k) at r * Ks + k
   const int Ks = slab_a_stride<R>(K);
   __shared__ double s_scale[R];
@@ -624,6 +626,7 @@ template <int R>
 __global__ void __launch_bounds__(MX_SLAB_THREADS)
     split_b_slab_kernel(int K, int N, int Kp, const double2* B, long long ldb, long long sb,
                         __half* out, int* eb, const int* steps, int step) {
+  dependent_begin();
   extern __shared__ double2 slab[];  // [R][K]: element (k, column c) at c * K + k
   __shared__ double s_scale[R];
   const int b = blockIdx.y;
@@ -695,12 +698,12 @@ static int launch_split_slab(bool a_role, int rows, int K, int Kp, const double2
   dim3 g((unsigned)((rows + R - 1) / R), batch);
   if (a_role) {
     EUV_CUDA_TRY(ensure_smem(split_a_slab_kernel<R>, smem, done_a));
-    split_a_slab_kernel<R><<<g, MX_SLAB_THREADS, smem, stream>>>(rows, K, Kp, X, ld, st, out, ex,
-                                                                  steps, step);
+    EUV_CUDA_TRY(launch_dependent(split_a_slab_kernel<R>, g, dim3(MX_SLAB_THREADS), smem, stream,
+                                  rows, K, Kp, X, ld, st, out, ex, steps, step));
   } else {
     EUV_CUDA_TRY(ensure_smem(split_b_slab_kernel<R>, smem, done_b));
-    split_b_slab_kernel<R><<<g, MX_SLAB_THREADS, smem, stream>>>(K, rows, Kp, X, ld, st, out, ex,
-                                                                  steps, step);
+    EUV_CUDA_TRY(launch_dependent(split_b_slab_kernel<R>, g, dim3(MX_SLAB_THREADS), smem, stream, K,
+                                  rows, Kp, X, ld, st, out, ex, steps, step));
   }
   EUV_LAUNCH_CHECK();
   return EUV_OK;
@@ -842,7 +845,7 @@ int gemm_mixed(int m, int n, int k, cplx alpha, const double* scale, const doubl
   static int smem_done[3][64];
   auto launch = [&](auto kernel, int* done) -> int {
     EUV_CUDA_TRY(ensure_smem(kernel, (int)MX_SMEM, done));
-    kernel<<<grid, MX_THREADS, MX_SMEM, stream>>>(ta, tb, p);
+    EUV_CUDA_TRY(launch_dependent(kernel, grid, dim3(MX_THREADS), MX_SMEM, stream, ta, tb, p));
     EUV_LAUNCH_CHECK();
     return EUV_OK;
   };

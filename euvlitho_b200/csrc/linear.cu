@@ -21,6 +21,7 @@ struct LinearArgs {
 
 __global__ void linear_amp_kernel(LinearArgs p, const double2* fvac, const double2* a0,
                                   const double2* ax, const double2* ay, double2* amp) {
+  dependent_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int s = blockIdx.y, c = blockIdx.z;
   if (i >= p.ncut) return;
@@ -78,10 +79,12 @@ extern "C" int euv_linear_amp(const euv_linear_desc* d, const euv_c64* d_fvac, c
   const double av = sqrt(p.vc.x * p.vc.x + p.vc.y * p.vc.y);
   p.phase0_inv = cdiv(mk(1.0, 0.0), mk(p.vc.x / av, p.vc.y / av));
   dim3 grid((d->ncut + 255) / 256, d->n_src, d->n_clips);
-  linear_amp_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(
-      p, reinterpret_cast<const double2*>(d_fvac), reinterpret_cast<const double2*>(d_a0),
-      reinterpret_cast<const double2*>(d_ax), reinterpret_cast<const double2*>(d_ay),
-      reinterpret_cast<double2*>(d_amp));
+  EUV_CUDA_TRY(launch_dependent(linear_amp_kernel, grid, dim3(256), 0, (cudaStream_t)stream, p,
+                                reinterpret_cast<const double2*>(d_fvac),
+                                reinterpret_cast<const double2*>(d_a0),
+                                reinterpret_cast<const double2*>(d_ax),
+                                reinterpret_cast<const double2*>(d_ay),
+                                reinterpret_cast<double2*>(d_amp)));
   EUV_LAUNCH_CHECK();
   return EUV_OK;
 }

@@ -193,6 +193,7 @@ template <int LC>
 __global__ void __launch_bounds__(LC_THREADS, 1)
     lu_panel_cluster_kernel(int n, int j0, int jb, double2* A, long long lda, long long sa,
                             int* ipiv, int* info) {
+  dependent_begin();
   cg::cluster_group cluster = cg::this_cluster();
   const int q = LC == 1 ? 0 : (int)cluster.block_rank();
   const int mat = blockIdx.x / LC;
@@ -329,26 +330,29 @@ __global__ void __launch_bounds__(LC_THREADS, 1)
   }
 }
 
+// behind: a launch like launch_dependent's
 template <int LC>
 static void panel_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int batch,
-                         cudaStream_t st) {
+                         cudaStream_t st, bool behind = false) {
   cfg = {};
   cfg.gridDim = dim3(LC * batch);
   cfg.blockDim = dim3(LC_THREADS);
   cfg.stream = st;
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = LC;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = behind ? 1 : 0;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = LC;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = LC > 1 ? 1 : 0;
+  cfg.numAttrs = LC > 1 ? 2 : 1;
 }
 
 template <int LC>
 static int launch_panel(int n, int j0, int jb, double2* A, long long lda, long long sa, int* ipiv,
-                        int* info, int batch, cudaStream_t st) {
+                        int* info, int batch, cudaStream_t st, bool behind) {
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[1];
-  panel_config<LC>(cfg, at, batch, st);
+  cudaLaunchAttribute at[2];
+  panel_config<LC>(cfg, at, batch, st, behind);
   EUV_CUDA_TRY(cudaLaunchKernelEx(&cfg, lu_panel_cluster_kernel<LC>, n, j0, jb, A, lda, sa, ipiv,
                                   info));
   EUV_LAUNCH_CHECK();
@@ -364,7 +368,7 @@ static bool panel16() {
   if (st == 0) {
     int clusters = 0;
     cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     panel_config<16>(cfg, at, 1, nullptr);
     const bool ok = cudaFuncSetAttribute(lu_panel_cluster_kernel<16>,
                                          cudaFuncAttributeNonPortableClusterSizeAllowed,
@@ -387,6 +391,7 @@ static bool panel16() {
 __global__ void lu_laswp_kernel(int n, int ncols, int j0, int jb, int skip0, int skip1,
                                 double2* A, long long lda, long long sa, const int* ipiv,
                                 long long ipiv_stride, int sub) {
+  dependent_begin();
   const int b = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncols) return;
@@ -417,6 +422,7 @@ constexpr int LU_TRSM_WARPS = 8;
 __global__ void __launch_bounds__(32 * LU_TRSM_WARPS)
     lu_trsm_warp_kernel(int jb, int ncols, int lower, const double2* T, long long ldt,
                         long long st, double2* X, long long ldx, long long sx) {
+  dependent_begin();
   __shared__ double2 Ts[LU_NB][LU_NB + 1];
   const int b = blockIdx.y;
   T += (long long)b * st;
@@ -489,20 +495,26 @@ static int panel_sub(int n, int j0) {
   return n - j0 <= 8 * LC_THREADS || (n - j0 <= 16 * LC_THREADS && panel16()) ? 1 : 0;
 }
 
+// CTAs of a trailing update up to which it runs before the next panel, on the same
+// stream: one wave of four per SM.  Such an update is over by the time the look-ahead's
+// events and its separate update of the panel's columns take (two units of N = 361
+// 2.11 -> 2.06 ms per call, four of N = 121 0.52 -> 0.51); at twice as many the update's
+// time shows (two units of N = 545 5.69 -> 5.74 ms).
+constexpr int LU_ONE_WAVE = 4 * 148;
 static int lu_panel(int n, int j0, int jb, double2* A, long long lda, long long sa, int* ipiv,
-                    int* info, int batch, cudaStream_t st) {
+                    int* info, int batch, cudaStream_t st, bool behind) {
   const int rows = n - j0;
   // the tuning table may spread a panel's rows over more CTAs than they need
   const int lc_min = tune_lookup(EUV_KNOB_LU_CLUSTER, n, batch);
   if (rows <= LC_THREADS && lc_min <= 1)
-    return launch_panel<1>(n, j0, jb, A, lda, sa, ipiv, info, batch, st);
+    return launch_panel<1>(n, j0, jb, A, lda, sa, ipiv, info, batch, st, behind);
   if (rows <= 2 * LC_THREADS && lc_min <= 2)
-    return launch_panel<2>(n, j0, jb, A, lda, sa, ipiv, info, batch, st);
+    return launch_panel<2>(n, j0, jb, A, lda, sa, ipiv, info, batch, st, behind);
   if (rows <= 4 * LC_THREADS && lc_min <= 4)
-    return launch_panel<4>(n, j0, jb, A, lda, sa, ipiv, info, batch, st);
-  if (rows <= 8 * LC_THREADS) return launch_panel<8>(n, j0, jb, A, lda, sa, ipiv, info, batch, st);
+    return launch_panel<4>(n, j0, jb, A, lda, sa, ipiv, info, batch, st, behind);
+  if (rows <= 8 * LC_THREADS) return launch_panel<8>(n, j0, jb, A, lda, sa, ipiv, info, batch, st, behind);
   if (rows <= 16 * LC_THREADS && panel16())
-    return launch_panel<16>(n, j0, jb, A, lda, sa, ipiv, info, batch, st);
+    return launch_panel<16>(n, j0, jb, A, lda, sa, ipiv, info, batch, st, behind);
   lu_panel_kernel<<<batch, LU_PANEL_THREADS, 0, st>>>(n, j0, jb, A, lda, sa, ipiv, info);
   EUV_LAUNCH_CHECK();
   return EUV_OK;
@@ -513,8 +525,9 @@ static int lu_panel(int n, int j0, int jb, double2* A, long long lda, long long 
 static int lu_update(int n, int j0, int jb, int c0, int nc, double2* A, long long lda,
                      long long sa, int batch, cudaStream_t st) {
   if (nc <= 0) return EUV_OK;
-  lu_trsm_warp_kernel<<<trsm_grid(nc, batch), 32 * LU_TRSM_WARPS, 0, st>>>(
-      jb, nc, 1, A + j0 + (long long)j0 * lda, lda, sa, A + j0 + (long long)c0 * lda, lda, sa);
+  EUV_CUDA_TRY(launch_dependent(lu_trsm_warp_kernel, trsm_grid(nc, batch), dim3(32 * LU_TRSM_WARPS),
+                                0, st, jb, nc, 1, A + j0 + (long long)j0 * lda, lda, sa,
+                                A + j0 + (long long)c0 * lda, lda, sa));
   EUV_LAUNCH_CHECK();
   const int rest = n - j0 - jb;
   if (rest <= 0) return EUV_OK;
@@ -542,11 +555,18 @@ int lu_factor(int n, double2* A, long long lda, long long sa, int* ipiv, int* in
   zero_int_kernel<<<(batch + 255) / 256, 256, 0, stream>>>(info, batch);
   EUV_LAUNCH_CHECK();
   int j0 = 0, jb = n < LU_NB ? n : LU_NB;
-  int rc = lu_panel(n, j0, jb, A, lda, sa, ipiv, info, batch, stream);
+  int rc = lu_panel(n, j0, jb, A, lda, sa, ipiv, info, batch, stream, true);
   if (rc) return rc;
+  bool behind = true;  // the last panel ran on this stream
   for (;;) {
     dim3 gs((n + extra + 127) / 128, batch);
-    lu_laswp_kernel<<<gs, 128, 0, stream>>>(n, n + extra, j0, jb, j0, j0 + jb, A, lda, sa, ipiv, n, panel_sub(n, j0));
+    if (behind) {
+      EUV_CUDA_TRY(launch_dependent(lu_laswp_kernel, gs, dim3(128), 0, stream, n, n + extra, j0, jb,
+                                    j0, j0 + jb, A, lda, sa, ipiv, n, panel_sub(n, j0)));
+    } else {
+      lu_laswp_kernel<<<gs, 128, 0, stream>>>(n, n + extra, j0, jb, j0, j0 + jb, A, lda, sa, ipiv, n,
+                                              panel_sub(n, j0));
+    }
     EUV_LAUNCH_CHECK();
     const int rest = n - j0 - jb;
     if (rest <= 0) {
@@ -554,16 +574,19 @@ int lu_factor(int n, double2* A, long long lda, long long sa, int* ipiv, int* in
       break;
     }
     const int j1 = j0 + jb, nb2 = rest < LU_NB ? rest : LU_NB, rem = rest - nb2 + extra;
-    if ((rc = lu_update(n, j0, jb, j1, nb2, A, lda, sa, batch, stream))) return rc;
-    if (rem > 0) {
+    const long long ctas = (long long)((rest + 31) / 32) * ((nb2 + rem + 63) / 64) * batch;
+    behind = rem <= 0 || ctas <= LU_ONE_WAVE;
+    if (behind) {
+      if ((rc = lu_update(n, j0, jb, j1, nb2 + rem, A, lda, sa, batch, stream))) return rc;
+      if ((rc = lu_panel(n, j1, nb2, A, lda, sa, ipiv, info, batch, stream, true))) return rc;
+    } else {
+      if ((rc = lu_update(n, j0, jb, j1, nb2, A, lda, sa, batch, stream))) return rc;
       EUV_CUDA_TRY(cudaEventRecord(side->fork, stream));
       EUV_CUDA_TRY(cudaStreamWaitEvent(side->hi, side->fork, 0));
-      if ((rc = lu_panel(n, j1, nb2, A, lda, sa, ipiv, info, batch, side->hi))) return rc;
+      if ((rc = lu_panel(n, j1, nb2, A, lda, sa, ipiv, info, batch, side->hi, false))) return rc;
       if ((rc = lu_update(n, j0, jb, j1 + nb2, rem, A, lda, sa, batch, stream))) return rc;
       EUV_CUDA_TRY(cudaEventRecord(side->join, side->hi));
       EUV_CUDA_TRY(cudaStreamWaitEvent(stream, side->join, 0));
-    } else if ((rc = lu_panel(n, j1, nb2, A, lda, sa, ipiv, info, batch, stream))) {
-      return rc;
     }
     j0 = j1;
     jb = nb2;
@@ -699,6 +722,7 @@ __global__ void __launch_bounds__(LS_THREADS) lu_subst_kernel(int n, int nrhs, c
                                                               double2* B, long long ldb,
                                                               long long sb, const int* order,
                                                               long long ostride) {
+  dependent_begin();
   extern __shared__ double2 xs[];
   __shared__ double2 ds[LS_BLK][LS_BLK + 1];
   const int b = blockIdx.y, c0 = blockIdx.x * RC;
@@ -781,8 +805,8 @@ static int launch_subst(int n, int nrhs, const double2* LU, long long lda, long 
   const int smem = (int)((size_t)RC * n * sizeof(double2));
   EUV_CUDA_TRY(ensure_smem(lu_subst_kernel<RC, BACK>, smem, smem_done));
   dim3 grid((nrhs + RC - 1) / RC, batch);
-  lu_subst_kernel<RC, BACK><<<grid, LS_THREADS, smem, stream>>>(n, nrhs, LU, lda, sa, B, ldb, sb, order,
-                                                          ostride);
+  EUV_CUDA_TRY(launch_dependent(lu_subst_kernel<RC, BACK>, grid, dim3(LS_THREADS), smem, stream, n,
+                                nrhs, LU, lda, sa, B, ldb, sb, order, ostride));
   EUV_LAUNCH_CHECK();
   return EUV_OK;
 }
@@ -847,8 +871,9 @@ static int blocked_solve(bool lower, int n, int nrhs, const double2* LU, long lo
   const int nblk = (n + LU_NB - 1) / LU_NB;
   for (int k = 0; k < nblk; ++k) {
     const int j0 = (lower ? k : nblk - 1 - k) * LU_NB, jb = (n - j0) < LU_NB ? (n - j0) : LU_NB;
-    lu_trsm_warp_kernel<<<trsm_grid(nrhs, batch), 32 * LU_TRSM_WARPS, 0, stream>>>(
-        jb, nrhs, lower ? 1 : 0, LU + j0 + (long long)j0 * lda, lda, sa, B + j0, ldb, sb);
+    EUV_CUDA_TRY(launch_dependent(lu_trsm_warp_kernel, trsm_grid(nrhs, batch),
+                                  dim3(32 * LU_TRSM_WARPS), 0, stream, jb, nrhs, lower ? 1 : 0,
+                                  LU + j0 + (long long)j0 * lda, lda, sa, B + j0, ldb, sb));
     EUV_LAUNCH_CHECK();
     const int r0 = lower ? j0 + jb : 0, rows = lower ? n - r0 : j0;
     if (rows > 0) {

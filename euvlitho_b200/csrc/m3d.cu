@@ -25,6 +25,7 @@ __device__ __forceinline__ cplx unit_phase(cplx v) {
 
 __global__ void m3d_fit_kernel(M3dParams p, int n_clips, const double2* ax_wide,
                                const double2* fmask, double2* a0, double2* ax, double2* ay) {
+  dependent_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_clips * p.ninput) return;
   const int c = t / p.ninput, n = t % p.ninput;
@@ -126,10 +127,12 @@ extern "C" int euv_m3d_fit(const euv_m3d_desc* d, const euv_c64* d_ax_wide,
   p.xin = d->d_xin;
   p.pair = d->d_pair_order;
   const int total = d->n_clips * d->ninput;
-  m3d_fit_kernel<<<(total + 127) / 128, 128, 0, (cudaStream_t)stream_>>>(
-      p, d->n_clips, reinterpret_cast<const double2*>(d_ax_wide),
-      reinterpret_cast<const double2*>(d_fmask), reinterpret_cast<double2*>(d_a0),
-      reinterpret_cast<double2*>(d_ax), reinterpret_cast<double2*>(d_ay));
+  EUV_CUDA_TRY(launch_dependent(m3d_fit_kernel, dim3((total + 127) / 128), dim3(128), 0,
+                                (cudaStream_t)stream_, p, d->n_clips,
+                                reinterpret_cast<const double2*>(d_ax_wide),
+                                reinterpret_cast<const double2*>(d_fmask),
+                                reinterpret_cast<double2*>(d_a0), reinterpret_cast<double2*>(d_ax),
+                                reinterpret_cast<double2*>(d_ay)));
   EUV_LAUNCH_CHECK();
   return EUV_OK;
 }

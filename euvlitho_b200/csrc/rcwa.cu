@@ -99,6 +99,7 @@ __global__ void spectrum_wx_kernel(int ndivx, int meshx, int fx, double scale, i
 }
 // Wy[m' + mr jj] = sum over the pattern rows of mask row jj of exp(-2 pi i m y / fy)
 __global__ void spectrum_wy_kernel(int ndivy, int meshy, int fy, int y_offset, int mh, double2* W) {
+  dependent_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x, mr = 2 * mh + 1;
   if (t >= ndivy * mr) return;
   const int m = t % mr - mh, jj = t / mr;
@@ -135,6 +136,7 @@ template <int NB>
 __global__ void __cluster_dims__(SP_CL, 1, 1) __launch_bounds__(256)
     spectrum_rows_kernel(const uint8_t* bits, long long mask_bytes, int ndivx, int ndivy, int lh,
                          const double* W, double2* T) {
+  dependent_begin();
   namespace cg = cooperative_groups;
   constexpr int ST = NB * 8 + 4;  // doubles per staged pixel: conflict-free fragments
   cg::cluster_group cluster = cg::this_cluster();
@@ -232,6 +234,7 @@ constexpr size_t spectrum_smem() {
 // unless select_vacuum, the absorber's spectrum delta - F
 __global__ void spectrum_reduce_kernel(const double2* part, int parts, int masks, int lh, int mh,
                                        int select_vacuum, double2* out) {
+  dependent_begin();
   const int lr = 2 * lh + 1, mr = 2 * mh + 1;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)masks * lr * mr) return;
@@ -283,6 +286,7 @@ __global__ void build_dg_kernel(SliceParams p, const double2* spectra, const int
                                 const double* ky0, const int* polar, const double2* adm,
                                 const double2* shift, const double* radius, double2* D,
                                 long long sd, double2* G, long long sg, int want_g) {
+  dependent_begin();
   // grid: x = column j, y = row chunk, z = unit (no 64-bit division per element)
   const int u = blockIdx.z, j = blockIdx.x;
   // the unit's and column's constants once per CTA: no FP64 division per element
@@ -450,6 +454,7 @@ __global__ void zero_f64_kernel(double* p, int n) {
 
 // norm[b] = max_j sum_i (|re|+|im|)(D[b](i,j)): one warp per column.
 __global__ void norm1_kernel(int n, const double2* D, double* norm) {
+  dependent_begin();
   const int b = blockIdx.y;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -465,6 +470,7 @@ __global__ void norm1_kernel(int n, const double2* D, double* norm) {
 // m = smallest m >= 0 with norm*(d/2^m)^2 <= theta (capped at m_max); h = d/2^m.
 __global__ void scale_kernel(int batch, double theta, const double* norm, const double* thick, int m_max,
                              int* steps, double* h, double* h2, double* h4, int* capped) {
+  dependent_begin();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= batch) return;
   double d = thick[b];
@@ -501,6 +507,7 @@ __global__ void taylor_prep_kernel(int n, int batch, const double2* D, const dou
                                    const double2* P3, const double2* P4, const double* h,
                                    const double* h2, double2* Cc, double2* Tc, double2* Cs,
                                    double2* Ts) {
+  dependent_begin();
   const long long nn = (long long)n * n;
   const int b = blockIdx.y;
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -706,6 +713,7 @@ __global__ void __launch_bounds__(PF_SAMPLES)
     poly_coef_kernel(PolySlices p, const int* lidx, const int* midx, const double* kx0,
                      const double* ky0, const int* polar, double2* coef, double2* ident,
                      double2* shift, double* radius, int* steps, int* blocks, int* status) {
+  dependent_begin();
   const int u = blockIdx.x, sl = blockIdx.y, tid = threadIdx.x;
   __shared__ double s_lo[2], s_hi[2], s_km[2];
   __shared__ cplx s_f[2][PF_SAMPLES], s_w[PF_SAMPLES], s_a[2][PF_K + 1];
@@ -827,6 +835,7 @@ template <int Q, int NB>
 __global__ void __launch_bounds__(256)
     poly_block_kernel(int n, const double2* pw, long long sp, const double2* coef, int n_units,
                       int slice, int b0, double2* top, double2* low, long long so) {
+  dependent_begin();
   __shared__ double2 s_c[NB][2][Q];
   const int u = blockIdx.z, j = blockIdx.x;
   if (threadIdx.x < NB * 2 * Q) {
@@ -856,12 +865,12 @@ static int poly_blocks(int q, int n, const double2* pw, long long sp, const doub
                        int slice, int b0, double2* top, double2* low, long long so,
                        cudaStream_t stream) {
   const dim3 g((unsigned)n, (unsigned)((n + 255) / 256), U);
-  switch (q) {
-    case 3: poly_block_kernel<3, NB><<<g, 256, 0, stream>>>(n, pw, sp, coef, U, slice, b0, top, low, so); break;
-    case 4: poly_block_kernel<4, NB><<<g, 256, 0, stream>>>(n, pw, sp, coef, U, slice, b0, top, low, so); break;
-    case 5: poly_block_kernel<5, NB><<<g, 256, 0, stream>>>(n, pw, sp, coef, U, slice, b0, top, low, so); break;
-    default: poly_block_kernel<6, NB><<<g, 256, 0, stream>>>(n, pw, sp, coef, U, slice, b0, top, low, so); break;
-  }
+  const auto kernel = q == 3   ? poly_block_kernel<3, NB>
+                      : q == 4 ? poly_block_kernel<4, NB>
+                      : q == 5 ? poly_block_kernel<5, NB>
+                               : poly_block_kernel<6, NB>;
+  EUV_CUDA_TRY(launch_dependent(kernel, g, dim3(256), 0, stream, n, pw, sp, coef, U, slice, b0, top,
+                                low, so));
   EUV_LAUNCH_CHECK();
   return EUV_OK;
 }
@@ -879,6 +888,7 @@ __global__ void top_rows_kernel(int n, const double* klm, const double2* shift,
                                 const double2* C, const double2* S, long long sc, const double2* E,
                                 double2* V, double2* W, double2* M, long long sw, const double2* P,
                                 const double2* Q, long long sp) {
+  dependent_begin();
   const int b = blockIdx.z, j = blockIdx.x;
   const int i = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -913,6 +923,7 @@ __global__ void source_rows_kernel(int n, int nsrc, const int* src_order, const 
                                    const double2* V, const double2* W, long long sw,
                                    const double2* P, const double2* Q, long long sp, double2* V2,
                                    double2* W2, double2* rhs, long long sr) {
+  dependent_begin();
   const int b = blockIdx.z, s = blockIdx.x;
   const int i = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -951,6 +962,7 @@ __global__ void bottom_rows_kernel(int n, const double2* shift, const double* ra
                                    const double2* S, long long sc, const double2* E, long long se,
                                    const double2* P, long long sp, double2* R1, double2* R2,
                                    long long sr) {
+  dependent_begin();
   const int b = blockIdx.z, j = blockIdx.x;
   const int i = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -973,6 +985,7 @@ __global__ void bottom_rows_kernel(int n, const double2* shift, const double* ra
 // weight (header.h:1394-1465); zero for empty slots.
 __global__ void ax_out_kernel(int n, int nsrc, const int* src_order, const double* src_2kz,
                               const double* klm, const double2* x, long long sx, double2* ax) {
+  dependent_begin();
   const int b = blockIdx.z, s = blockIdx.x;
   const int i = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -1013,6 +1026,7 @@ __global__ void fill_f64_kernel(double* p, int n, double v) {
 
 // An LU's zero pivots (info != 0) as EUV_STATUS_SINGULAR in the status word.
 __global__ void flag_singular_kernel(const int* info, int n, int* status) {
+  dependent_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && info[i] != 0) atomicOr(status, EUV_STATUS_SINGULAR);
 }
@@ -1071,11 +1085,11 @@ int matfun(int n, int batch, const double2* D, const double* thick, double2** pc
   zero_f64_kernel<<<grid1(batch, 256), 256, 0, stream>>>(w.norm, batch);
   EUV_LAUNCH_CHECK();
   dim3 gn(grid1((long long)n * 32, 256), batch);
-  norm1_kernel<<<gn, 256, 0, stream>>>(n, D, w.norm);
+  EUV_CUDA_TRY(launch_dependent(norm1_kernel, gn, dim3(256), 0, stream, n, D, w.norm));
   EUV_LAUNCH_CHECK();
-  scale_kernel<<<grid1(batch, 128), 128, 0, stream>>>(batch, theta_for(gemm.precision), w.norm,
-                                                      thick, m_max, w.steps, w.h,
-                                                      w.h2, w.h4, w.capped);
+  EUV_CUDA_TRY(launch_dependent(scale_kernel, dim3(grid1(batch, 128)), dim3(128), 0, stream, batch,
+                                theta_for(gemm.precision), w.norm, thick, m_max, w.steps, w.h, w.h2,
+                                w.h4, w.capped));
   EUV_LAUNCH_CHECK();
   const cplx one = mk(1.0, 0.0), zero = mk(0.0, 0.0);
   int rc;
@@ -1087,8 +1101,8 @@ int matfun(int n, int batch, const double2* D, const double* thick, double2** pc
                  nullptr, 0, kReuseA))) return rc;  // P2 as A again
   double2* C = *pc;
   double2* S = *ps;
-  taylor_prep_kernel<<<ge, bs, 0, stream>>>(n, batch, D, w.P2, w.P3, w.P4, w.h, w.h2, C, w.T1, S,
-                                            w.T2);
+  EUV_CUDA_TRY(launch_dependent(taylor_prep_kernel, ge, dim3(bs), 0, stream, n, batch, D, w.P2,
+                                w.P3, w.P4, w.h, w.h2, C, w.T1, S, w.T2));
   EUV_LAUNCH_CHECK();
   if ((rc = gemm(n, n, n, one, nullptr, w.P4, n, nn, w.T1, n, nn, one, C, n, nn, zero, batch))) return rc;
   if ((rc = gemm(n, n, n, one, nullptr, w.P4, n, nn, w.T2, n, nn, one, S, n, nn, zero, batch,
@@ -1352,9 +1366,9 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
     ps.m[n] = r.m;
     ps.m_limit[n] = d->m_max > 0 && d->m_max < r.m ? d->m_max : r.m;
   }
-  poly_coef_kernel<<<dim3(U, NS), PF_SAMPLES, 0, stream>>>(ps, d->d_lindex, d->d_mindex, d->d_kx0,
-                                                           d->d_ky0, d->d_polar, w.coef, w.ident, w.shift,
-                                                           w.radius, w.steps, w.blocks, status);
+  EUV_CUDA_TRY(launch_dependent(poly_coef_kernel, dim3(U, NS), dim3(PF_SAMPLES), 0, stream, ps,
+                                d->d_lindex, d->d_mindex, d->d_kx0, d->d_ky0, d->d_polar, w.coef,
+                                w.ident, w.shift, w.radius, w.steps, w.blocks, status));
   EUV_LAUNCH_CHECK();
 
   // Mixed form: G^-1 by the Euler product (I - E)^-1 = prod_f (I + E^(2^f)),
@@ -1372,10 +1386,11 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
   Mat pw[6], cs[2] = {{w.pair[0], 2 * nn}, {w.pair[1], 2 * nn}}, pq = {w.pair[2], 2 * nn};
   for (int i = 0; i < 6; ++i) pw[i] = Mat{w.pw + i * nn, 6 * nn};
   auto build = [&](int slice, const Mat* E, const Mat* G, int want_g) -> int {
-    build_dg_kernel<<<gdg, bs, 0, stream>>>(
-        slice_params(slice), spec, d->d_spec, d->d_lindex, d->d_mindex, d->d_kx0, d->d_ky0,
-        d->d_polar, w.adm, w.shift + (size_t)slice * U, w.radius + (size_t)slice * U,
-        E ? E->p : nullptr, E ? E->s : 0, G ? G->p : nullptr, G ? G->s : 0, want_g);
+    EUV_CUDA_TRY(launch_dependent(build_dg_kernel, gdg, bs, 0, stream, slice_params(slice), spec,
+                                  d->d_spec, d->d_lindex, d->d_mindex, d->d_kx0, d->d_ky0,
+                                  d->d_polar, w.adm, w.shift + (size_t)slice * U,
+                                  w.radius + (size_t)slice * U, E ? E->p : nullptr, E ? E->s : 0,
+                                  G ? G->p : nullptr, G ? G->s : 0, want_g));
     EUV_LAUNCH_CHECK();
     return EUV_OK;
   };
@@ -1497,7 +1512,8 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
         if ((rc = build(n + 1, nullptr, &E, 1))) return rc;
         if ((rc = build(n, nullptr, &En, 1))) return rc;
         if ((rc = lu_factor(N, E.p, N, E.s, w.ipiv, w.info, U, stream))) return rc;
-        flag_singular_kernel<<<grid1(U, 256), 256, 0, stream>>>(w.info, U, status);
+        EUV_CUDA_TRY(launch_dependent(flag_singular_kernel, dim3(grid1(U, 256)), dim3(256), 0,
+                                      stream, w.info, U, status));
         EUV_LAUNCH_CHECK();
         if ((rc = lu_solve(N, N, E.p, N, E.s, w.ipiv, En.p, N, En.s, U, stream))) return rc;
         if ((rc = mul(one, nullptr, P, En, zero, pw[2], 0))) return rc;
@@ -1529,14 +1545,14 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
       const Mat ax = behind ? pw[4] : Mat{reinterpret_cast<double2*>(d_ax), sn};
       const double2* Qp = bottom ? nullptr : Q.p;
       if ((rc = mul(pi_, rad, E, S, zero, W, 0))) return rc;
-      top_rows_kernel<<<gdg, bs, 0, stream>>>(N, w.klm, ia, rad, c0, s0, C.p, S.p, C.s, E.p, V.p,
-                                              W.p, M.p, E.s, P.p, Qp, P.s);
+      EUV_CUDA_TRY(launch_dependent(top_rows_kernel, gdg, dim3(bs), 0, stream, N, w.klm, ia, rad,
+                                    c0, s0, C.p, S.p, C.s, E.p, V.p, W.p, M.p, E.s, P.p, Qp, P.s));
       EUV_LAUNCH_CHECK();
       const dim3 gs((unsigned)ns, (unsigned)((N + bs - 1) / bs), U);
       if (ns > 0) {
-        source_rows_kernel<<<gs, bs, 0, stream>>>(N, ns, d->d_src_order, w.klm, ia, c0, s0, C.p, S.p,
-                                                  C.s, V.p, W.p, V.s, P.p, Qp, P.s, V2.p, W2.p,
-                                                  ax.p, ax.s);
+        EUV_CUDA_TRY(launch_dependent(source_rows_kernel, gs, dim3(bs), 0, stream, N, ns,
+                                      d->d_src_order, w.klm, ia, c0, s0, C.p, S.p, C.s, V.p, W.p,
+                                      V.s, P.p, Qp, P.s, V2.p, W2.p, ax.p, ax.s));
         EUV_LAUNCH_CHECK();
       }
       if ((rc = mul(one, nullptr, P, V, one, M, 0))) return rc;
@@ -1546,7 +1562,8 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
         if (ns > 0 && (rc = mul(m1, nullptr, Q, W2, one, ax, kReuseA, Term{}, ns))) return rc;
       }
       if ((rc = lu_factor(N, M.p, N, M.s, w.ipiv, w.info, U, stream, behind ? ns : 0))) return rc;
-      flag_singular_kernel<<<grid1(U, 256), 256, 0, stream>>>(w.info, U, status);
+      EUV_CUDA_TRY(launch_dependent(flag_singular_kernel, dim3(grid1(U, 256)), dim3(256), 0, stream,
+                                    w.info, U, status));
       EUV_LAUNCH_CHECK();
       if (ns > 0) {
         // empty source slots (order < 0, zero columns) skip their CTAs
@@ -1554,8 +1571,9 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
                          : lu_solve(N, ns, M.p, N, M.s, w.ipiv, ax.p, N, ax.s, U, stream,
                                     d->d_src_order, ns)))
           return rc;
-        ax_out_kernel<<<gs, bs, 0, stream>>>(N, ns, d->d_src_order, d->d_src_2kz, w.klm, ax.p, ax.s,
-                                             reinterpret_cast<double2*>(d_ax));
+        EUV_CUDA_TRY(launch_dependent(ax_out_kernel, gs, dim3(bs), 0, stream, N, ns, d->d_src_order,
+                                      d->d_src_2kz, w.klm, ax.p, ax.s,
+                                      reinterpret_cast<double2*>(d_ax)));
         EUV_LAUNCH_CHECK();
       }
       return EUV_OK;
@@ -1563,8 +1581,8 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
     const Mat R1 = cs[1], R2{cs[1].p + nn, 2 * nn};
     if (bottom) {
       // Q = I: R1 = P c + i D s, R2 = c + i P s
-      bottom_rows_kernel<<<gdg, bs, 0, stream>>>(N, ia, rad, c0, s0, C.p, S.p, C.s, E.p, E.s, P.p,
-                                                 P.s, R1.p, R2.p, R1.s);
+      EUV_CUDA_TRY(launch_dependent(bottom_rows_kernel, gdg, dim3(bs), 0, stream, N, ia, rad, c0,
+                                    s0, C.p, S.p, C.s, E.p, E.s, P.p, P.s, R1.p, R2.p, R1.s));
       EUV_LAUNCH_CHECK();
       if ((rc = mul(pi_, rad, E, S, one, R1, 0))) return rc;
       if ((rc = mul(pi_, nullptr, P, S, one, R2, kReuseB))) return rc;  // S as B again
@@ -1607,7 +1625,8 @@ static int launch_spectrum_rows(const uint8_t* bits, long long mask_bytes, int n
   constexpr size_t sm = spectrum_smem<NB>();
   EUV_CUDA_TRY(ensure_smem(spectrum_rows_kernel<NB>, (int)sm, done));
   const dim3 g(SP_CL * ((ndivy + SP_ROWS - 1) / SP_ROWS), tiles, masks);
-  spectrum_rows_kernel<NB><<<g, 256, sm, stream>>>(bits, mask_bytes, ndivx, ndivy, lh, W, T);
+  EUV_CUDA_TRY(launch_dependent(spectrum_rows_kernel<NB>, g, dim3(256), sm, stream, bits,
+                                mask_bytes, ndivx, ndivy, lh, W, T));
   EUV_LAUNCH_CHECK();
   return EUV_OK;
 }
@@ -1644,8 +1663,8 @@ extern "C" int euv_mask_spectrum(const uint8_t* d_bits, int n_masks, int ndivx, 
   spectrum_wx_kernel<<<grid1((long long)ndivx * lp, 256), 256, 0, stream>>>(
       ndivx, meshx, fdivx, 1.0 / ((double)fdivx * (double)fdivy), lh, Wx);
   EUV_LAUNCH_CHECK();
-  spectrum_wy_kernel<<<grid1((long long)ndivy * mr, 256), 256, 0, stream>>>(ndivy, meshy, fdivy,
-                                                                           y_offset, mh, Wy);
+  EUV_CUDA_TRY(launch_dependent(spectrum_wy_kernel, dim3(grid1((long long)ndivy * mr, 256)),
+                                dim3(256), 0, stream, ndivy, meshy, fdivy, y_offset, mh, Wy));
   EUV_LAUNCH_CHECK();
   const long long mask_bytes = (long long)ndivx * ndivy / 8;
   // column tiles of at most eight blocks of 8, as even as they come
@@ -1677,8 +1696,9 @@ extern "C" int euv_mask_spectrum(const uint8_t* d_bits, int n_masks, int ndivx, 
                mk(0.0, 0.0), P, mr, (long long)mr * cols, mk(0.0, 0.0), parts, nullptr, 0, stream);
     if (rc) return rc;
     const long long total = (long long)ng * lr * mr;
-    spectrum_reduce_kernel<<<grid1(total, 256), 256, 0, stream>>>(
-        P, parts, ng, lh, mh, select_vacuum, reinterpret_cast<double2*>(d_out) + g0 * lr * mr);
+    EUV_CUDA_TRY(launch_dependent(spectrum_reduce_kernel, dim3(grid1(total, 256)), dim3(256), 0,
+                                  stream, P, parts, ng, lh, mh, select_vacuum,
+                                  reinterpret_cast<double2*>(d_out) + g0 * lr * mr));
     EUV_LAUNCH_CHECK();
   }
   return EUV_OK;

@@ -35,6 +35,7 @@ struct SocsArgs {
 // G[(c*rows + r)*nout^2 + px + nout*py], px = lp mod nout.
 __global__ void socs_rows_kernel(SocsArgs p, const double2* fvac, const double2* a0,
                                  const double2* ax, const double2* ay, double2* G) {
+  dependent_begin();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   const int r = blockIdx.y, c = blockIdx.z;
   if (n >= p.ncut) return;
@@ -75,6 +76,7 @@ __global__ void socs_rows_kernel(SocsArgs p, const double2* fvac, const double2*
 __global__ void socs_accum_kernel(int nout, int rows, int nsocs, int nxy, const double* al0,
                                   const double* alx, const double* aly, const double2* F,
                                   double2* smallT) {
+  dependent_begin();
   const int g = blockIdx.x * blockDim.x + threadIdx.x;  // u + nout*v (F's column-major index)
   const int c = blockIdx.y;
   const int nn = nout * nout;
@@ -172,9 +174,11 @@ extern "C" int euv_socs_image(const euv_socs_desc* d, const euv_c64* d_fvac, con
   p.phix = reinterpret_cast<const double2*>(d->d_phi_sx);
   p.phiy = reinterpret_cast<const double2*>(d->d_phi_sy);
   EUV_CUDA_TRY(cudaMemsetAsync(G, 0, gb, stream));
-  socs_rows_kernel<<<dim3((d->ncut + 127) / 128, rows, d->n_clips), 128, 0, stream>>>(
-      p, reinterpret_cast<const double2*>(d_fvac), reinterpret_cast<const double2*>(d_a0),
-      reinterpret_cast<const double2*>(d_ax), reinterpret_cast<const double2*>(d_ay), G);
+  EUV_CUDA_TRY(launch_dependent(socs_rows_kernel, dim3((d->ncut + 127) / 128, rows, d->n_clips),
+                                dim3(128), 0, stream, p, reinterpret_cast<const double2*>(d_fvac),
+                                reinterpret_cast<const double2*>(d_a0),
+                                reinterpret_cast<const double2*>(d_ax),
+                                reinterpret_cast<const double2*>(d_ay), G));
   EUV_LAUNCH_CHECK();
   const cplx one = mk(1.0, 0.0), zero = mk(0.0, 0.0);
   const double2* E = reinterpret_cast<const double2*>(d->d_e);
@@ -186,8 +190,9 @@ extern "C" int euv_socs_image(const euv_socs_desc* d, const euv_c64* d_fvac, con
   rc = zgemm(nout, nout, nout, one, nullptr, E, nout, 0, T, nout, nn, zero, G, nout, nn, zero, nb,
              nullptr, 0, stream);
   if (rc) return rc;
-  socs_accum_kernel<<<dim3((nn + 127) / 128, d->n_clips), 128, 0, stream>>>(
-      nout, rows, d->nsocs, d->nsocsxy, d->d_alpha_s0, d->d_alpha_sx, d->d_alpha_sy, G, smallT);
+  EUV_CUDA_TRY(launch_dependent(socs_accum_kernel, dim3((nn + 127) / 128, d->n_clips), dim3(128), 0,
+                                stream, nout, rows, d->nsocs, d->nsocsxy, d->d_alpha_s0,
+                                d->d_alpha_sx, d->d_alpha_sy, G, smallT));
   EUV_LAUNCH_CHECK();
   // T3 = small^T . Kx^T (nout x XDIV), image^T = Ky . T3 (YDIV x XDIV) = image[x][y]
   const double2* kxT = reinterpret_cast<const double2*>(d->d_kxT);

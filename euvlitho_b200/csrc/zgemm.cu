@@ -82,6 +82,7 @@ __device__ __forceinline__ int b_at(int k, int j) { return j * GBK + (k ^ ((j & 
 // MI: 8-row blocks per warp (tile BM = 16 MI rows x 64 columns); ST: cp.async stages.
 template <int MI, int ST>
 __global__ void __launch_bounds__(GTHREADS, MI == 2 ? 4 : 2) zgemm_upd_kernel(GemmArgs p) {
+  dependent_begin();
   constexpr int BM = 16 * MI;
   constexpr int AP = BM + 2;
   extern __shared__ double2 smem[];
@@ -230,6 +231,7 @@ struct Flag {
 
 template <bool THREE, int MI>
 __global__ void __launch_bounds__(GTHREADS, 3) zgemm_kernel(GemmArgs p) {
+  dependent_begin();
   constexpr int BM = 32 * MI, AP = BM + 2, NACC = THREE ? 3 : 2;
   extern __shared__ double2 smem[];
   double2* As = smem;
@@ -446,7 +448,7 @@ static int zgemm_run(K kernel, int rows, int cols, size_t smem, int* done, const
                      int batch, cudaStream_t stream) {
   dim3 grid((p.m + rows - 1) / rows, (p.n + cols - 1) / cols, batch);
   EUV_CUDA_TRY(ensure_smem(kernel, (int)smem, done));
-  kernel<<<grid, GTHREADS, smem, stream>>>(p);
+  EUV_CUDA_TRY(launch_dependent(kernel, grid, dim3(GTHREADS), smem, stream, p));
   EUV_LAUNCH_CHECK();
   return EUV_OK;
 }
