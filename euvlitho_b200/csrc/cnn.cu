@@ -183,6 +183,14 @@ __global__ void cnn_input_kernel(const uint8_t* bits, float* x0) {
   x0[(size_t)img * CNN_IN * CNN_IN + t] = (float)cnt * 0.0625f;
 }
 
+// 32 bytes in one store, p 32-byte aligned: a whole sector, where two of 16 bytes
+// from lanes 64 bytes apart each take L2 a partial write.
+__device__ __forceinline__ void store8(float* p, const float* v) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]),
+               "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+
 // Writes 16 channels [c0, c0+16) of pooled pixel (py, px) to the (hi, lo)
 // planes of an activation [img][so+2p][so+2p][C] (plane stride `plane`), with
 // the circular halo copies when padded.
@@ -202,24 +210,39 @@ __device__ __forceinline__ void cnn_store16(float* hi_base, long long plane, int
   for (int i = 0; i < nr; ++i)
     for (int j = 0; j < nc; ++j) {
       float* d = hi_base + ((long long)ry[i] * hp + rx[j]) * cch + c0;
-      float4* dh = reinterpret_cast<float4*>(d);
-      float4* dl = reinterpret_cast<float4*>(d + plane);
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        dh[v] = make_float4(hi[4 * v], hi[4 * v + 1], hi[4 * v + 2], hi[4 * v + 3]);
-        dl[v] = make_float4(lo[4 * v], lo[4 * v + 1], lo[4 * v + 2], lo[4 * v + 3]);
+      for (int v = 0; v < 16; v += 8) {
+        store8(d + v, hi + v);
+        store8(d + plane + v, lo + v);
       }
     }
 }
 
+// Two FP32 FMAs in one instruction, each rounded as fmaf
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, c, d;\n\t"
+      "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
 // conv1 (1 -> 16 channels, 512^2) + bias, ReLU, 2x2 max-pool, BN for pooled
-// pixel (py, px) of image blockIdx.y, model blockIdx.z.
+// pixel (py, px) of image blockIdx.y, model blockIdx.z.  576 FMAs per pooled pixel,
+// two channels to an instruction; four channels share the loads of their weights.
+// Bound by its instructions (about 700 per pixel, 184 us) and its 1.2 GB of stores
+// (187 us): six networks, 24 masks 446 us with scalar FMAs and 16-byte stores, 409 with
+// the pairs, 388 with store8 (the other convolutions 2246 -> 2164 with it).
 __global__ void cnn_conv1_kernel(int B, const float* x0, const float* w, const float* bias,
                                  const float* scale, const float* shift, float* out) {
   dependent_begin();
-  __shared__ float sw[144], sb[16], ss[16], sh[16];
+  __shared__ float4 sw[4][9];  // weights of channels 4 g .. 4 g + 3, by tap
+  __shared__ float sb[16], ss[16], sh[16];
   const int m = blockIdx.z, img = blockIdx.y;
-  for (int i = threadIdx.x; i < 144; i += blockDim.x) sw[i] = w[m * 144 + i];
+  for (int i = threadIdx.x; i < 144; i += blockDim.x)
+    reinterpret_cast<float*>(&sw[i / 36][i % 9])[(i / 9) % 4] = w[m * 144 + i];
   if (threadIdx.x < 16) {
     sb[threadIdx.x] = bias[m * 16 + threadIdx.x];
     ss[threadIdx.x] = scale[m * 16 + threadIdx.x];
@@ -231,30 +254,44 @@ __global__ void cnn_conv1_kernel(int B, const float* x0, const float* w, const f
   if (t >= SO * SO) return;
   const int py = t / SO, px = t % SO;
   const float* X = x0 + (size_t)img * CNN_IN * CNN_IN;
-  float win[4][4];
+  float2 win[4][4];  // each value twice
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
     const int r = (2 * py - 1 + a) & (CNN_IN - 1);
 #pragma unroll
-    for (int b = 0; b < 4; ++b) win[a][b] = X[r * CNN_IN + ((2 * px - 1 + b) & (CNN_IN - 1))];
+    for (int b = 0; b < 4; ++b) {
+      const float v = X[r * CNN_IN + ((2 * px - 1 + b) & (CNN_IN - 1))];
+      win[a][b] = make_float2(v, v);
+    }
   }
   float hi[16], lo[16];
 #pragma unroll
-  for (int o = 0; o < 16; ++o) {
-    float best = -INFINITY;
+  for (int g = 0; g < 4; ++g) {
+    float2 acc[2][2][2] = {};  // dy, dx, channel pair
 #pragma unroll
-    for (int dy = 0; dy < 2; ++dy)
+    for (int tap = 0; tap < 9; ++tap) {
+      const float4 v = sw[g][tap];
 #pragma unroll
-      for (int dx = 0; dx < 2; ++dx) {
-        float acc = 0.0f;
+      for (int dy = 0; dy < 2; ++dy)
 #pragma unroll
-        for (int ky = 0; ky < 3; ++ky)
+        for (int dx = 0; dx < 2; ++dx) {
+          const float2 x = win[dy + tap / 3][dx + tap % 3];
+          acc[dy][dx][0] = fma2(make_float2(v.x, v.y), x, acc[dy][dx][0]);
+          acc[dy][dx][1] = fma2(make_float2(v.z, v.w), x, acc[dy][dx][1]);
+        }
+    }
 #pragma unroll
-          for (int kx = 0; kx < 3; ++kx) acc = fmaf(sw[o * 9 + ky * 3 + kx], win[dy + ky][dx + kx], acc);
-        best = fmaxf(best, acc);
+    for (int e = 0; e < 4; ++e) {
+      const int o = 4 * g + e;
+      float best = -INFINITY;
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        const float2 v = acc[d >> 1][d & 1][e >> 1];
+        best = fmaxf(best, e & 1 ? v.y : v.x);
       }
-    const float y = fmaxf(best + sb[o], 0.0f) * ss[o] + sh[o];
-    split_tf32f(y, hi[o], lo[o]);
+      const float y = fmaxf(best + sb[o], 0.0f) * ss[o] + sh[o];
+      split_tf32f(y, hi[o], lo[o]);
+    }
   }
   const long long plane = (long long)B * (SO + 2) * (SO + 2) * 16;
   float* base = out + ((long long)m * 2 * B + img) * (SO + 2) * (SO + 2) * 16;
