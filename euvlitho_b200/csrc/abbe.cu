@@ -333,8 +333,8 @@ __global__ void __launch_bounds__(AB_THREADS) abbe_kernel(AbbeParams p, const do
 // what remains is the load of the E factors and a few microseconds of set-up and
 // interpolation, so it serves the calls with enough sources x pixels (band_form).
 // B200: linear model, 1024 nm, two clips of 916 sources, FP64, per launch 4930 ->
-// 129 us; 24 units of 1024 nm, 67 sources each, FP32 1215 -> 191 us; four units of
-// 2048 nm, 380 sources, FP32 7.3 -> 0.80 ms.  What bounds it now is latency: three
+// 129 us; 24 units of 1024 nm, 67 sources each, FP32 1215 -> 192 us; four units of
+// 2048 nm, 380 sources, FP32 7.3 -> 0.86 ms.  What bounds it now is latency: three
 // block barriers and one round of gathered loads per source.
 //
 // A cluster of 8 CTAs takes a share of one unit's sources: per source the E
@@ -405,11 +405,15 @@ __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(512)
   const int nloc = (p.n_src + s_step - 1) / s_step;
   int2* org = reinterpret_cast<int2*>(sm_raw);  // first order of each source's support
 
-  // origins and widths of the supports: a warp per source
+  // origins of this CTA's supports, a warp per source.  FP32: widths over all of the
+  // unit's sources, an eighth per CTA where the cluster has not all of them; the coarse
+  // grid, and with it the rounding of a field, is then the unit's alone, however many
+  // clusters share it (FP64 takes the cluster's own: 45 us less for 916 sources)
   if (tid < 2) s_w[tid] = 0;
   __syncthreads();
-  for (int ls = tid >> 5; s_first + ls * s_step < nsrc_u; ls += nt >> 5) {
-    const int* idx = p.nidx + (tab + s_first + ls * s_step) * p.ncut;
+  const bool all = s_step == BD_CL || sizeof(R) == 8;
+  auto support = [&](int s, bool width) {
+    const int* idx = p.nidx + (tab + s) * p.ncut;
     int lo = 1 << 30, hi = -(1 << 30), mo = 1 << 30, mi = -(1 << 30);
     for (int i = tid & 31; i < p.ncut; i += 32)
       if (idx[i] >= 0) {
@@ -425,14 +429,18 @@ __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(512)
       mo = min(mo, __shfl_xor_sync(0xffffffffu, mo, off));
       mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, off));
     }
-    if ((tid & 31) == 0) {
-      org[ls] = make_int2(lo, mo);
-      if (hi >= lo) {
-        atomicMax(&s_w[0], hi - lo);
-        atomicMax(&s_w[1], mi - mo);
-      }
+    if (width && (tid & 31) == 0 && hi >= lo) {
+      atomicMax(&s_w[0], hi - lo);
+      atomicMax(&s_w[1], mi - mo);
     }
+    return make_int2(lo, mo);
+  };
+  for (int ls = tid >> 5; s_first + ls * s_step < nsrc_u; ls += nt >> 5) {
+    const int2 o = support(s_first + ls * s_step, all);
+    if ((tid & 31) == 0) org[ls] = o;
   }
+  if (!all)
+    for (int s = rank + BD_CL * (tid >> 5); s < nsrc_u; s += BD_CL * (nt >> 5)) support(s, true);
   __syncthreads();
   if (tid < 2) s_all[tid] = s_w[tid];
   cluster.sync();
@@ -635,14 +643,17 @@ __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(512)
 using namespace euv;
 
 // The band-limited form pays from 2e7 field evaluations (sources x pixels x pupil
-// rows) per launch on, below that its set-up costs more than it saves, and where
-// one row pass of the widest possible support fits shared memory.
+// rows) on, and where one row pass of the widest possible support fits shared memory:
+// FP64 per launch (a 512 nm clip, 1 unit 18 us against 15, 8 units 20 against
+// 97), FP32 per unit, so that a clip's image has the same rounding in every batch (one
+// unit of 768 nm, 1e7: 42 us against 20; the eight of it 48 against 107 are forgone).
 static size_t band_least(const euv_abbe_desc* d) {
   return d->precision == EUV_PREC_MIXED ? band_bytes<float>(d->n_src, 2 * d->lpx, 2 * d->lpy, 1)
                                         : band_bytes<double>(d->n_src, 2 * d->lpx, 2 * d->lpy, 1);
 }
 static bool band_form(const euv_abbe_desc* d) {
-  const double work = (double)d->n_units * d->n_src * d->xdiv * d->ydiv * (2 * d->lpx + 1);
+  double work = (double)d->n_src * d->xdiv * d->ydiv * (2 * d->lpx + 1);
+  if (d->precision == EUV_PREC_FP64) work *= d->n_units;
   return work >= 2e7 && band_least(d) <= BD_SMEM_MAX &&
          (double)(4 * d->lpx + 8) * d->xdiv * (4 * d->lpx + 1) < 2e9 &&
          (double)(4 * d->lpy + 8) * d->ydiv * (4 * d->lpy + 1) < 2e9;  // dirichlet's range

@@ -17,11 +17,11 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("precision,tol", [(0, 1e-13), (1, 2e-5)])
 @pytest.mark.parametrize("lpx,lpy,xdiv,ydiv,units,n_src,width", [
-    (4, 4, 130, 90, 6, 41, 4),       # image sizes that are no multiples of four or eight
-    (4, 2, 256, 61, 5, 33, 8),       # supports as wide as the box
-    (20, 10, 255, 128, 4, 9, 20),    # fewer sources than two per CTA
-    (20, 20, 96, 96, 3, 40, 40),     # wide supports: several passes over rows
-    (3, 1, 512, 256, 8, 8, 0),       # a single order per source
+    (4, 4, 130, 90, 6, 200, 4),      # image sizes that are no multiples of four or eight
+    (4, 2, 256, 61, 5, 150, 8),      # supports as wide as the box
+    (20, 10, 255, 128, 4, 15, 20),   # fewer sources than two per CTA
+    (20, 20, 96, 96, 3, 60, 40),     # wide supports: several passes over rows
+    (3, 1, 512, 256, 8, 24, 0),      # a single order per source
     (41, 20, 128, 64, 2, 30, 41),    # coarse grid finer than the image along x
 ])
 def test_band_form_matches_the_sum(cuda, precision, tol, lpx, lpy, xdiv, ydiv, units, n_src, width):
@@ -53,7 +53,7 @@ def test_band_form_matches_the_sum(cuda, precision, tol, lpx, lpy, xdiv, ydiv, u
     nsrc[0] = n_src
     weight = 1.0 / rng.integers(1, 90, n_img)
     start = rng.standard_normal((n_img, xdiv, ydiv))
-    assert units * n_src * xdiv * ydiv * (2 * lpx + 1) >= 2e7  # the band form's side of the rule
+    assert n_src * xdiv * ydiv * (2 * lpx + 1) >= 2e7  # the band form's side of the rule
 
     dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
     rs = np.searchsorted(px, np.arange(-lpx, lpx + 2)).astype(np.int32)
@@ -86,3 +86,52 @@ def test_band_form_matches_the_sum(cuda, precision, tol, lpx, lpy, xdiv, ydiv, u
             ref[img[u]] += float(weight[img[u]]) * (f.real ** 2 + f.imag ** 2).sum(0)
     err = float((image - ref).abs().max() / ref.abs().max())
     assert err < tol, err
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("lpx,lpy,xdiv,ydiv,n_src", [
+    (12, 6, 256, 128, 67),    # band-limited in both precisions
+    (8, 8, 128, 128, 30),     # FP32: below the rule for one unit, so for twelve too
+])
+def test_a_unit_alone_and_among_others(cuda, precision, lpx, lpy, xdiv, ydiv, n_src):
+    """Supports of many widths: neither the form nor a source's coarse grid may depend
+    on how many units share the launch.  1e-13: only the order of the FP64 sums over
+    sources does."""
+    import torch
+    from euvlitho_b200 import _lib as L
+    units = 12
+    rng = np.random.default_rng(n_src)
+    px, py = [a.ravel().astype(np.int32) for a in np.meshgrid(
+        np.arange(-lpx, lpx + 1), np.arange(-lpy, lpy + 1), indexing="ij")]
+    ncut, n_order = px.size, 40
+    nidx = np.full((1, n_src, ncut), -1, np.int32)
+    for s in range(n_src):
+        w = rng.integers(1, 2 * lpx + 1)
+        ok = (px >= -lpx) & (px <= -lpx + w) & (np.abs(py) <= rng.integers(1, lpy + 1))
+        nidx[0, s, ok] = rng.integers(0, n_order, ok.sum())
+    cplx = lambda *sh: rng.standard_normal(sh) + 1j * rng.standard_normal(sh)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    t = {k: dev(v) for k, v in dict(
+        coef=cplx(1, n_src, ncut, 3), nidx=nidx, px=px, py=py, ax=cplx(units, n_src, n_order),
+        rs=np.searchsorted(px, np.arange(-lpx, lpx + 2)).astype(np.int32),
+        tab=np.zeros(units, np.int32), img=np.arange(units, dtype=np.int32),
+        nsrc=np.full(units, n_src, np.int32), w=np.ones(units)).items()}
+
+    def run(first, count):
+        d = L.AbbeDesc()
+        d.xdiv, d.ydiv, d.lpx, d.lpy = xdiv, ydiv, lpx, lpy
+        d.ncut, d.n_units, d.n_src, d.n_order, d.n_images = ncut, count, n_src, n_order, count
+        d.d_coef, d.d_nidx = t["coef"].data_ptr(), t["nidx"].data_ptr()
+        d.d_px, d.d_py, d.d_row_start = t["px"].data_ptr(), t["py"].data_ptr(), t["rs"].data_ptr()
+        d.d_tab_of_unit, d.d_img_of_unit = t["tab"].data_ptr(), t["img"].data_ptr()
+        d.d_nsrc_of_unit, d.d_inv_weight = t["nsrc"].data_ptr(), t["w"].data_ptr()
+        d.precision = precision
+        image = torch.zeros(count, xdiv, ydiv, dtype=torch.float64, device="cuda")
+        L.call("euv_abbe", C.byref(d), t["ax"][first:].data_ptr(), image.data_ptr(),
+               torch.cuda.current_stream().cuda_stream)
+        return image
+
+    many = run(0, units)
+    for u in (0, 7):
+        one = run(u, 1)[0]
+        assert float((one - many[u]).abs().max() / one.abs().max()) < 1e-13, u
