@@ -244,7 +244,7 @@ def dominant_kernel_roofline(plan, U, precision, dev, stream, L):
         X = torch.randn(4096, 4096, dtype=torch.complex128, device=dev)
         Y = torch.randn(4096, 4096, dtype=torch.complex128, device=dev)
         zg = 8.0 * 4096 ** 3 / (_time_ms(lambda: torch.matmul(X, Y), stream, 3) / 1e3) / 1e12
-        out = {"bound": "tensor", "kernel": "zgemm_kernel (DMMA m8n8k4 f64), batch %d x %d^3" % (U, N),
+        out = {"bound": "tensor", "kernel": "zgemm_kernel (DMMA m16n8k4 f64), batch %d x %d^3" % (U, N),
                "traffic": _traffic("zgemm_n961.json"),
                "cublas_zgemm_tflops_in_run": zg}
         out["frac_of_cublas_zgemm"] = flop / (ms / 1e3) / 1e12 / zg

@@ -259,8 +259,8 @@ typedef struct {
                             NULL: dx for every unit.  With it, dx must be the smallest
                             period over the units (it bounds the matrix norms) */
   const double* d_dy;    /* optional [U], as d_dx */
-  int euler_f;           /* EUV_PREC_MIXED: factors of the Euler product that inverts the
-                            interface matrix (1..8); 0: derived from dx, dy and k0_max so
+  int euler_f;           /* EUV_PREC_MIXED with refresh_sigma: factors of the Euler product
+                            that inverts a slice's interface matrix (1..8); 0: derived from dx, dy and k0_max so
                             that the truncation is <= 1e-7; -1: an FP64 LU instead.  Fix it
                             to make a unit's result independent of the other units of the
                             launch (the derived count depends on the smallest period) */
