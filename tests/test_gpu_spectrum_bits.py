@@ -43,3 +43,24 @@ def test_spectrum_matches_fft(cuda, vacuum, nx, ny, mesh, lh, mh, yoff, masks):
         L.call("euv_mask_spectrum", d.data_ptr(), masks, nx, ny, fx, fy, lh, mh, vacuum, yoff,
                out.data_ptr(), ws.data_ptr(), nbytes, torch.cuda.current_stream().cuda_stream)
         assert np.max(np.abs(out.cpu().numpy() - ref)) < 1e-14 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("vacuum", [0, 1])
+@pytest.mark.parametrize("nx,ny,mesh", [(672, 280, 1), (584, 424, 1), (250, 252, 2), (8, 400, 3)])
+def test_mean_is_exact(cuda, vacuum, nx, ny, mesh):
+    """F(0, 0) is a whole number of cells over all of them, rounded once (twice for the
+    absorber's 1 - F); an all-vacuum mask has exactly 1 and 0."""
+    import torch
+    from euvlitho_b200 import _lib as L
+    rng = np.random.default_rng(nx)
+    m = np.stack([np.ones((ny, nx), np.uint8), (rng.random((ny, nx)) < 0.6).astype(np.uint8)])
+    d = torch.from_numpy(np.stack([np.packbits(x.reshape(-1)) for x in m])).cuda()
+    fx, fy, lh, mh = mesh * nx, mesh * ny, 3, 2
+    out = torch.empty((2, 2 * mh + 1, 2 * lh + 1), dtype=torch.complex128, device="cuda")
+    n = L.lib().euv_mask_spectrum_workspace_bytes(2, nx, ny, fx, fy, lh, mh)
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    L.call("euv_mask_spectrum", d.data_ptr(), 2, nx, ny, fx, fy, lh, mh, vacuum, 0, out.data_ptr(),
+           ws.data_ptr(), n, torch.cuda.current_stream().cuda_stream)
+    got = out[:, mh, lh].cpu().numpy()
+    f = np.array([float(x.sum()) * mesh * mesh / (fx * fy) for x in m])
+    np.testing.assert_array_equal(got.real, f if vacuum else 1.0 - f)
