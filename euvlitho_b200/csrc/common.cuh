@@ -66,6 +66,10 @@ struct GemmTerms {
   bool paired = false;
   // FP64 form: three real products per complex one (zgemm.cu)
   bool three = false;
+  // mixed form, C = A B (m = k, n = k or 2 k): entries with apart[b] != 0 multiply the
+  // operands without the diagonals of their k x k blocks and add those rows and columns
+  // in FP64 (gemm_mixed.cu)
+  const int* apart = nullptr;
 };
 
 // Whether an inactive entry (step >= steps) of a step-predicated GEMM copies A to C.

@@ -2,7 +2,8 @@
 //
 // C = alpha*scale[b] * A B + beta C + diag*I for complex FP64 A (MxK), B (KxN),
 // C (MxN), column-major and batched (GemmTerms: the beta term may read another
-// matrix of C's shape, and a second such term may be added), computed as split-FP16x3 with power-of-two scaling: every row of
+// matrix of C's shape, and a second such term may be added; the operands' diagonals may
+// be multiplied apart), computed as split-FP16x3 with power-of-two scaling: every row of
 // A and every column of B is scaled by 2^e (e from its largest |re|, |im|, so
 // that the scaled values lie below 2^15), each scaled FP64 real is split into
 // two fp16 values x = hi + lo (hi = x rounded to fp16, lo = the remainder
@@ -58,7 +59,8 @@ constexpr int MX_EPI_WARPS = 8;
 constexpr int MX_THREADS = 64 + 32 * MX_EPI_WARPS;
 constexpr int MX_TMEM_COLS = 512;
 constexpr int MX_COL_OFF = MX_STAGES * MX_STAGE_BYTES + 256;  // column factors, after the barriers
-constexpr size_t MX_SMEM = (size_t)MX_COL_OFF + MX_BN * sizeof(double) + 1024;
+constexpr int MX_DIAG_OFF = MX_COL_OFF + MX_BN * (int)sizeof(double);  // B's diagonal (NX = 3)
+constexpr size_t MX_SMEM = (size_t)MX_DIAG_OFF + MX_BN * sizeof(double2) + 1024;
 constexpr unsigned long long MX_TIMEOUT_NS = 2000000000ull;
 // stage slot of each B plane (gmem order Re_hi, Re_lo, Im_hi, Im_lo)
 __device__ constexpr int kBSlot[4] = {0, 2, 1, 3};
@@ -67,8 +69,10 @@ struct MixedArgs {
   int m, n, kp;
   double2 alpha, beta, diag;
   const double* scale;
-  const double2* a;  // original FP64 A (copy mode)
+  const double2* a;  // original FP64 operands (copy mode, GemmTerms::apart)
   long long lda, sa;
+  const double2* b;
+  long long ldb, sb;
   double2* c;
   GemmTerms t;
   long long ldc, sc;
@@ -146,7 +150,8 @@ struct KOrder {
   }
 };
 
-// NX: matrices the epilogue adds (0: none, 1: the beta term, 2: GemmTerms::cin2 too).
+// NX: matrices the epilogue adds (0: none, 1: the beta term, 2: GemmTerms::cin2 too, 3:
+// the diagonals' rows and columns of GemmTerms::apart).
 // The epilogue cannot overlap the main loop (the four accumulators fill TMEM, the
 // stages shared memory, so an SM holds one CTA) and moves 256 KB per matrix and
 // tile: eight warps, the first chunk of the added matrices loaded and the rest
@@ -324,12 +329,24 @@ __global__ void __launch_bounds__(MX_THREADS, 1)
     const int row = m0 + q * 32 + lane;
     const bool rok = row < p.m;
     double* s_cf = reinterpret_cast<double*>(smem + MX_COL_OFF);
-    const double2* Cin = p.t.cin ? p.t.cin + (long long)b * p.t.scin : C;
-    const double2* Cin2 = NX == 2 ? p.t.cin2 + (long long)b * p.t.scin2 : C;
+    // NX = 3: C += diag(A) B + A diag(B) - diag(A) diag(B), B's k x k blocks one by one
+    const bool apart = NX == 3 && p.t.apart[b] != 0;
+    double2* s_db = reinterpret_cast<double2*>(smem + MX_DIAG_OFF);
+    const long long ld1 = NX == 3 ? p.ldb : p.ldc, ld2 = NX == 3 ? p.lda : p.ldc;
+    const double2* Cin = NX == 3  ? p.b + (long long)b * p.sb
+                         : p.t.cin ? p.t.cin + (long long)b * p.t.scin
+                                   : C;
+    const double2* Cin2 = NX == 3   ? p.a + (long long)b * p.sa
+                          : NX == 2 ? p.t.cin2 + (long long)b * p.t.scin2
+                                    : C;
+    auto block_col = [&](int col) { return NX == 3 && col >= p.m ? col - p.m : col; };
     // undo the power-of-two scaling of the operands: 2^-(exponents of row and column)
     if (threadIdx.x - 64 < MX_BN) {
       const int col = n0 + (int)threadIdx.x - 64;
       s_cf[threadIdx.x - 64] = col < p.n ? ldexp(1.0, -p.eb[(long long)b * p.n + col]) : 0.0;
+      if (NX == 3)
+        s_db[threadIdx.x - 64] = apart && col < p.n ? Cin[block_col(col) + (long long)col * ld1]
+                                                    : make_double2(0.0, 0.0);
     }
     asm volatile("bar.sync 1, %0;" ::"r"(32 * MX_EPI_WARPS) : "memory");
     const double sc = (p.scale ? p.scale[b] : 1.0) *
@@ -339,29 +356,35 @@ __global__ void __launch_bounds__(MX_THREADS, 1)
     if (NX >= 1 && p.t.beta_b) beta = beta * mk(p.t.beta_b[b].x, p.t.beta_b[b].y);
     if (NX == 2) beta2 = mk(p.t.beta2.x, p.t.beta2.y) * mk(p.t.beta2_b[b].x, p.t.beta2_b[b].y);
     const cplx dg = mk(p.diag.x, p.diag.y);
-    if (NX >= 1) {
+    if (NX == 3) {
+      const double2 da = apart && rok ? Cin2[row + (long long)row * ld2] : make_double2(0.0, 0.0);
+      beta = mk(da.x, da.y);
+    }
+    const bool adds = NX == 3 ? apart : NX >= 1;
+    if (adds) {
       // four lanes per column, one 128-byte line each
 #pragma unroll
       for (int c = lane >> 2; c < MX_BN / 2; c += 8) {
         const int r = m0 + q * 32 + (lane & 3) * 8, col = cb + c;
         if (r < p.m && col < p.n) {
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(Cin + r + (long long)col * p.ldc));
-          if (NX == 2)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(Cin2 + r + (long long)col * p.ldc));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(Cin + r + (long long)col * ld1));
+          if (NX >= 2)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(Cin2 + r +
+                                                           (long long)block_col(col) * ld2));
         }
       }
     }
-    // NX = 2: one buffer (registers), each chunk's reads with its own TMEM loads
-    constexpr int NB = NX == 2 ? 1 : 2;
+    // NX >= 2: one buffer (registers), each chunk's reads with its own TMEM loads
+    constexpr int NB = NX >= 2 ? 1 : 2;
     double2 o1[NB][EC], o2[NB][EC];
     auto fetch = [&](int ch, double2(&x1)[EC], double2(&x2)[EC]) {
 #pragma unroll
       for (int j = 0; j < EC; ++j) {
         const int col = cb + ch * EC + j;
-        const bool in = rok && col < p.n;
-        const long long at = row + (long long)col * p.ldc;
-        if (NX >= 1) x1[j] = in ? Cin[at] : make_double2(0.0, 0.0);
-        if (NX == 2) x2[j] = in ? Cin2[at] : make_double2(0.0, 0.0);
+        const bool in = adds && rok && col < p.n;
+        if (NX >= 1) x1[j] = in ? Cin[row + (long long)col * ld1] : make_double2(0.0, 0.0);
+        if (NX >= 2)
+          x2[j] = in ? Cin2[row + (long long)block_col(col) * ld2] : make_double2(0.0, 0.0);
       }
     };
     if (NX >= 1) fetch(0, o1[0], o2[0]);
@@ -381,7 +404,7 @@ __global__ void __launch_bounds__(MX_THREADS, 1)
         // the next chunk's reads before this chunk's stores: a load after a
         // store through the same pointer type would otherwise wait for it
         if (NX == 1 && ch + 1 < NCH) fetch(ch + 1, o1[(ch + 1) % NB], o2[(ch + 1) % NB]);
-        if (NX == 2 && ch > 0) fetch(ch, o1[0], o2[0]);
+        if (NX >= 2 && ch > 0) fetch(ch, o1[0], o2[0]);
         tmem_ld_wait();
         if (rok) {
 #pragma unroll
@@ -395,7 +418,9 @@ __global__ void __launch_bounds__(MX_THREADS, 1)
               cplx v = alpha * mk(f * ((double)__uint_as_float(vr[j]) + s1r),
                                   f * ((double)__uint_as_float(vi[j]) + s1i));
               if (NX >= 1) v = v + beta * mk(o1[ch % NB][j].x, o1[ch % NB][j].y);
-              if (NX == 2) v = v + beta2 * mk(o2[ch % NB][j].x, o2[ch % NB][j].y);
+              if (NX == 3) beta2 = mk(s_db[col - n0].x, s_db[col - n0].y);
+              if (NX >= 2) v = v + beta2 * mk(o2[ch % NB][j].x, o2[ch % NB][j].y);
+              if (NX == 3 && row == block_col(col)) v = v - beta * beta2;
               if (row == col) v = v + dg;
               C[row + (long long)col * p.ldc] = make_double2(v.x, v.y);
             }
@@ -443,13 +468,15 @@ __device__ __forceinline__ int scale_exponent(double mx) {
 // coalesced 512-byte column slice per warp load), pass 2 splits 32 x 32 tiles
 // transposed through shared memory (the slab is re-read from L2).
 __global__ void split_a_kernel(int M, int K, int Kp, const double2* A, long long lda,
-                               long long sa, __half* out, int* ea, const int* steps, int step) {
+                               long long sa, __half* out, int* ea, const int* steps, int step,
+                               const int* apart) {
   __shared__ double2 tile[32][33];
   __shared__ double red[8][32];
   __shared__ double s_scale[32];
   const int b = blockIdx.y;
   if (steps != nullptr && step >= steps[b]) return;  // inactive entry: the GEMM copies
   const int m0 = blockIdx.x * 32;
+  const bool ap = apart != nullptr && apart[b] != 0;
   A += (long long)b * sa;
   const int tx = threadIdx.x, ty = threadIdx.y;
   {
@@ -457,6 +484,7 @@ __global__ void split_a_kernel(int M, int K, int Kp, const double2* A, long long
     const int r = m0 + tx;
     if (r < M)
       for (int k = ty; k < K; k += 8) {
+        if (ap && k == r) continue;
         const double2 v = A[r + (long long)k * lda];
         mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
       }
@@ -476,7 +504,8 @@ __global__ void split_a_kernel(int M, int K, int Kp, const double2* A, long long
   for (int k0 = 0; k0 < Kp; k0 += 32) {
     for (int j = ty; j < 32; j += 8) {
       const int m = m0 + tx, k = k0 + j;
-      tile[j][tx] = (m < M && k < K) ? A[m + (long long)k * lda] : make_double2(0.0, 0.0);
+      tile[j][tx] = (m < M && k < K && !(ap && k == m)) ? A[m + (long long)k * lda]
+                                                        : make_double2(0.0, 0.0);
     }
     __syncthreads();
     for (int j = ty; j < 32; j += 8) {
@@ -501,15 +530,18 @@ __global__ void split_a_kernel(int M, int K, int Kp, const double2* A, long long
 // B (col-major complex K x N) -> planes [b][4][N][Kp] of fp16, K contiguous,
 // each column scaled by 2^eb[b][col]; one warp per column (max, then split).
 __global__ void split_b_kernel(int K, int N, int Kp, const double2* B, long long ldb,
-                               long long sb, __half* out, int* eb, const int* steps, int step) {
+                               long long sb, __half* out, int* eb, const int* steps, int step,
+                               const int* apart) {
   const int b = blockIdx.y;
   if (steps != nullptr && step >= steps[b]) return;
+  const bool ap = apart != nullptr && apart[b] != 0;
   const int lane = threadIdx.x & 31;
   const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (n >= N) return;  // warp-uniform
   const double2* col = B + (long long)b * sb + (long long)n * ldb;
   double mx = 0.0;
   for (int k = lane; k < K; k += 32) {
+    if (ap && k == n % K) continue;
     const double2 v = col[k];
     mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
   }
@@ -521,7 +553,7 @@ __global__ void split_b_kernel(int K, int N, int Kp, const double2* B, long long
   const long long plane = (long long)N * Kp;
   __half* o = out + (long long)b * MX_PLANES * plane + (long long)n * Kp;
   for (int k = lane; k < Kp; k += 32) {
-    const double2 v = k < K ? col[k] : make_double2(0.0, 0.0);
+    const double2 v = k < K && !(ap && k == n % K) ? col[k] : make_double2(0.0, 0.0);
     __half rh, rl, ih, il;
     split_f16(v.x * sc, rh, rl);
     split_f16(v.y * sc, ih, il);
@@ -564,7 +596,7 @@ __host__ __device__ constexpr int slab_a_stride(int K) {
 template <int R>
 __global__ void __launch_bounds__(MX_SLAB_THREADS)
     split_a_slab_kernel(int M, int K, int Kp, const double2* A, long long lda, long long sa,
-                        __half* out, int* ea, const int* steps, int step) {
+                        __half* out, int* ea, const int* steps, int step, const int* apart) {
   dependent_begin();
   extern __shared__ double2 slab[];  // [R][Ks]: element (row r, column k) at r * Ks + k
   const int Ks = slab_a_stride<R>(K);
@@ -583,6 +615,11 @@ __global__ void __launch_bounds__(MX_SLAB_THREADS)
   }
   slab_cp_wait();
   __syncthreads();
+  if (apart != nullptr && apart[b] != 0) {
+    if ((int)threadIdx.x < rows && m0 + (int)threadIdx.x < K)
+      slab[threadIdx.x * Ks + m0 + threadIdx.x] = make_double2(0.0, 0.0);
+    __syncthreads();
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < R) {
     double mx = 0.0;
@@ -625,7 +662,7 @@ __global__ void __launch_bounds__(MX_SLAB_THREADS)
 template <int R>
 __global__ void __launch_bounds__(MX_SLAB_THREADS)
     split_b_slab_kernel(int K, int N, int Kp, const double2* B, long long ldb, long long sb,
-                        __half* out, int* eb, const int* steps, int step) {
+                        __half* out, int* eb, const int* steps, int step, const int* apart) {
   dependent_begin();
   extern __shared__ double2 slab[];  // [R][K]: element (k, column c) at c * K + k
   __shared__ double s_scale[R];
@@ -641,6 +678,11 @@ __global__ void __launch_bounds__(MX_SLAB_THREADS)
   }
   slab_cp_wait();
   __syncthreads();
+  if (apart != nullptr && apart[b] != 0) {
+    if ((int)threadIdx.x < cols)
+      slab[threadIdx.x * K + (n0 + threadIdx.x) % K] = make_double2(0.0, 0.0);
+    __syncthreads();
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < R) {
     double mx = 0.0;
@@ -692,18 +734,18 @@ static int split_slab_rows(int K) {
 template <int R>
 static int launch_split_slab(bool a_role, int rows, int K, int Kp, const double2* X, long long ld,
                              long long st, __half* out, int* ex, int batch, const int* steps,
-                             int step, cudaStream_t stream) {
+                             int step, const int* apart, cudaStream_t stream) {
   static int done_a[64], done_b[64];
   const int smem = R * (a_role ? slab_a_stride<R>(K) : K) * (int)sizeof(double2);
   dim3 g((unsigned)((rows + R - 1) / R), batch);
   if (a_role) {
     EUV_CUDA_TRY(ensure_smem(split_a_slab_kernel<R>, smem, done_a));
     EUV_CUDA_TRY(launch_dependent(split_a_slab_kernel<R>, g, dim3(MX_SLAB_THREADS), smem, stream,
-                                  rows, K, Kp, X, ld, st, out, ex, steps, step));
+                                  rows, K, Kp, X, ld, st, out, ex, steps, step, apart));
   } else {
     EUV_CUDA_TRY(ensure_smem(split_b_slab_kernel<R>, smem, done_b));
     EUV_CUDA_TRY(launch_dependent(split_b_slab_kernel<R>, g, dim3(MX_SLAB_THREADS), smem, stream, K,
-                                  rows, Kp, X, ld, st, out, ex, steps, step));
+                                  rows, Kp, X, ld, st, out, ex, steps, step, apart));
   }
   EUV_LAUNCH_CHECK();
   return EUV_OK;
@@ -712,20 +754,20 @@ static int launch_split_slab(bool a_role, int rows, int K, int Kp, const double2
 // Split of one operand: A role (rows = M) or B role (rows = N, the columns).
 static int split_operand(bool a_role, int rows, int K, int Kp, const double2* X, long long ld,
                          long long st, __half* out, int* ex, int batch, const int* steps, int step,
-                         cudaStream_t stream) {
+                         const int* apart, cudaStream_t stream) {
   switch (split_slab_rows(K)) {
-    case 8: return launch_split_slab<8>(a_role, rows, K, Kp, X, ld, st, out, ex, batch, steps, step, stream);
-    case 4: return launch_split_slab<4>(a_role, rows, K, Kp, X, ld, st, out, ex, batch, steps, step, stream);
-    case 2: return launch_split_slab<2>(a_role, rows, K, Kp, X, ld, st, out, ex, batch, steps, step, stream);
-    case 1: return launch_split_slab<1>(a_role, rows, K, Kp, X, ld, st, out, ex, batch, steps, step, stream);
+    case 8: return launch_split_slab<8>(a_role, rows, K, Kp, X, ld, st, out, ex, batch, steps, step, apart, stream);
+    case 4: return launch_split_slab<4>(a_role, rows, K, Kp, X, ld, st, out, ex, batch, steps, step, apart, stream);
+    case 2: return launch_split_slab<2>(a_role, rows, K, Kp, X, ld, st, out, ex, batch, steps, step, apart, stream);
+    case 1: return launch_split_slab<1>(a_role, rows, K, Kp, X, ld, st, out, ex, batch, steps, step, apart, stream);
     default: break;
   }
   if (a_role) {
     dim3 g((rows + 31) / 32, batch), t(32, 8);
-    split_a_kernel<<<g, t, 0, stream>>>(rows, K, Kp, X, ld, st, out, ex, steps, step);
+    split_a_kernel<<<g, t, 0, stream>>>(rows, K, Kp, X, ld, st, out, ex, steps, step, apart);
   } else {
     dim3 gb((unsigned)((rows + 7) / 8), batch);
-    split_b_kernel<<<gb, 256, 0, stream>>>(K, rows, Kp, X, ld, st, out, ex, steps, step);
+    split_b_kernel<<<gb, 256, 0, stream>>>(K, rows, Kp, X, ld, st, out, ex, steps, step, apart);
   }
   EUV_LAUNCH_CHECK();
   return EUV_OK;
@@ -772,6 +814,11 @@ int gemm_mixed(int m, int n, int k, cplx alpha, const double* scale, const doubl
                const int* steps, int step, void* work, size_t work_bytes, int* status,
                cudaStream_t stream, int reuse, const GemmTerms& terms) {
   if (m <= 0 || n <= 0 || batch <= 0) return EUV_OK;
+  if (terms.apart && (m != k || (n != k && n != 2 * k) || alpha.x != 1.0 || alpha.y != 0.0 ||
+                      scale || beta.x != 0.0 || beta.y != 0.0 || steps)) {
+    euv_set_error("gemm_mixed: diagonals apart are for plain products of square blocks");
+    return EUV_ERR_BAD_ARG;
+  }
   if (k <= 0 || batch > 65535 || (size_t)batch * MX_PLANES > 0x7fffffff) {
     euv_set_error("gemm_mixed: unsupported shape");
     return EUV_ERR_BAD_ARG;
@@ -810,10 +857,12 @@ int gemm_mixed(int m, int n, int k, cplx alpha, const double* scale, const doubl
   const int sk_at = terms.need ? terms.need_above : step;
   int rc;
   if (!(reuse & 1) &&
-      (rc = split_operand(true, m, k, kp, a, lda, sa, pa, ea, batch, steps, step, stream)))
+      (rc = split_operand(true, m, k, kp, a, lda, sa, pa, ea, batch, steps, step, terms.apart,
+                          stream)))
     return rc;
   if (!(reuse & 2) &&
-      (rc = split_operand(false, n, k, kp, b, ldb, sb, pb, eb, batch, sk, sk_at, stream)))
+      (rc = split_operand(false, n, k, kp, b, ldb, sb, pb, eb, batch, sk, sk_at, terms.apart,
+                          stream)))
     return rc;
   CUtensorMap ta, tb;
   rc = make_map(&ta, pa, m, kp, batch * MX_PLANES, MX_BM);
@@ -831,6 +880,9 @@ int gemm_mixed(int m, int n, int k, cplx alpha, const double* scale, const doubl
   p.a = a;
   p.lda = lda;
   p.sa = sa;
+  p.b = b;
+  p.ldb = ldb;
+  p.sb = sb;
   p.c = c;
   p.t = terms;
   p.ldc = ldc;
@@ -841,8 +893,8 @@ int gemm_mixed(int m, int n, int k, cplx alpha, const double* scale, const doubl
   p.ea = ea;
   p.eb = eb;
   dim3 grid((m + MX_BM - 1) / MX_BM, (n + MX_BN - 1) / MX_BN, batch);
-  const int nx = terms.cin2 ? 2 : (beta.x != 0.0 || beta.y != 0.0) ? 1 : 0;
-  static int smem_done[3][64];
+  const int nx = terms.apart ? 3 : terms.cin2 ? 2 : (beta.x != 0.0 || beta.y != 0.0) ? 1 : 0;
+  static int smem_done[4][64];
   auto launch = [&](auto kernel, int* done) -> int {
     EUV_CUDA_TRY(ensure_smem(kernel, (int)MX_SMEM, done));
     EUV_CUDA_TRY(launch_dependent(kernel, grid, dim3(MX_THREADS), MX_SMEM, stream, ta, tb, p));
@@ -851,7 +903,8 @@ int gemm_mixed(int m, int n, int k, cplx alpha, const double* scale, const doubl
   };
   if (nx == 0) return launch(gemm_split3_kernel<0>, smem_done[0]);
   if (nx == 1) return launch(gemm_split3_kernel<1>, smem_done[1]);
-  return launch(gemm_split3_kernel<2>, smem_done[2]);
+  if (nx == 2) return launch(gemm_split3_kernel<2>, smem_done[2]);
+  return launch(gemm_split3_kernel<3>, smem_done[3]);
 }
 
 }  // namespace euv

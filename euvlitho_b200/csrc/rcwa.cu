@@ -566,10 +566,11 @@ __global__ void taylor_prep_kernel(int n, int batch, const double2* D, const dou
 // sum at every step; with the identity inside the operands the 2048 nm
 // eight-slice image was 1.6e-5 off, 7e-6 for the expansion about 0).  Products: q - 1 for the powers and
 // 2 (J - 1) for the two functions; q and J from poly_plan, a double-angle step
-// only where degree q * jcap is not enough (orders near grazing): a step is two
-// products, as many as one more block, and each doubles the error.  With the row recursion of euv_amp (no G^-1, no product
-// with the solved columns) the call takes 8 N^3 products instead of 25 for a 60
-// nm slab in the mixed form.  B200, whole image calls: four 1024 nm clips at N =
+// (two products, as many as one more block; it doubles the error of its operands) only
+// where degree q * jcap is not enough (orders near grazing) or the terms outgrow their
+// sum (kPolyWide).  With the row recursion of euv_amp (no G^-1, no product with the
+// solved columns) the call takes 8 N^3 products instead of 25 for a 60 nm slab in the
+// mixed form.  B200, whole image calls: four 1024 nm clips at N =
 // 625 (24 units, mixed) 11.64 -> 8.15 ms and 1.1e-5 -> 1.5e-6 of the exact image;
 // N = 961, 6 units, FP64 46.9 -> 27.2 ms; M3D at N = 2177, FP64 94.1 -> 53.5 ms.
 constexpr int PF_K = 30;       // largest degree (one per lane of a warp)
@@ -578,6 +579,17 @@ constexpr int PF_J = 5;        // largest block count
 constexpr int PF_SAMPLES = 64; // points on the ellipse
 constexpr double kPolyTolFp64 = 1e-15;  // first dropped term; the ones after it fall factorially
 constexpr double kPolyTolMixed = 5e-8;  // the split products carry ~1e-6
+// A unit in split-plane products whose poly_growth exceeds kPolyWide (an order box that is
+// wide against a period) takes double-angle steps down to kPolyGrowth, and its powers are
+// multiplied with the diagonals apart: the powers' terms are there up to e^growth / 2
+// larger than their sum, and E is mostly its diagonal, of which the FP32 sums of a power
+// lose 2^-24 at every step (GemmTerms::apart).  Image errors, root mean square of eight
+// masks, steps by degree alone -> these -> one step without the diagonals apart:
+// 1088 x 272 nm, 25 x 25 orders (growth 5.4) 1.2e-5 -> 1.4e-6 -> 5.3e-6; 256 nm, 17 x 17
+// (5.2) 5.7e-6 -> 1.0e-6 -> 4.9e-6, 19 x 19 (6.4) 5.4e-6 -> 0.9e-6 (to growth 3.2: 4.7e-6).
+// Below the line the error is 0.3 to 3e-6 as it is (296 x 1104 nm, growth 3.9: 2.4e-6).
+constexpr double kPolyWide = 4.0;
+constexpr double kPolyGrowth = 2.5;
 
 struct PolyRegion {
   cplx a, c;         // centre, focal half-axis (complex)
@@ -640,8 +652,16 @@ __host__ __device__ inline int poly_degree(const PolyRegion& g, double h, double
   return PF_K + 1;
 }
 
+// ln of the largest term of the functions' powers of E at thickness h: the maximum of
+// h |Im sqrt(a + R E)| over |E| = 1.
+__host__ __device__ inline double poly_growth(const PolyRegion& g, double h) {
+  const double a = cabs(g.a);
+  return h * (g.r <= 2.0 * a ? g.r / (2.0 * sqrt(a)) : sqrt(g.r - a));
+}
+
 struct PolyPlan {
   int q, jcap, j, m;  // powers, block limit; blocks and double-angle steps launched
+  bool apart;         // a unit's powers may need their diagonals apart
 };
 
 // q, and the block limit.  deg > 0: an estimate of the degree the launch's units
@@ -676,21 +696,20 @@ __host__ __device__ inline void poly_shape(int precision, double k, cplx eps_m1,
 }
 
 // Blocks and double-angle steps of one unit: the fewest steps with which jcap
-// blocks reach the degree, at most m_max steps.  Returns false when they do not.
-__host__ __device__ inline bool poly_pick(const PolyRegion& g, double d, double tol, int q,
-                                          int jcap, int m_max, int* j, int* m) {
+// blocks reach the degree, and of a unit beyond `wide` down to kPolyGrowth, at most m_max.
+// Returns false when the degree is not reached.
+__host__ __device__ inline bool poly_pick(const PolyRegion& g, double d, double tol, double wide,
+                                          int q, int jcap, int m_max, int* j, int* m) {
+  const double growth = poly_growth(g, d) > wide ? kPolyGrowth : 1e300;
   for (int mm = 0;; ++mm) {
-    const int deg = poly_degree(g, ldexp(d, -mm), tol);
+    const double h = ldexp(d, -mm);
+    const int deg = poly_degree(g, h, tol);
     const int jj = (deg + q - 1) / q;
-    if (jj <= jcap && deg <= PF_K) {
-      *j = jj;
+    const bool ok = jj <= jcap && deg <= PF_K;
+    if ((ok && poly_growth(g, h) <= growth) || mm >= m_max) {
+      *j = ok ? jj : jcap;
       *m = mm;
-      return true;
-    }
-    if (mm >= m_max) {
-      *j = jcap;
-      *m = mm;
-      return false;
+      return ok;
     }
   }
 }
@@ -700,13 +719,14 @@ struct PolySlices {
   const double* dxs;
   const double* dys;
   int n, lmax, mmax, n_slices, n_units;
-  double tol;
+  double tol, wide;  // wide: kPolyWide in split-plane products, else without limit
   cplx eps_m1[EUV_MAX_SLICES];
   double leps[EUV_MAX_SLICES];  // |log eps|
   double d[EUV_MAX_SLICES];
-  // blocks and steps launched (an even number) and the steps a unit may take
+  // blocks and steps launched and the steps a unit may take
   int q[EUV_MAX_SLICES], jcap[EUV_MAX_SLICES], j[EUV_MAX_SLICES], m[EUV_MAX_SLICES];
   int m_limit[EUV_MAX_SLICES];
+  bool apart[EUV_MAX_SLICES];  // some unit may be wide
 };
 
 // Coefficients of block b, function f of (unit, slice): PF_Q complex values, the
@@ -727,7 +747,8 @@ __host__ __device__ inline long long poly_id_at(int n_units, int slice, int t, i
 __global__ void __launch_bounds__(PF_SAMPLES)
     poly_coef_kernel(PolySlices p, const int* lidx, const int* midx, const double* kx0,
                      const double* ky0, const int* polar, double2* coef, double2* ident,
-                     double2* shift, double* radius, int* steps, int* blocks, int* status) {
+                     double2* shift, double* radius, int* steps, int* blocks, int* wide,
+                     int* status) {
   dependent_begin();
   const int u = blockIdx.x, sl = blockIdx.y, tid = threadIdx.x;
   __shared__ double s_lo[2], s_hi[2], s_km[2];
@@ -763,7 +784,7 @@ __global__ void __launch_bounds__(PF_SAMPLES)
   const PolyRegion g = poly_region(p.k, p.eps_m1[sl], lo, hi, w);
   const int q = p.q[sl], jl = p.j[sl];
   int jb, m;
-  bool ok = poly_pick(g, p.d[sl], p.tol, q, p.jcap[sl], p.m_limit[sl], &jb, &m);
+  bool ok = poly_pick(g, p.d[sl], p.tol, p.wide, q, p.jcap[sl], p.m_limit[sl], &jb, &m);
   if (jb > jl) {  // more blocks than launched
     jb = jl;
     ok = poly_degree(g, ldexp(p.d[sl], -m), 100.0 * p.tol) <= q * jb;
@@ -830,6 +851,7 @@ __global__ void __launch_bounds__(PF_SAMPLES)
     radius[t] = g.r;
     steps[t] = m;
     blocks[t] = jb;
+    wide[t] = poly_growth(g, p.d[sl]) > p.wide;
     cplx c = s_a[0][0], sn = s_a[1][0];
     for (int i = 0; i <= p.m[sl]; ++i) {
       ident[poly_id_at(p.n_units, sl, i, 0) + u] = make_double2(c.x, c.y);
@@ -1147,7 +1169,7 @@ int matfun(int n, int batch, const double2* D, const double* thick, double2** pc
 // Launch shape of a slice's polynomials: q of the slab, and the blocks and
 // double-angle steps of the widest ellipse any unit of the descriptor can have
 // (smallest period, incidence up to k0_max on both axes).
-static PolyPlan poly_plan(const euv_amp_desc* d, int slice, double tol) {
+static PolyPlan poly_plan(const euv_amp_desc* d, int slice, double tol, double wide) {
   const double twopi = 6.283185307179586476925286766559;
   const double gx = twopi / d->dx, gy = twopi / d->dy;
   const double k0 = d->k0_max > 0 ? d->k0_max : d->k;
@@ -1156,6 +1178,7 @@ static PolyPlan poly_plan(const euv_amp_desc* d, int slice, double tol) {
   const double leps = hypot(0.5 * log(e.x * e.x + e.y * e.y), atan2(e.y, e.x));
   const double wx = gx * d->lmax * kx, wy = gy * d->mmax * ky;
   const PolyRegion g = poly_region(d->k, em1, 0.0, kx * kx + ky * ky, leps * (wx > wy ? wx : wy));
+  const int limit = d->m_max > 0 && d->m_max < kMaxSteps ? d->m_max : kMaxSteps;
   PolyPlan r;
   int deg = 0;
   if (!d->d_dx && !d->d_dy) {
@@ -1164,15 +1187,17 @@ static PolyPlan poly_plan(const euv_amp_desc* d, int slice, double tol) {
     const double lx = gx * d->lmax, ly = gy * d->mmax;
     const bool box = d->n_orders == (2 * d->lmax + 1) * (2 * d->mmax + 1);
     const double ax = kx * kx + (box ? ly * ly : 0.0), ay = ky * ky + (box ? lx * lx : 0.0);
-    deg = poly_degree(poly_region(d->k, em1, 0.0, ax > ay ? ax : ay, leps * (wx > wy ? wx : wy)),
-                      d->dabs[slice], tol);
+    const PolyRegion t = poly_region(d->k, em1, 0.0, ax > ay ? ax : ay, leps * (wx > wy ? wx : wy));
+    double h = d->dabs[slice];
+    if (poly_growth(t, h) > wide)
+      for (int m = 0; m < limit && poly_growth(t, h) > kPolyGrowth; ++m) h *= 0.5;
+    deg = poly_degree(t, h, tol);
     if (deg > PF_K) deg = 0;
   }
   poly_shape(d->precision, d->k, em1, d->dabs[slice], deg, &r.q, &r.jcap);
-  const int limit = d->m_max > 0 && d->m_max < kMaxSteps ? d->m_max : kMaxSteps;
-  poly_pick(g, d->dabs[slice], tol, r.q, r.jcap, limit, &r.j, &r.m);
+  poly_pick(g, d->dabs[slice], tol, wide, r.q, r.jcap, limit, &r.j, &r.m);
+  r.apart = poly_growth(g, d->dabs[slice]) > wide;
   if (r.m > 0) r.j = r.jcap;  // a unit that needs fewer steps may need all the blocks
-  r.m += r.m & 1;             // steps are launched in pairs (GemmTerms::paired)
   return r;
 }
 
@@ -1210,7 +1235,7 @@ struct AmpWork {
   double2 *pw, *pair[3];  // per unit: 6 powers, three pairs of N^2 matrices
   double2 *adm, *V2, *W2, *coef, *ident, *shift;
   double *klm, *radius;
-  int *steps, *blocks, *ipiv, *info, *capped;
+  int *steps, *blocks, *wide, *ipiv, *info, *capped;
   void* mwork;
   size_t mbytes;
 };
@@ -1230,6 +1255,7 @@ static bool carve(const euv_amp_desc* d, Bump& bp, AmpWork& w) {
   w.radius = bp.take<double>(NS * U);
   w.steps = bp.take<int>(NS * U);
   w.blocks = bp.take<int>(NS * U);
+  w.wide = bp.take<int>(NS * U);
   w.ipiv = bp.take<int>(U * N);
   w.info = bp.take<int>(U);
   w.capped = bp.take<int>(1);
@@ -1369,8 +1395,9 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
   ps.n_slices = NS;
   ps.n_units = U;
   ps.tol = d->precision == EUV_PREC_MIXED ? kPolyTolMixed : kPolyTolFp64;
+  ps.wide = gemm.precision == EUV_PREC_MIXED ? kPolyWide : 1e300;
   for (int n = 0; n < NS; ++n) {
-    const PolyPlan r = poly_plan(d, n, ps.tol);
+    const PolyPlan r = poly_plan(d, n, ps.tol, ps.wide);
     const SliceParams q = slice_params(n);
     ps.eps_m1[n] = q.eps_m1;
     ps.leps[n] = cabs(q.logeps);
@@ -1379,11 +1406,13 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
     ps.jcap[n] = r.jcap;
     ps.j[n] = r.j;
     ps.m[n] = r.m;
+    ps.apart[n] = r.apart;
     ps.m_limit[n] = d->m_max > 0 && d->m_max < r.m ? d->m_max : r.m;
   }
   EUV_CUDA_TRY(launch_dependent(poly_coef_kernel, dim3(U, NS), dim3(PF_SAMPLES), 0, stream, ps,
                                 d->d_lindex, d->d_mindex, d->d_kx0, d->d_ky0, d->d_polar, w.coef,
-                                w.ident, w.shift, w.radius, w.steps, w.blocks, status));
+                                w.ident, w.shift, w.radius, w.steps, w.blocks, w.wide,
+                                status));
   EUV_LAUNCH_CHECK();
 
   // Mixed form: G^-1 by the Euler product (I - E)^-1 = prod_f (I + E^(2^f)),
@@ -1418,6 +1447,7 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
     cplx beta2 = mk(1.0, 0.0);
     const int* need = nullptr;
     int need_above = 0;
+    const int* apart = nullptr;
   };
   auto mul = [&](cplx alpha, const double* scale, const Mat& A, const Mat& B, cplx beta,
                  const Mat& C, int reuse, const Term& x = Term{}, int n = 0) -> int {
@@ -1431,6 +1461,7 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
     t.beta2_b = x.beta2_b;
     t.need = x.need;
     t.need_above = x.need_above;
+    t.apart = x.apart;
     t.three = true;
     return gemm(N, n > 0 ? n : N, N, alpha, scale, A.p, N, A.s, B.p, N, B.s, beta, C.p, N, C.s,
                 zero, U, nullptr, 0, reuse, t);
@@ -1445,10 +1476,12 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
     const int q = ps.q[n], J = ps.j[n], m = ps.m[n];
     int r2;
     // E^2; [E^3 | E^4] = E^2 [E | E^2]; [E^5 | E^6] = E^2 [E^3 | E^4]
-    if ((r2 = mul(one, nullptr, pw[0], pw[0], zero, pw[1], 0))) return r2;
-    if ((r2 = mul(one, nullptr, pw[1], pw[0], zero, pw[2], 0, Term{}, q > 3 ? 2 * N : N)))
+    Term apart;
+    if (ps.apart[n]) apart.apart = w.wide + (size_t)n * U;
+    if ((r2 = mul(one, nullptr, pw[0], pw[0], zero, pw[1], 0, apart))) return r2;
+    if ((r2 = mul(one, nullptr, pw[1], pw[0], zero, pw[2], 0, apart, q > 3 ? 2 * N : N)))
       return r2;
-    if (q > 4 && (r2 = mul(one, nullptr, pw[1], pw[2], zero, pw[4], kReuseA, Term{},
+    if (q > 4 && (r2 = mul(one, nullptr, pw[1], pw[2], zero, pw[4], kReuseA, apart,
                            q > 5 ? 2 * N : N)))
       return r2;
     const double2* pb = pw[0].p;
@@ -1479,7 +1512,8 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
       GemmTerms t;
       t.cin = s;
       t.scin = t.scin2 = 2 * nn;
-      t.three = t.paired = true;
+      t.three = true;
+      t.paired = (step | 1) < m;  // an odd count ends with a step that all units enter
       t.beta_b = w.ident + poly_id_at(U, n, step, 0);
       t.cin2 = c;
       t.beta2 = make_double2(2.0, 0.0);
