@@ -323,7 +323,8 @@ def call(fn: str, *args) -> None:
 
 _STATUS_TEXT = (
     (EUV_STATUS_TIMEOUT, "a bounded device wait gave up (results incomplete)"),
-    (EUV_STATUS_STEPS_CLAMPED, "a unit needed more double-angle steps than m_max"),
+    (EUV_STATUS_STEPS_CLAMPED, "a unit needed more double-angle steps than m_max or more blocks "
+                               "than launched, or its spectrum has no bound"),
     (EUV_STATUS_SINGULAR, "an LU met an exactly zero pivot"),
     (EUV_STATUS_NOT_CONVERGED, "an eigensolver stopped at its sweep limit"),
 )

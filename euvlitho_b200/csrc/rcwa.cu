@@ -726,6 +726,7 @@ struct PolySlices {
   // blocks and steps launched and the steps a unit may take
   int q[EUV_MAX_SLICES], jcap[EUV_MAX_SLICES], j[EUV_MAX_SLICES], m[EUV_MAX_SLICES];
   int m_limit[EUV_MAX_SLICES];
+  int m_any;  // the steps of a unit whose spectrum is no pattern's (slab_steps_kernel)
   bool apart[EUV_MAX_SLICES];  // some unit may be wide
 };
 
@@ -745,10 +746,10 @@ __host__ __device__ inline long long poly_id_at(int n_units, int slice, int t, i
 // coefficients.  Latency of one small launch for all slices; it replaces the
 // three norm / scaling launches per slice of the expansion about 0.
 __global__ void __launch_bounds__(PF_SAMPLES)
-    poly_coef_kernel(PolySlices p, const int* lidx, const int* midx, const double* kx0,
-                     const double* ky0, const int* polar, double2* coef, double2* ident,
-                     double2* shift, double* radius, int* steps, int* blocks, int* wide,
-                     int* status) {
+    poly_coef_kernel(PolySlices p, const double2* spectra, const int* spec_of_unit,
+                     const int* lidx, const int* midx, const double* kx0, const double* ky0,
+                     const int* polar, double2* coef, double2* ident, double2* shift,
+                     double* radius, int* steps, int* blocks, int* wide, int* more, int* status) {
   dependent_begin();
   const int u = blockIdx.x, sl = blockIdx.y, tid = threadIdx.x;
   __shared__ double s_lo[2], s_hi[2], s_km[2];
@@ -770,21 +771,50 @@ __global__ void __launch_bounds__(PF_SAMPLES)
     hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, off));
     km = fmax(km, __shfl_xor_sync(0xffffffffu, km, off));
   }
+  // Is this the spectrum F of a pattern with values in [0, 1]?  Then F is Hermitian, F(0)
+  // lies in [0, 1] and sum |F|^2 <= F(0).  B = sum |F| bounds any other's field of values.
+  const int W = (4 * p.lmax + 1) * (4 * p.mmax + 1);
+  const double2* F = spectra + ((long long)spec_of_unit[u] * p.n_slices + sl) * W;
+  double sum = 0.0, sq = 0.0, skew = 0.0;
+#pragma unroll 8
+  for (int i = tid; i < W; i += PF_SAMPLES) {
+    const double2 a = F[i], b = F[W - 1 - i];
+    sum += fabs(a.x) + fabs(a.y);
+    sq = fma(a.x, a.x, fma(a.y, a.y, sq));
+    skew += fabs(a.x - b.x) + fabs(a.y + b.y);
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    sq += __shfl_xor_sync(0xffffffffu, sq, off);
+    skew += __shfl_xor_sync(0xffffffffu, skew, off);
+  }
   if ((tid & 31) == 0) {
     s_lo[tid >> 5] = lo;
     s_hi[tid >> 5] = hi;
     s_km[tid >> 5] = km;
+    s_f[0][tid >> 5] = mk(sum, sq);
+    s_f[1][tid >> 5] = mk(skew, 0.0);
   }
   __syncthreads();
   lo = fmin(s_lo[0], s_lo[1]);
   hi = fmax(s_hi[0], s_hi[1]);
   km = fmax(s_km[0], s_km[1]);
+  const cplx fs = s_f[0][0] + s_f[0][1];
+  const double bound = fs.x, f0 = F[W / 2].x;
+  const bool pattern = s_f[1][0].x + s_f[1][1].x <= 1e-6 && f0 >= -1e-9 && f0 <= 1.0 + 1e-9 &&
+                       fs.y <= 1.000001 * f0 + 1e-9;
+  __syncthreads();  // s_f is written again
   // every thread takes the same decisions from the same numbers
-  const double w = (pol_x ? gx * p.lmax : gy * p.mmax) * p.leps[sl] * km;
-  const PolyRegion g = poly_region(p.k, p.eps_m1[sl], lo, hi, w);
+  double w = (pol_x ? gx * p.lmax : gy * p.mmax) * p.leps[sl] * km;
+  if (!pattern) w = 2.0 * bound * w + bound * p.k * p.k * cabs(p.eps_m1[sl]);
+  // beyond twice any pattern's (sum |re| + |im| <= sqrt(2 W)), infinite or NaN: flagged
+  const bool sane = bound <= 2.0 * sqrt(2.0 * W);
+  const PolyRegion g = poly_region(p.k, p.eps_m1[sl], lo, hi, sane ? w : 0.0);
   const int q = p.q[sl], jl = p.j[sl];
   int jb, m;
-  bool ok = poly_pick(g, p.d[sl], p.tol, p.wide, q, p.jcap[sl], p.m_limit[sl], &jb, &m);
+  bool ok = pattern ? poly_pick(g, p.d[sl], p.tol, p.wide, q, p.jcap[sl], p.m_limit[sl], &jb, &m)
+                    : poly_pick(g, p.d[sl], p.tol, p.wide, q, jl, sane ? p.m_any : 0, &jb, &m) && sane;
   if (jb > jl) {  // more blocks than launched
     jb = jl;
     ok = poly_degree(g, ldexp(p.d[sl], -m), 100.0 * p.tol) <= q * jb;
@@ -849,19 +879,93 @@ __global__ void __launch_bounds__(PF_SAMPLES)
     const cplx ia = cmul_i(g.a);
     shift[t] = make_double2(ia.x, ia.y);
     radius[t] = g.r;
-    steps[t] = m;
+    steps[t] = m < p.m[sl] ? m : p.m[sl];
+    more[t] = m - steps[t];
     blocks[t] = jb;
     wide[t] = poly_growth(g, p.d[sl]) > p.wide;
     cplx c = s_a[0][0], sn = s_a[1][0];
     for (int i = 0; i <= p.m[sl]; ++i) {
       ident[poly_id_at(p.n_units, sl, i, 0) + u] = make_double2(c.x, c.y);
       ident[poly_id_at(p.n_units, sl, i, 1) + u] = make_double2(sn.x, sn.y);
-      if (i < m) {
+      if (i < steps[t]) {
         sn = 2.0 * (sn * c);
         c = 2.0 * (c * c) - mk(1.0, 0.0);
       }
     }
     if (!ok) atomicOr(status, EUV_STATUS_STEPS_CLAMPED);
+  }
+}
+
+// Double-angle steps beyond the launched ones, of units whose spectrum is no pattern's (more
+// > 0; the others return at once: 1.5 us per slice).  A cluster of 8 CTAs per unit, S <-
+// 2 S C + 2 c0 S + 2 s0 C, C <- 2 C C + 4 c0 C between the pairs [C | S] in a and b, the
+// result in a, the identity parts in c0, s0.  Plain FP64 tiles: no caller of this library
+// takes them, they keep euv_amp right for any spectrum.
+constexpr int SX_CL = 8, SX_T = 32, SX_K = 16;
+__global__ void __cluster_dims__(SX_CL, 1, 1) __launch_bounds__(256)
+    slab_steps_kernel(int n, const int* more, double2* c0, double2* s0, double2* a, double2* b,
+                      long long sp) {
+  dependent_begin();
+  const int u = blockIdx.y;
+  const int steps = more[u];
+  if (steps <= 0) return;
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ double2 s_l[2][SX_K][SX_T], s_r[SX_T][SX_K + 1];
+  const int rank = (int)cluster.block_rank(), tx = threadIdx.x % SX_T, ty = threadIdx.x / SX_T;
+  const long long nn = (long long)n * n;
+  const int tiles = (n + SX_T - 1) / SX_T;
+  cplx c = mk(c0[u].x, c0[u].y), s = mk(s0[u].x, s0[u].y);
+  const double2* src = a + u * sp;
+  double2* dst = b + u * sp;
+  for (int t = 0; t < steps; ++t) {
+    for (int tile = rank; tile < tiles * tiles; tile += SX_CL) {
+      const int i = tile % tiles * SX_T + tx, j0 = tile / tiles * SX_T;
+      cplx acc[2][4] = {};
+      for (int k0 = 0; k0 < n; k0 += SX_K) {
+        for (int y = ty; y < SX_K; y += 8)
+          for (int f = 0; f < 2; ++f)
+            s_l[f][y][tx] = i < n && k0 + y < n ? src[f * nn + (long long)(k0 + y) * n + i]
+                                                : make_double2(0.0, 0.0);
+        for (int t2 = threadIdx.x; t2 < SX_T * SX_K; t2 += 256) {
+          const int k = k0 + t2 % SX_K, j = j0 + t2 / SX_K;
+          s_r[t2 / SX_K][t2 % SX_K] =
+              k < n && j < n ? src[(long long)j * n + k] : make_double2(0.0, 0.0);
+        }
+        __syncthreads();
+        for (int k = 0; k < SX_K; ++k)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const double2 r = s_r[ty + 8 * e][k];
+#pragma unroll
+            for (int f = 0; f < 2; ++f)
+              acc[f][e] = acc[f][e] + mk(s_l[f][k][tx].x, s_l[f][k][tx].y) * mk(r.x, r.y);
+          }
+        __syncthreads();
+      }
+      for (int e = 0; e < 4; ++e) {
+        const int j = j0 + ty + 8 * e;
+        if (i >= n || j >= n) continue;
+        const long long at = (long long)j * n + i;
+        const cplx C = mk(src[at].x, src[at].y), S = mk(src[nn + at].x, src[nn + at].y);
+        const cplx cn = 2.0 * (acc[0][e] + 2.0 * (c * C));
+        const cplx sn = 2.0 * (acc[1][e] + c * S + s * C);
+        dst[at] = make_double2(cn.x, cn.y);
+        dst[nn + at] = make_double2(sn.x, sn.y);
+      }
+    }
+    s = 2.0 * (s * c);
+    c = 2.0 * (c * c) - mk(1.0, 0.0);
+    cluster.sync();
+    const double2* p = src;
+    src = dst;
+    dst = const_cast<double2*>(p);
+  }
+  if (src != a + u * sp)
+    for (long long t = rank * 256 + threadIdx.x; t < 2 * nn; t += SX_CL * 256) dst[t] = src[t];
+  if (rank == 0 && threadIdx.x == 0) {
+    c0[u] = make_double2(c.x, c.y);
+    s0[u] = make_double2(s.x, s.y);
   }
 }
 
@@ -1235,7 +1339,7 @@ struct AmpWork {
   double2 *pw, *pair[3];  // per unit: 6 powers, three pairs of N^2 matrices
   double2 *adm, *V2, *W2, *coef, *ident, *shift;
   double *klm, *radius;
-  int *steps, *blocks, *wide, *ipiv, *info, *capped;
+  int *steps, *blocks, *wide, *more, *ipiv, *info, *capped;
   void* mwork;
   size_t mbytes;
 };
@@ -1256,6 +1360,7 @@ static bool carve(const euv_amp_desc* d, Bump& bp, AmpWork& w) {
   w.steps = bp.take<int>(NS * U);
   w.blocks = bp.take<int>(NS * U);
   w.wide = bp.take<int>(NS * U);
+  w.more = bp.take<int>(NS * U);
   w.ipiv = bp.take<int>(U * N);
   w.info = bp.take<int>(U);
   w.capped = bp.take<int>(1);
@@ -1395,6 +1500,7 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
   ps.n_slices = NS;
   ps.n_units = U;
   ps.tol = d->precision == EUV_PREC_MIXED ? kPolyTolMixed : kPolyTolFp64;
+  ps.m_any = d->m_max > 0 && d->m_max < kMaxSteps ? d->m_max : kMaxSteps;
   ps.wide = gemm.precision == EUV_PREC_MIXED ? kPolyWide : 1e300;
   for (int n = 0; n < NS; ++n) {
     const PolyPlan r = poly_plan(d, n, ps.tol, ps.wide);
@@ -1410,9 +1516,9 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
     ps.m_limit[n] = d->m_max > 0 && d->m_max < r.m ? d->m_max : r.m;
   }
   EUV_CUDA_TRY(launch_dependent(poly_coef_kernel, dim3(U, NS), dim3(PF_SAMPLES), 0, stream, ps,
-                                d->d_lindex, d->d_mindex, d->d_kx0, d->d_ky0, d->d_polar, w.coef,
+                                spec, d->d_spec, d->d_lindex, d->d_mindex, d->d_kx0, d->d_ky0, d->d_polar, w.coef,
                                 w.ident, w.shift, w.radius, w.steps, w.blocks, w.wide,
-                                status));
+                                w.more, status));
   EUV_LAUNCH_CHECK();
 
   // Mixed form: G^-1 by the Euler product (I - E)^-1 = prod_f (I + E^(2^f)),
@@ -1528,6 +1634,10 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
         return r2;
       swap(cs[0], cs[1]);
     }
+    EUV_CUDA_TRY(launch_dependent(slab_steps_kernel, dim3(SX_CL, U), dim3(256), 0, stream, N,
+                                  w.more + (size_t)n * U, w.ident + poly_id_at(U, n, m, 0),
+                                  w.ident + poly_id_at(U, n, m, 1), cs[0].p, cs[1].p, 2 * nn));
+    EUV_LAUNCH_CHECK();
     return EUV_OK;
   };
   // The boundary relation P X + Q Y = 0 of the fields at the top of the slices

@@ -46,7 +46,10 @@ extern "C" {
  * in; the caller zeroes the word and reads it when the stream is idle (the
  * reference checks none of these conditions, header.h:498,888,1529). */
 #define EUV_STATUS_TIMEOUT 1       /* a bounded device wait gave up: that call's results are incomplete */
-#define EUV_STATUS_STEPS_CLAMPED 2 /* a unit needed more double-angle steps than m_max */
+/* a unit's slab functions needed more double-angle steps than m_max (or than 40), more
+ * polynomial blocks than a launch takes, or its spectrum is not finite or too large: that
+ * unit's results are not good to the form's precision */
+#define EUV_STATUS_STEPS_CLAMPED 2
 #define EUV_STATUS_SINGULAR 4      /* an LU met an exactly zero pivot */
 #define EUV_STATUS_NOT_CONVERGED 8 /* an eigensolver stopped at its sweep limit */
 
@@ -249,9 +252,7 @@ typedef struct {
   const int* d_src_order;  /* [U][n_src] order index of each source (-1: none) */
   const double* d_src_2kz; /* [U][n_src] 2*kz of each source (header.h:1401-1409) */
   int precision;         /* EUV_PREC_FP64 or EUV_PREC_MIXED */
-  int m_max;             /* upper bound on double-angle steps; <= 0: derived.  The slab's
-                            polynomials take the spectra as those of an indicator with
-                            values in [0, 1] (euv_mask_spectrum) */
+  int m_max;             /* upper bound on double-angle steps; <= 0: derived */
   double k0_max;         /* bound on |kx0|, |ky0| over the units (<= 0: k) */
   int* d_status;         /* optional device int: EUV_STATUS_* bits OR-ed in (NULL: none) */
   const double* d_dx;    /* optional [U] clip period of each unit (nm), so that clips of
@@ -271,6 +272,11 @@ size_t euv_amp_workspace_bytes(const euv_amp_desc* desc);
  * rule above): 1..8, -1 for the FP64 LU, 0 for EUV_PREC_FP64 (the LU always);
  * -2 for an invalid descriptor.  Host only. */
 int euv_amp_euler_factors(const euv_amp_desc* desc);
+/* d_spectra: absorber spectra per clip and slice (d_spec above).  The fast path is for those
+ * of a pattern with values in [0, 1] (euv_mask_spectrum), recognised by F(-l,-m) = conj
+ * F(l,m), 0 <= F(0,0) <= 1 and sum |F|^2 <= F(0,0).  A unit with any other spectrum takes the
+ * spectrum's own bound and more steps, some by a slower kernel; one whose sum |re| + |im|
+ * exceeds twice what a pattern's can be is flagged EUV_STATUS_STEPS_CLAMPED. */
 int euv_amp(const euv_amp_desc* desc, const euv_c64* d_spectra, euv_c64* d_ax, void* d_work,
             size_t work_bytes, void* stream);
 
