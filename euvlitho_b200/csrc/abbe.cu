@@ -400,6 +400,9 @@ __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(512)
   const int rank = (int)cluster.block_rank();
   const int u = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
   const int nsrc_u = p.nsrc_of_unit[u], img = p.img_of_unit[u];
+  // clusters past the unit's sources (its slots may be padded) have nothing to add (B200,
+  // FP32, four units of 12 sources in 200 slots, 512 x 256 pixels: 337 us adding zeros, 121)
+  if ((int)(blockIdx.x / BD_CL) * BD_CL >= nsrc_u) return;
   const int s_first = blockIdx.x, s_step = gridDim.x;
   const long long tab = (long long)p.tab_of_unit[u] * p.n_src;
   const int nloc = (p.n_src + s_step - 1) / s_step;
@@ -642,11 +645,13 @@ __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(512)
 
 using namespace euv;
 
-// The band-limited form pays from 2e7 field evaluations (sources x pixels x pupil
+// The band-limited form pays from 2e7 field evaluations (source slots x pixels x pupil
 // rows) on, and where one row pass of the widest possible support fits shared memory:
 // FP64 per launch (a 512 nm clip, 1 unit 18 us against 15, 8 units 20 against
 // 97), FP32 per unit, so that a clip's image has the same rounding in every batch (one
 // unit of 768 nm, 1e7: 42 us against 20; the eight of it 48 against 107 are forgone).
+// Slots, not the unit's sources, which the host does not know: tables padded to another
+// slot count may take the other form and round differently (a server pads all alike).
 static size_t band_least(const euv_abbe_desc* d) {
   return d->precision == EUV_PREC_MIXED ? band_bytes<float>(d->n_src, 2 * d->lpx, 2 * d->lpy, 1)
                                         : band_bytes<double>(d->n_src, 2 * d->lpx, 2 * d->lpy, 1);
