@@ -72,6 +72,20 @@ struct GemmTerms {
   const int* apart = nullptr;
 };
 
+// Columns of a matrix that are source slots: column c >= first is slot c - first, and one
+// with order[b * stride + slot] < 0 is empty (a zero column, which swaps, solves and updates
+// leave as it is).
+struct Slots {
+  const int* order = nullptr;  // null: every column counts
+  long long stride = 0;
+  int first = 0;
+  __device__ __forceinline__ bool empty(int b, int c) const {
+    return order != nullptr && c >= first && order[b * stride + (c - first)] < 0;
+  }
+  // the same columns counted from column c0
+  __host__ __device__ Slots from(int c0) const { return Slots{order, stride, first - c0}; }
+};
+
 // Whether an inactive entry (step >= steps) of a step-predicated GEMM copies A to C.
 __host__ __device__ __forceinline__ bool step_copies(bool paired, int steps, int step) {
   return !paired || ((step & 1) && steps == step);

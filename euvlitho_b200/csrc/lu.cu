@@ -27,7 +27,7 @@ namespace cg = cooperative_groups;
 
 int zgemm_sub(int m, int n, int k, const double2* a, long long lda, long long sa,
               const double2* b, long long ldb, long long sb, double2* c, long long ldc,
-              long long sc, int batch, cudaStream_t stream);
+              long long sc, int batch, cudaStream_t stream, const Slots& slots = Slots{});
 int zgemm(int m, int n, int k, cplx alpha, const double* scale, const double2* a, long long lda,
           long long sa, const double2* b, long long ldb, long long sb, cplx beta, double2* c,
           long long ldc, long long sc, cplx diag, int batch, const int* steps, int step,
@@ -390,11 +390,11 @@ static bool panel16() {
 // only the later ones remain.
 __global__ void lu_laswp_kernel(int n, int ncols, int j0, int jb, int skip0, int skip1,
                                 double2* A, long long lda, long long sa, const int* ipiv,
-                                long long ipiv_stride, int sub) {
+                                long long ipiv_stride, int sub, Slots slots) {
   dependent_begin();
   const int b = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncols) return;
+  if (c >= ncols || slots.empty(b, c)) return;
   int first = j0;
   if (c >= skip0 && c < skip1) {
     if (sub <= 0) return;
@@ -421,10 +421,14 @@ __global__ void lu_laswp_kernel(int n, int ncols, int j0, int jb, int skip0, int
 constexpr int LU_TRSM_WARPS = 8;
 __global__ void __launch_bounds__(32 * LU_TRSM_WARPS)
     lu_trsm_warp_kernel(int jb, int ncols, int lower, const double2* T, long long ldt,
-                        long long st, double2* X, long long ldx, long long sx) {
+                        long long st, double2* X, long long ldx, long long sx, Slots slots) {
   dependent_begin();
   __shared__ double2 Ts[LU_NB][LU_NB + 1];
   const int b = blockIdx.y;
+  const int lane = threadIdx.x & 31;
+  const int col = blockIdx.x * LU_TRSM_WARPS + (threadIdx.x >> 5);
+  const bool live = col < ncols && !slots.empty(b, col);  // warp-uniform
+  if (slots.order != nullptr && !__syncthreads_or(live)) return;
   T += (long long)b * st;
   X += (long long)b * sx;
   for (int idx = threadIdx.x; idx < jb * jb; idx += blockDim.x) {
@@ -432,9 +436,7 @@ __global__ void __launch_bounds__(32 * LU_TRSM_WARPS)
     Ts[r][c] = T[r + (long long)c * ldt];
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int col = blockIdx.x * LU_TRSM_WARPS + (threadIdx.x >> 5);
-  if (col >= ncols) return;  // whole warps: col is warp-uniform
+  if (!live) return;  // whole warps
   double2* Xc = X + (long long)col * ldx;
   cplx x = lane < jb ? ld2(&Xc[lane]) : mk(0.0, 0.0);
   if (lower) {
@@ -523,17 +525,17 @@ static int lu_panel(int n, int j0, int jb, double2* A, long long lda, long long 
 // U12 = L11^-1 A12 and A22 -= L21 U12 of panel [j0, j0+jb) for the columns
 // [c0, c0+nc) (rows j0.. of the factor).
 static int lu_update(int n, int j0, int jb, int c0, int nc, double2* A, long long lda,
-                     long long sa, int batch, cudaStream_t st) {
+                     long long sa, int batch, cudaStream_t st, const Slots& slots) {
   if (nc <= 0) return EUV_OK;
   EUV_CUDA_TRY(launch_dependent(lu_trsm_warp_kernel, trsm_grid(nc, batch), dim3(32 * LU_TRSM_WARPS),
                                 0, st, jb, nc, 1, A + j0 + (long long)j0 * lda, lda, sa,
-                                A + j0 + (long long)c0 * lda, lda, sa));
+                                A + j0 + (long long)c0 * lda, lda, sa, slots.from(c0)));
   EUV_LAUNCH_CHECK();
   const int rest = n - j0 - jb;
   if (rest <= 0) return EUV_OK;
   return zgemm_sub(rest, nc, jb, A + (j0 + jb) + (long long)j0 * lda, lda, sa,
                    A + j0 + (long long)c0 * lda, lda, sa, A + (j0 + jb) + (long long)c0 * lda,
-                   lda, sa, batch, st);
+                   lda, sa, batch, st, slots.from(c0));
 }
 
 // Right-looking LU with one panel of look-ahead: after panel j, its update of
@@ -546,10 +548,13 @@ static int lu_update(int n, int j0, int jb, int c0, int nc, double2* A, long lon
 // finishes them).  The forward substitution so rides in launches that are there
 // anyway, most of it under the panel chain (B200, image calls, with the blocked
 // backward pass above N = 1562: 2048 nm, eight slices, 61.7 -> 53.4 ms; M3D at N =
-// 2121 44.0 -> 38.1 ms; 24 units of N = 625 6.50 -> 6.23 ms).
+// 2121 44.0 -> 38.1 ms; 24 units of N = 625 6.50 -> 6.23 ms).  order: the source slots that
+// those columns are; CTAs of empty ones only return (12 of 200 slots filled: four units of N
+// = 1681 10.70 -> 10.36 ms, six of 961 5.05 -> 4.98).
 int lu_factor(int n, double2* A, long long lda, long long sa, int* ipiv, int* info, int batch,
-              cudaStream_t stream, int extra) {
+              cudaStream_t stream, int extra, const int* order, long long ostride) {
   if (n <= 0 || batch <= 0) return EUV_OK;
+  const Slots slots{order, ostride, n};
   LuSide* side = nullptr;
   EUV_CUDA_TRY(lu_side(&side));
   zero_int_kernel<<<(batch + 255) / 256, 256, 0, stream>>>(info, batch);
@@ -562,29 +567,29 @@ int lu_factor(int n, double2* A, long long lda, long long sa, int* ipiv, int* in
     dim3 gs((n + extra + 127) / 128, batch);
     if (behind) {
       EUV_CUDA_TRY(launch_dependent(lu_laswp_kernel, gs, dim3(128), 0, stream, n, n + extra, j0, jb,
-                                    j0, j0 + jb, A, lda, sa, ipiv, n, panel_sub(n, j0)));
+                                    j0, j0 + jb, A, lda, sa, ipiv, n, panel_sub(n, j0), slots));
     } else {
       lu_laswp_kernel<<<gs, 128, 0, stream>>>(n, n + extra, j0, jb, j0, j0 + jb, A, lda, sa, ipiv, n,
-                                              panel_sub(n, j0));
+                                              panel_sub(n, j0), slots);
     }
     EUV_LAUNCH_CHECK();
     const int rest = n - j0 - jb;
     if (rest <= 0) {
-      if ((rc = lu_update(n, j0, jb, n, extra, A, lda, sa, batch, stream))) return rc;
+      if ((rc = lu_update(n, j0, jb, n, extra, A, lda, sa, batch, stream, slots))) return rc;
       break;
     }
     const int j1 = j0 + jb, nb2 = rest < LU_NB ? rest : LU_NB, rem = rest - nb2 + extra;
     const long long ctas = (long long)((rest + 31) / 32) * ((nb2 + rem + 63) / 64) * batch;
     behind = rem <= 0 || ctas <= LU_ONE_WAVE;
     if (behind) {
-      if ((rc = lu_update(n, j0, jb, j1, nb2 + rem, A, lda, sa, batch, stream))) return rc;
+      if ((rc = lu_update(n, j0, jb, j1, nb2 + rem, A, lda, sa, batch, stream, slots))) return rc;
       if ((rc = lu_panel(n, j1, nb2, A, lda, sa, ipiv, info, batch, stream, true))) return rc;
     } else {
-      if ((rc = lu_update(n, j0, jb, j1, nb2, A, lda, sa, batch, stream))) return rc;
+      if ((rc = lu_update(n, j0, jb, j1, nb2, A, lda, sa, batch, stream, slots))) return rc;
       EUV_CUDA_TRY(cudaEventRecord(side->fork, stream));
       EUV_CUDA_TRY(cudaStreamWaitEvent(side->hi, side->fork, 0));
       if ((rc = lu_panel(n, j1, nb2, A, lda, sa, ipiv, info, batch, side->hi, false))) return rc;
-      if ((rc = lu_update(n, j0, jb, j1 + nb2, rem, A, lda, sa, batch, stream))) return rc;
+      if ((rc = lu_update(n, j0, jb, j1 + nb2, rem, A, lda, sa, batch, stream, slots))) return rc;
       EUV_CUDA_TRY(cudaEventRecord(side->join, side->hi));
       EUV_CUDA_TRY(cudaStreamWaitEvent(stream, side->join, 0));
     }
@@ -867,18 +872,19 @@ static int subst(int rc, int n, int nrhs, const double2* LU, long long lda, long
 
 // U X = Y or (lower) L Y = B by blocks of LU_NB rows, two launches each.
 static int blocked_solve(bool lower, int n, int nrhs, const double2* LU, long long lda, long long sa,
-                         double2* B, long long ldb, long long sb, int batch, cudaStream_t stream) {
+                         double2* B, long long ldb, long long sb, int batch, cudaStream_t stream,
+                         const Slots& slots) {
   const int nblk = (n + LU_NB - 1) / LU_NB;
   for (int k = 0; k < nblk; ++k) {
     const int j0 = (lower ? k : nblk - 1 - k) * LU_NB, jb = (n - j0) < LU_NB ? (n - j0) : LU_NB;
     EUV_CUDA_TRY(launch_dependent(lu_trsm_warp_kernel, trsm_grid(nrhs, batch),
                                   dim3(32 * LU_TRSM_WARPS), 0, stream, jb, nrhs, lower ? 1 : 0,
-                                  LU + j0 + (long long)j0 * lda, lda, sa, B + j0, ldb, sb));
+                                  LU + j0 + (long long)j0 * lda, lda, sa, B + j0, ldb, sb, slots));
     EUV_LAUNCH_CHECK();
     const int r0 = lower ? j0 + jb : 0, rows = lower ? n - r0 : j0;
     if (rows > 0) {
       const int rc = zgemm_sub(rows, nrhs, jb, LU + r0 + (long long)j0 * lda, lda, sa, B + j0, ldb, sb,
-                               B + r0, ldb, sb, batch, stream);
+                               B + r0, ldb, sb, batch, stream, slots);
       if (rc != EUV_OK) return rc;
     }
   }
@@ -889,16 +895,17 @@ int lu_solve(int n, int nrhs, const double2* LU, long long lda, long long sa, co
              double2* B, long long ldb, long long sb, int batch, cudaStream_t stream,
              const int* order, long long ostride) {
   if (n <= 0 || nrhs <= 0 || batch <= 0) return EUV_OK;
+  const Slots slots{order, ostride, 0};
   dim3 gs((nrhs + 127) / 128, batch);
-  lu_laswp_kernel<<<gs, 128, 0, stream>>>(n, nrhs, 0, n, 0, 0, B, ldb, sb, ipiv, n, 0);
+  lu_laswp_kernel<<<gs, 128, 0, stream>>>(n, nrhs, 0, n, 0, 0, B, ldb, sb, ipiv, n, 0, slots);
   EUV_LAUNCH_CHECK();
   int cols = 0;
   int rc = subst_columns(n, nrhs, batch, order != nullptr, &cols);
   if (rc) return rc;
   if (subst_pays(cols, nrhs))
     return subst<false>(cols, n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
-  if ((rc = blocked_solve(true, n, nrhs, LU, lda, sa, B, ldb, sb, batch, stream))) return rc;
-  return blocked_solve(false, n, nrhs, LU, lda, sa, B, ldb, sb, batch, stream);
+  if ((rc = blocked_solve(true, n, nrhs, LU, lda, sa, B, ldb, sb, batch, stream, slots))) return rc;
+  return blocked_solve(false, n, nrhs, LU, lda, sa, B, ldb, sb, batch, stream, slots);
 }
 
 // U X = Y for columns that lu_factor carried along.
@@ -911,7 +918,7 @@ int lu_back(int n, int nrhs, const double2* LU, long long lda, long long sa, dou
   if (rc) return rc;
   if (subst_pays(cols, nrhs))
     return subst<true>(cols, n, nrhs, LU, lda, sa, B, ldb, sb, batch, order, ostride, stream);
-  return blocked_solve(false, n, nrhs, LU, lda, sa, B, ldb, sb, batch, stream);
+  return blocked_solve(false, n, nrhs, LU, lda, sa, B, ldb, sb, batch, stream, Slots{order, ostride, 0});
 }
 
 }  // namespace euv
@@ -929,7 +936,7 @@ extern "C" int euv_lu_factor(int n, euv_c64* d_a, int lda, long long stride_a, i
     return EUV_ERR_BAD_ARG;
   }
   return euv::lu_factor(n, reinterpret_cast<double2*>(d_a), lda, stride_a, d_ipiv, d_info, batch,
-                        (cudaStream_t)stream, 0);
+                        (cudaStream_t)stream, 0, nullptr, 0);
 }
 
 extern "C" int euv_lu_solve(int n, int nrhs, const euv_c64* d_lu, int lda, long long stride_a,

@@ -35,9 +35,10 @@ int zgemm(int m, int n, int k, cplx alpha, const double* scale, const double2* a
           long long sa, const double2* b, long long ldb, long long sb, cplx beta, double2* c,
           long long ldc, long long sc, cplx diag, int batch, const int* steps, int step,
           cudaStream_t stream, const GemmTerms& terms = GemmTerms{});
-// extra: right-hand sides in the columns after A's (L^-1 P B on return, for lu_back)
+// extra: right-hand sides in the columns after A's (L^-1 P B on return, for lu_back), order
+// as for lu_solve
 int lu_factor(int n, double2* A, long long lda, long long sa, int* ipiv, int* info, int batch,
-              cudaStream_t stream, int extra = 0);
+              cudaStream_t stream, int extra = 0, const int* order = nullptr, long long ostride = 0);
 int lu_back(int n, int nrhs, const double2* LU, long long lda, long long sa, double2* B,
             long long ldb, long long sb, int batch, cudaStream_t stream, const int* order,
             long long ostride);
@@ -1720,12 +1721,14 @@ extern "C" int euv_amp(const euv_amp_desc* d, const euv_c64* d_spectra, euv_c64*
         if ((rc = mul(one, nullptr, Q, W, one, M, 0))) return rc;
         if (ns > 0 && (rc = mul(m1, nullptr, Q, W2, one, ax, kReuseA, Term{}, ns))) return rc;
       }
-      if ((rc = lu_factor(N, M.p, N, M.s, w.ipiv, w.info, U, stream, behind ? ns : 0))) return rc;
+      if ((rc = lu_factor(N, M.p, N, M.s, w.ipiv, w.info, U, stream, behind ? ns : 0,
+                          behind ? d->d_src_order : nullptr, ns)))
+        return rc;
       EUV_CUDA_TRY(launch_dependent(flag_singular_kernel, dim3(grid1(U, 256)), dim3(256), 0, stream,
                                     w.info, U, status));
       EUV_LAUNCH_CHECK();
       if (ns > 0) {
-        // empty source slots (order < 0, zero columns) skip their CTAs
+        // CTAs of empty source slots only (order < 0, zero columns) return, as above
         if ((rc = behind ? lu_back(N, ns, M.p, N, M.s, ax.p, N, ax.s, U, stream, d->d_src_order, ns)
                          : lu_solve(N, ns, M.p, N, M.s, w.ipiv, ax.p, N, ax.s, U, stream,
                                     d->d_src_order, ns)))

@@ -49,6 +49,7 @@ struct GemmArgs {
   long long ldc, sc;
   const int* steps;
   int step;
+  Slots slots;  // of B's and C's columns (zgemm_upd_kernel)
 };
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool pred) {
@@ -95,6 +96,11 @@ __global__ void __launch_bounds__(GTHREADS, MI == 2 ? 4 : 2) zgemm_upd_kernel(Ge
   const double2* B = p.b + (long long)bz * p.sb;
   double2* C = p.c + (long long)bz * p.sc;
   const int tid = threadIdx.x;
+  if (p.slots.order != nullptr && n0 >= p.slots.first) {  // nothing but empty slots
+    const int col = n0 + tid;
+    const bool live = tid < GBN && col < p.n && !p.slots.empty(bz, col);
+    if (!__syncthreads_or(live)) return;
+  }
 
   const int warp = tid >> 5, lane = tid & 31;
   const int wm = (warp & 1) * (8 * MI), wn = (warp >> 1) * 32;
@@ -481,7 +487,7 @@ int zgemm_launch(const GemmArgs& p, int batch, cudaStream_t stream, bool upd = f
 // C -= A B (the rank-k updates of the blocked LU and its solves)
 int zgemm_sub(int m, int n, int k, const double2* a, long long lda, long long sa,
               const double2* b, long long ldb, long long sb, double2* c, long long ldc,
-              long long sc, int batch, cudaStream_t stream) {
+              long long sc, int batch, cudaStream_t stream, const Slots& slots) {
   GemmArgs p = {};
   p.m = m;
   p.n = n;
@@ -495,6 +501,7 @@ int zgemm_sub(int m, int n, int k, const double2* a, long long lda, long long sa
   p.c = c;
   p.ldc = ldc;
   p.sc = sc;
+  p.slots = slots;
   return zgemm_launch(p, batch, stream, true);
 }
 
@@ -522,6 +529,7 @@ int zgemm(int m, int n, int k, cplx alpha, const double* scale, const double2* a
   p.sc = sc;
   p.steps = steps;
   p.step = step;
+  p.slots = Slots{};
   return zgemm_launch(p, batch, stream);
 }
 
