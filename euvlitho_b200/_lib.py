@@ -33,7 +33,7 @@ EXPORTS = (
     "euv_version", "euv_last_error", "euv_kernel_launches",
     "euv_mask_spectrum_workspace_bytes", "euv_mask_spectrum",
     "euv_amp_workspace_bytes", "euv_amp", "euv_amp_euler_factors",
-    "euv_abbe", "euv_m3d_fit",
+    "euv_abbe", "euv_abbe_band", "euv_m3d_fit",
     "euv_zgemm", "euv_zgemm_mixed_workspace_bytes", "euv_zgemm_mixed", "euv_lu_workspace_bytes", "euv_lu_factor", "euv_lu_solve",
     "euv_matfun_workspace_bytes", "euv_matfun_cs", "euv_matfun_cs_noalloc",
     "euv_wait_probe", "euv_linear_amp", "euv_mask_raster_workspace_bytes", "euv_mask_raster",
@@ -48,6 +48,7 @@ EXPORTS = (
     "euv_plan_m3d_workspace_bytes", "euv_plan_m3d",
     "euv_tune_set", "euv_tune_get", "euv_tune_clear",
 )
+EUV_MIXED_FP64_ORDERS = 128
 EUV_KNOB_ABBE_SPLIT = 1
 EUV_KNOB_LU_CLUSTER = 2
 EUV_KNOB_ZGEMM_ROWS = 3
@@ -206,6 +207,8 @@ def _declare(lib: C.CDLL) -> None:
     lib.euv_mask_spectrum.argtypes = [P, i, i, i, i, i, i, i, i, i, P, P, sz, P]
     lib.euv_amp_workspace_bytes.restype = sz
     lib.euv_amp_workspace_bytes.argtypes = [C.POINTER(AmpDesc)]
+    lib.euv_abbe_band.restype = i
+    lib.euv_abbe_band.argtypes = [C.POINTER(AbbeDesc)]
     lib.euv_amp_euler_factors.restype = i
     lib.euv_amp_euler_factors.argtypes = [C.POINTER(AmpDesc)]
     lib.euv_amp.restype = i

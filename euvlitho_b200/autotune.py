@@ -9,21 +9,23 @@ built-in choice.
 
 Knobs (``EUV_KNOB_*`` in include/euvl_b200.h):
 
-* ``abbe_split``  -- key (units, source slots) of the Abbe launch: how many CTAs
-  share a unit's sources (built in: the split that fills the waves of
-  resident CTAs);
+* ``abbe_split``  -- key (units, source slots) of an Abbe launch that evaluates
+  every pixel (``euv_abbe_band`` 0): how many CTAs share a unit's sources
+  (built in: the split that fills the waves of resident CTAs);
 * ``lu_cluster``  -- key (n, batch) of an LU: the smallest CTA cluster that
   factors a panel (built in: the fewest CTAs whose registers hold its rows);
 * ``lu_subst_cols`` -- key (n, batch) of an LU solve: right-hand sides per CTA,
   8 or 12 (built in: 12 where that takes fewer waves of CTAs);
-* ``zgemm_rows``  -- key (m, batch) of the FP64 GEMM: 64- or 32-row tiles
-  (FP64 form only; the mixed form's products run on the split-FP16x3 kernel).
+* ``zgemm_rows``  -- key (m, batch) of the FP64 GEMM: 64- or 32-row tiles (the
+  FP64 form, and the mixed form up to ``EUV_MIXED_FP64_ORDERS`` orders; its
+  larger products run on the split-FP16x3 kernel).
 
 The cache file is ``$EUVLITHO_TUNE_CACHE`` or
 ``~/.cache/euvlitho_b200/tuning.json``: ``{gpu name: {"knob/k0/k1": value}}``.
 """
 from __future__ import annotations
 
+import ctypes as C
 import json
 import os
 from typing import Dict, List, Optional, Sequence, Tuple
@@ -112,9 +114,10 @@ def shapes(batch) -> Dict[str, List[Tuple[int, int]]]:
     """The keys each knob sees in one run of the batch."""
     plan = batch.plan
     N, U = plan.orders.n, batch.U
-    out = {"abbe_split": [(U, batch.ax.shape[1])], "lu_cluster": [(N, U)],
-           "lu_subst_cols": [(N, U)]}
-    if plan.precision == L.EUV_PREC_FP64:
+    out = {"lu_cluster": [(N, U)], "lu_subst_cols": [(N, U)]}
+    if not L.lib().euv_abbe_band(C.byref(batch.adesc)):
+        out["abbe_split"] = [(U, batch.ax.shape[1])]
+    if plan.precision == L.EUV_PREC_FP64 or N <= L.EUV_MIXED_FP64_ORDERS:
         out["zgemm_rows"] = [(N, U)]
     return out
 

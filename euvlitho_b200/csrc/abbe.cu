@@ -695,6 +695,13 @@ static int launch_band(const euv_abbe_desc* d, const AbbeParams& p, const double
   return EUV_OK;
 }
 
+extern "C" int euv_abbe_band(const euv_abbe_desc* d) {
+  if (!d || d->xdiv <= 0 || d->ydiv <= 0 || d->lpx < 0 || d->lpy < 0 || d->n_units <= 0 ||
+      d->n_src <= 0)
+    return -1;
+  return band_form(d) ? 1 : 0;
+}
+
 extern "C" int euv_abbe(const euv_abbe_desc* d, const euv_c64* d_ax, double* d_image,
                         void* stream_) {
   if (!d || !d_ax || !d_image || d->xdiv <= 0 || d->ydiv <= 0 ||

@@ -1189,7 +1189,7 @@ constexpr int kReuseB = 2;
 // 4.69 ms; at N = 169 4 units gain as much and 48 lose a third, so the line is drawn
 // below.  Launches of several periods (the served form) are batches by purpose and
 // keep the split planes.
-constexpr int kMixedFp64Orders = 128;
+constexpr int kMixedFp64Orders = EUV_MIXED_FP64_ORDERS;
 
 struct Gemm {
   int precision;

@@ -267,6 +267,10 @@ typedef struct {
                             launch (the derived count depends on the smallest period) */
 } euv_amp_desc;
 
+/* EUV_PREC_MIXED multiplies in FP64 up to this many orders, unless the units' periods differ
+ * (d_dx, d_dy). */
+#define EUV_MIXED_FP64_ORDERS 128
+
 size_t euv_amp_workspace_bytes(const euv_amp_desc* desc);
 /* The Euler factor count a launch with this descriptor uses (the euler_f
  * rule above): 1..8, -1 for the FP64 LU, 0 for EUV_PREC_FP64 (the LU always);
@@ -346,6 +350,10 @@ typedef struct {
   int precision;               /* EUV_PREC_FP64, or EUV_PREC_MIXED: DFT sums in FP32 */
 } euv_abbe_desc;
 
+/* 1: a launch with this descriptor's sizes takes the band-limited form (each source on the
+ * grid that its support needs), which EUV_KNOB_ABBE_SPLIT does not concern; 0: the form that
+ * evaluates every image pixel; -1: invalid sizes.  Host only. */
+int euv_abbe_band(const euv_abbe_desc* desc);
 int euv_abbe(const euv_abbe_desc* desc, const euv_c64* d_ax, double* d_image, void* stream);
 
 /* ------------------------------------------------------------------------ */
@@ -542,11 +550,13 @@ int euv_zgemm_mixed(int m, int n, int k, euv_c64 alpha, const double* d_scale,
  * themselves).  The autotuner (euvlitho_b200.autotune) times the candidates
  * on the device and writes its picks here; value 0 clears an entry, get
  * returns 0 when there is none.  Process-wide, all devices. */
-#define EUV_KNOB_ABBE_SPLIT 1 /* key (n_units, n_src) of euv_abbe: CTAs sharing a unit's
-                                 sources, 1..64 (built in: fills the waves of resident CTAs) */
+#define EUV_KNOB_ABBE_SPLIT 1 /* key (n_units, n_src) of euv_abbe (euv_abbe_band = 0): CTAs
+                                 sharing a unit's sources, 1..64 (built in: fills the waves
+                                 of resident CTAs) */
 #define EUV_KNOB_LU_CLUSTER 2 /* key (n, batch) of the LU: smallest CTA cluster of a panel,
                                  1, 2, 4 or 8 (built in: the fewest CTAs that hold the rows) */
-#define EUV_KNOB_ZGEMM_ROWS 3 /* key (m, batch) of the FP64 GEMM: row tile 64 or 32 */
+#define EUV_KNOB_ZGEMM_ROWS 3 /* key (m, batch) of the FP64 GEMM: row tile 64 or 32 (built in:
+                                 32 where 64 leaves SMs without a CTA) */
 #define EUV_KNOB_LU_SUBST_COLS 4 /* key (n, batch) of an LU solve: right-hand sides per CTA,
                                     8 or 12 (built in: 12 where that takes fewer waves,
                                     or as many when empty source slots are skipped) */
