@@ -469,6 +469,26 @@ int zgemm_launch(const GemmArgs& p, int batch, cudaStream_t stream, bool upd = f
   if (upd)
     return zgemm_run(zgemm_upd_kernel<4, GSTAGES>, GBM, GBN, zgemm_smem<4, GSTAGES>(), done[1], p,
                      batch, stream);
+  // a grid holds 65535 column tiles: the columns beyond in launches of their own (a copying
+  // step or a diagonal there would take an operand of that many rows)
+  constexpr int kCols = 65535 * PBN;
+  if (p.n > kCols) {
+    if (p.steps != nullptr || (p.m > kCols && (p.diag.x != 0.0 || p.diag.y != 0.0))) {
+      euv_set_error("zgemm: unsupported shape");
+      return EUV_ERR_BAD_ARG;
+    }
+    GemmArgs q = p;
+    for (int c0 = 0; c0 < p.n; c0 += kCols) {
+      q.n = p.n - c0 < kCols ? p.n - c0 : kCols;
+      const int rc = zgemm_launch(q, batch, stream);
+      if (rc || p.n - c0 <= kCols) return rc;
+      q.b += (long long)kCols * p.ldb;
+      q.c += (long long)kCols * p.ldc;
+      if (q.t.cin) q.t.cin += (long long)kCols * p.ldc;
+      if (q.t.cin2) q.t.cin2 += (long long)kCols * p.ldc;
+      q.diag = make_double2(0.0, 0.0);
+    }
+  }
   // 64 x 32 tiles; 32 x 32 where those leave SMs without a CTA (or the tuning
   // table says so)
   const int tuned = tune_lookup(EUV_KNOB_ZGEMM_ROWS, p.m, batch);
