@@ -160,7 +160,8 @@ static_assert(LU_NB % LC_BLK == 0, "whole blocks");
 // is left is a chain of two barriers, the reductions, the division and 31 updates of
 // a row by every thread.
 // Candidates compare as the bits of |re|+|im| (order of non-negative doubles), ties
-// to the smallest row: three warp reductions in hardware.  Lanes without a row hold
+// to the smallest row: three warp reductions in hardware.  A NaN compares as zero, so
+// that it is no pivot beside a number, as in lu_panel_kernel.  Lanes without a row hold
 // key 0 and row n.
 struct Cand {
   unsigned long long key;
@@ -174,7 +175,8 @@ __device__ __forceinline__ Cand warp_argmax(unsigned long long key, int row) {
   return Cand{((unsigned long long)mh << 32) | ml, r};
 }
 __device__ __forceinline__ unsigned long long abs_key(cplx v) {
-  return (unsigned long long)__double_as_longlong(cabs1(v));
+  const double a = cabs1(v);
+  return __double2hiint(a) > 0x7ff00000 ? 0ull : (unsigned long long)__double_as_longlong(a);
 }
 
 // 1 / d: one real division, d scaled by a power of two so that |d|^2 neither
