@@ -42,11 +42,6 @@
 
 namespace euv {
 
-int zgemm(int m, int n, int k, cplx alpha, const double* scale, const double2* a, long long lda,
-          long long sa, const double2* b, long long ldb, long long sb, cplx beta, double2* c,
-          long long ldc, long long sc, cplx diag, int batch, const int* steps, int step,
-          cudaStream_t stream);
-
 constexpr int MX_BM = 128;
 constexpr int MX_BN = 128;
 constexpr int MX_BK = 32;  // fp16 elements: 64-byte rows, one 64B swizzle span

@@ -1161,11 +1161,6 @@ struct Bump {
 
 inline unsigned grid1(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
-__global__ void fill_f64_kernel(double* p, int n, double v) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = v;
-}
-
 // An LU's zero pivots (info != 0) as EUV_STATUS_SINGULAR in the status word.
 __global__ void flag_singular_kernel(const int* info, int n, int* status) {
   dependent_begin();
