@@ -489,13 +489,17 @@ int zgemm_launch(const GemmArgs& p, int batch, cudaStream_t stream, bool upd = f
       q.diag = make_double2(0.0, 0.0);
     }
   }
-  // 64 x 32 tiles; 32 x 32 where those leave SMs without a CTA (or the tuning
-  // table says so)
+  // 64 x 32 tiles; 32 x 32 where those leave SMs without a CTA (or the tuning table says
+  // so), and of the four-product form where up to four waves of three CTAs per SM end in one
+  // of a single CTA per SM (B200, us, 64 -> 32 rows -> the tiles of 64 x 64 before: N = 961
+  // 346 -> 262 -> 303; N = 121, 64 entries, 56 -> 46 -> 49; N = 441, six, 172 -> 138 -> 145;
+  // 700 x 40 x 700, 24 entries, 255 -> 202 -> 218)
   const int tuned = tune_lookup(EUV_KNOB_ZGEMM_ROWS, p.m, batch);
   bool small = tuned == 32;
   if (tuned == 0) {
     const long long ctas = (long long)((p.m + 63) / 64) * ((p.n + PBN - 1) / PBN) * batch;
-    small = ctas < 148;
+    const int wave = 3 * 148;
+    small = ctas < 148 || (!p.t.three && ctas > wave && ctas < 4 * wave && (ctas - 1) % wave < 148);
   }
   if (p.t.three)
     return small ? zgemm_run(zgemm_kernel<true, 1>, 32, PBN, prod_smem<1>(), done[2], p, batch, stream)
