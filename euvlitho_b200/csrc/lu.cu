@@ -392,11 +392,11 @@ static bool panel16() {
 // only the later ones remain.
 __global__ void lu_laswp_kernel(int n, int ncols, int j0, int jb, int skip0, int skip1,
                                 double2* A, long long lda, long long sa, const int* ipiv,
-                                long long ipiv_stride, int sub, Slots slots) {
+                                long long ipiv_stride, int sub) {
   dependent_begin();
   const int b = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncols || slots.empty(b, c)) return;
+  if (c >= ncols) return;
   int first = j0;
   if (c >= skip0 && c < skip1) {
     if (sub <= 0) return;
@@ -430,7 +430,6 @@ __global__ void __launch_bounds__(32 * LU_TRSM_WARPS)
   const int lane = threadIdx.x & 31;
   const int col = blockIdx.x * LU_TRSM_WARPS + (threadIdx.x >> 5);
   const bool live = col < ncols && !slots.empty(b, col);  // warp-uniform
-  if (slots.order != nullptr && !__syncthreads_or(live)) return;
   T += (long long)b * st;
   X += (long long)b * sx;
   for (int idx = threadIdx.x; idx < jb * jb; idx += blockDim.x) {
@@ -438,7 +437,7 @@ __global__ void __launch_bounds__(32 * LU_TRSM_WARPS)
     Ts[r][c] = T[r + (long long)c * ldt];
   }
   __syncthreads();
-  if (!live) return;  // whole warps
+  if (!live) return;  // whole warps (the flag's load is under the staging's)
   double2* Xc = X + (long long)col * ldx;
   cplx x = lane < jb ? ld2(&Xc[lane]) : mk(0.0, 0.0);
   if (lower) {
@@ -569,10 +568,10 @@ int lu_factor(int n, double2* A, long long lda, long long sa, int* ipiv, int* in
     dim3 gs((n + extra + 127) / 128, batch);
     if (behind) {
       EUV_CUDA_TRY(launch_dependent(lu_laswp_kernel, gs, dim3(128), 0, stream, n, n + extra, j0, jb,
-                                    j0, j0 + jb, A, lda, sa, ipiv, n, panel_sub(n, j0), slots));
+                                    j0, j0 + jb, A, lda, sa, ipiv, n, panel_sub(n, j0)));
     } else {
       lu_laswp_kernel<<<gs, 128, 0, stream>>>(n, n + extra, j0, jb, j0, j0 + jb, A, lda, sa, ipiv, n,
-                                              panel_sub(n, j0), slots);
+                                              panel_sub(n, j0));
     }
     EUV_LAUNCH_CHECK();
     const int rest = n - j0 - jb;
@@ -710,11 +709,25 @@ __device__ __forceinline__ void update_rows(double2* xs, int n, const double2* L
       cplx acc[RC];
 #pragma unroll
       for (int c = 0; c < RC; ++c) acc[c] = mk(0.0, 0.0);
-#pragma unroll 8
-      for (int q = 0; q < jb; ++q) {
-        const cplx lv = ld2(&LU[r + (long long)(j0 + q) * lda]);
+      // eight loads in flight, then their products in order (left to the compiler, the
+      // loads of one right-hand side waited for each other: six matrices of N = 961 1090 or
+      // 1177 us by its version of the loop, 838 so; four of 1681, eight columns, 4.12 -> 3.83 ms)
+      const double2* lp = LU + r + (long long)j0 * lda;
+      int q = 0;
+      for (; q + 8 <= jb; q += 8) {
+        double2 lv[8];
 #pragma unroll
-        for (int c = 0; c < RC; ++c) acc[c] = acc[c] + lv * ld2(&xs[c * n + j0 + q]);
+        for (int e = 0; e < 8; ++e, lp += lda) lv[e] = *lp;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+#pragma unroll
+          for (int c = 0; c < RC; ++c)
+            acc[c] = acc[c] + mk(lv[e].x, lv[e].y) * ld2(&xs[c * n + j0 + q + e]);
+      }
+      for (; q < jb; ++q, lp += lda) {
+        const cplx l1 = ld2(lp);
+#pragma unroll
+        for (int c = 0; c < RC; ++c) acc[c] = acc[c] + l1 * ld2(&xs[c * n + j0 + q]);
       }
 #pragma unroll
       for (int c = 0; c < RC; ++c) st2(&xs[c * n + r], ld2(&xs[c * n + r]) - acc[c]);
@@ -899,7 +912,7 @@ int lu_solve(int n, int nrhs, const double2* LU, long long lda, long long sa, co
   if (n <= 0 || nrhs <= 0 || batch <= 0) return EUV_OK;
   const Slots slots{order, ostride, 0};
   dim3 gs((nrhs + 127) / 128, batch);
-  lu_laswp_kernel<<<gs, 128, 0, stream>>>(n, nrhs, 0, n, 0, 0, B, ldb, sb, ipiv, n, 0, slots);
+  lu_laswp_kernel<<<gs, 128, 0, stream>>>(n, nrhs, 0, n, 0, 0, B, ldb, sb, ipiv, n, 0);
   EUV_LAUNCH_CHECK();
   int cols = 0;
   int rc = subst_columns(n, nrhs, batch, order != nullptr, &cols);
