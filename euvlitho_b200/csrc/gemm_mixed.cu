@@ -54,8 +54,11 @@ constexpr int MX_EPI_WARPS = 8;
 constexpr int MX_THREADS = 64 + 32 * MX_EPI_WARPS;
 constexpr int MX_TMEM_COLS = 512;
 constexpr int MX_COL_OFF = MX_STAGES * MX_STAGE_BYTES + 256;  // column factors, after the barriers
-constexpr int MX_DIAG_OFF = MX_COL_OFF + MX_BN * (int)sizeof(double);  // B's diagonal (NX = 3)
-constexpr size_t MX_SMEM = (size_t)MX_DIAG_OFF + MX_BN * sizeof(double2) + 1024;
+constexpr int MX_DIAG_OFF = MX_COL_OFF + MX_BN * (int)sizeof(double);
+constexpr size_t MX_SMEM = (size_t)MX_DIAG_OFF + 1024;
+// NX = 3 holds B's diagonal too; 2 KB more for the others took L1 from their epilogues (N =
+// 169, 48 entries, 59.0 -> 59.9 us)
+constexpr size_t MX_SMEM_DIAG = MX_SMEM + MX_BN * sizeof(double2);
 constexpr unsigned long long MX_TIMEOUT_NS = 2000000000ull;
 // stage slot of each B plane (gmem order Re_hi, Re_lo, Im_hi, Im_lo)
 __device__ constexpr int kBSlot[4] = {0, 2, 1, 3};
@@ -324,23 +327,20 @@ __global__ void __launch_bounds__(MX_THREADS, 1)
     const int row = m0 + q * 32 + lane;
     const bool rok = row < p.m;
     double* s_cf = reinterpret_cast<double*>(smem + MX_COL_OFF);
+    const double2* Cin = p.t.cin ? p.t.cin + (long long)b * p.t.scin : C;
+    const double2* Cin2 = NX == 2 ? p.t.cin2 + (long long)b * p.t.scin2 : C;
     // NX = 3: C += diag(A) B + A diag(B) - diag(A) diag(B), B's k x k blocks one by one
     const bool apart = NX == 3 && p.t.apart[b] != 0;
+    const double2* Bf = NX == 3 ? p.b + (long long)b * p.sb : C;
+    const double2* Af = NX == 3 ? p.a + (long long)b * p.sa : C;
     double2* s_db = reinterpret_cast<double2*>(smem + MX_DIAG_OFF);
-    const long long ld1 = NX == 3 ? p.ldb : p.ldc, ld2 = NX == 3 ? p.lda : p.ldc;
-    const double2* Cin = NX == 3  ? p.b + (long long)b * p.sb
-                         : p.t.cin ? p.t.cin + (long long)b * p.t.scin
-                                   : C;
-    const double2* Cin2 = NX == 3   ? p.a + (long long)b * p.sa
-                          : NX == 2 ? p.t.cin2 + (long long)b * p.t.scin2
-                                    : C;
-    auto block_col = [&](int col) { return NX == 3 && col >= p.m ? col - p.m : col; };
+    auto block_col = [&](int col) { return col >= p.m ? col - p.m : col; };
     // undo the power-of-two scaling of the operands: 2^-(exponents of row and column)
     if (threadIdx.x - 64 < MX_BN) {
       const int col = n0 + (int)threadIdx.x - 64;
       s_cf[threadIdx.x - 64] = col < p.n ? ldexp(1.0, -p.eb[(long long)b * p.n + col]) : 0.0;
       if (NX == 3)
-        s_db[threadIdx.x - 64] = apart && col < p.n ? Cin[block_col(col) + (long long)col * ld1]
+        s_db[threadIdx.x - 64] = apart && col < p.n ? Bf[block_col(col) + (long long)col * p.ldb]
                                                     : make_double2(0.0, 0.0);
     }
     asm volatile("bar.sync 1, %0;" ::"r"(32 * MX_EPI_WARPS) : "memory");
@@ -352,20 +352,23 @@ __global__ void __launch_bounds__(MX_THREADS, 1)
     if (NX == 2) beta2 = mk(p.t.beta2.x, p.t.beta2.y) * mk(p.t.beta2_b[b].x, p.t.beta2_b[b].y);
     const cplx dg = mk(p.diag.x, p.diag.y);
     if (NX == 3) {
-      const double2 da = apart && rok ? Cin2[row + (long long)row * ld2] : make_double2(0.0, 0.0);
+      const double2 da = apart && rok ? Af[row + (long long)row * p.lda] : make_double2(0.0, 0.0);
       beta = mk(da.x, da.y);
     }
-    const bool adds = NX == 3 ? apart : NX >= 1;
-    if (adds) {
+    if (NX == 1 || NX == 2 || apart) {
       // four lanes per column, one 128-byte line each
 #pragma unroll
       for (int c = lane >> 2; c < MX_BN / 2; c += 8) {
         const int r = m0 + q * 32 + (lane & 3) * 8, col = cb + c;
         if (r < p.m && col < p.n) {
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(Cin + r + (long long)col * ld1));
-          if (NX >= 2)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(Cin2 + r +
-                                                           (long long)block_col(col) * ld2));
+          if (NX == 3) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(Bf + r + (long long)col * p.ldb));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(Af + r + (long long)block_col(col) * p.lda));
+          } else {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(Cin + r + (long long)col * p.ldc));
+            if (NX == 2)
+              asm volatile("prefetch.global.L2 [%0];" ::"l"(Cin2 + r + (long long)col * p.ldc));
+          }
         }
       }
     }
@@ -376,10 +379,16 @@ __global__ void __launch_bounds__(MX_THREADS, 1)
 #pragma unroll
       for (int j = 0; j < EC; ++j) {
         const int col = cb + ch * EC + j;
-        const bool in = adds && rok && col < p.n;
-        if (NX >= 1) x1[j] = in ? Cin[row + (long long)col * ld1] : make_double2(0.0, 0.0);
-        if (NX >= 2)
-          x2[j] = in ? Cin2[row + (long long)block_col(col) * ld2] : make_double2(0.0, 0.0);
+        if (NX == 3) {
+          const bool in = apart && rok && col < p.n;
+          x1[j] = in ? Bf[row + (long long)col * p.ldb] : make_double2(0.0, 0.0);
+          x2[j] = in ? Af[row + (long long)block_col(col) * p.lda] : make_double2(0.0, 0.0);
+        } else {
+          const bool in = rok && col < p.n;
+          const long long at = row + (long long)col * p.ldc;
+          if (NX >= 1) x1[j] = in ? Cin[at] : make_double2(0.0, 0.0);
+          if (NX == 2) x2[j] = in ? Cin2[at] : make_double2(0.0, 0.0);
+        }
       }
     };
     if (NX >= 1) fetch(0, o1[0], o2[0]);
@@ -890,16 +899,16 @@ int gemm_mixed(int m, int n, int k, cplx alpha, const double* scale, const doubl
   dim3 grid((m + MX_BM - 1) / MX_BM, (n + MX_BN - 1) / MX_BN, batch);
   const int nx = terms.apart ? 3 : terms.cin2 ? 2 : (beta.x != 0.0 || beta.y != 0.0) ? 1 : 0;
   static int smem_done[4][64];
-  auto launch = [&](auto kernel, int* done) -> int {
-    EUV_CUDA_TRY(ensure_smem(kernel, (int)MX_SMEM, done));
-    EUV_CUDA_TRY(launch_dependent(kernel, grid, dim3(MX_THREADS), MX_SMEM, stream, ta, tb, p));
+  auto launch = [&](auto kernel, int* done, size_t smem = MX_SMEM) -> int {
+    EUV_CUDA_TRY(ensure_smem(kernel, (int)smem, done));
+    EUV_CUDA_TRY(launch_dependent(kernel, grid, dim3(MX_THREADS), smem, stream, ta, tb, p));
     EUV_LAUNCH_CHECK();
     return EUV_OK;
   };
   if (nx == 0) return launch(gemm_split3_kernel<0>, smem_done[0]);
   if (nx == 1) return launch(gemm_split3_kernel<1>, smem_done[1]);
   if (nx == 2) return launch(gemm_split3_kernel<2>, smem_done[2]);
-  return launch(gemm_split3_kernel<3>, smem_done[3]);
+  return launch(gemm_split3_kernel<3>, smem_done[3], MX_SMEM_DIAG);
 }
 
 }  // namespace euv

@@ -534,9 +534,10 @@ static int lu_update(int n, int j0, int jb, int c0, int nc, double2* A, long lon
   EUV_LAUNCH_CHECK();
   const int rest = n - j0 - jb;
   if (rest <= 0) return EUV_OK;
+  // (below 256 rows the look at the slots takes as long as the tiles that it saves)
   return zgemm_sub(rest, nc, jb, A + (j0 + jb) + (long long)j0 * lda, lda, sa,
                    A + j0 + (long long)c0 * lda, lda, sa, A + (j0 + jb) + (long long)c0 * lda,
-                   lda, sa, batch, st, slots.from(c0));
+                   lda, sa, batch, st, rest > 256 ? slots.from(c0) : Slots{});
 }
 
 // Right-looking LU with one panel of look-ahead: after panel j, its update of

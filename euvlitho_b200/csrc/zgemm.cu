@@ -96,6 +96,11 @@ __global__ void __launch_bounds__(GTHREADS, MI == 2 ? 4 : 2) zgemm_upd_kernel(Ge
   const double2* B = p.b + (long long)bz * p.sb;
   double2* C = p.c + (long long)bz * p.sc;
   const int tid = threadIdx.x;
+  if (p.slots.order != nullptr && n0 >= p.slots.first) {  // nothing but empty slots
+    const int col = n0 + tid;
+    const bool live = tid < GBN && col < p.n && !p.slots.empty(bz, col);
+    if (!__syncthreads_or(live)) return;
+  }
 
   const int warp = tid >> 5, lane = tid & 31;
   const int wm = (warp & 1) * (8 * MI), wn = (warp >> 1) * 32;
@@ -137,14 +142,6 @@ __global__ void __launch_bounds__(GTHREADS, MI == 2 ? 4 : 2) zgemm_upd_kernel(Ge
   for (int s = 0; s < ST - 1; ++s) {
     if (s < ktiles) load_tile(s, s);
     cp_async_commit();
-  }
-  if (p.slots.order != nullptr && n0 >= p.slots.first) {  // nothing but empty slots?
-    const int col = n0 + tid;
-    const bool live = tid < GBN && col < p.n && !p.slots.empty(bz, col);
-    if (!__syncthreads_or(live)) {
-      cp_async_wait<0>();
-      return;
-    }
   }
   {
 #pragma unroll
