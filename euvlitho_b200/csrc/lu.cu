@@ -8,7 +8,7 @@
 // Blocked right-looking LU, panel width LU_NB:
 //   panel  : columns [j0, j0+nb) of rows [j0, n) (pivot = first max of
 //            |re|+|im| as LAPACK izamax, row swap, scale, rank-1 update), the
-//            rows in the registers of a cluster of up to 8 CTAs per matrix;
+//            rows in the registers of a cluster of up to 16 CTAs per matrix;
 //   laswp  : the panel's row swaps applied to the other columns;
 //   trsm   : U12 = L11^-1 A12 (unit lower, L11 staged in shared memory);
 //   update : A22 -= L21 U12 with the batched DMMA zgemm;
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(LU_PANEL_THREADS) lu_panel_kernel(int n, int j
 // register row is rotated by LC_BLK after each block (one block's code for the
 // whole panel, no runtime register indexing).  One cluster barrier per column
 // jj (a block barrier for one CTA): before it, every CTA finds its candidate (first
-// max of |re|+|im| in its rows >= jj, as izamax; every warp reduces the warp maxima
+// max of |re|+|im| in its rows >= jj, a NaN as zero; every warp reduces the warp maxima
 // itself) and sends
 // the candidate's value, index and row to every CTA through distributed shared
 // memory, one column per lane of the warp that holds the row, and rank 0 sends

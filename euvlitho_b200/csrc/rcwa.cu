@@ -565,15 +565,15 @@ __global__ void taylor_prep_kernel(int n, int batch, const double2* D, const dou
 // s - s_0 that enter later products are then small against c_0 and s_0, and so is
 // the error the split products make (their FP32 sums lose 2^-24 of the running
 // sum at every step; with the identity inside the operands the 2048 nm
-// eight-slice image was 1.6e-5 off, 7e-6 for the expansion about 0).  Products: q - 1 for the powers and
-// 2 (J - 1) for the two functions; q and J from poly_plan, a double-angle step
-// (two products, as many as one more block; it doubles the error of its operands) only
-// where degree q * jcap is not enough (orders near grazing) or the terms outgrow their
-// sum (kPolyWide).  With the row recursion of euv_amp (no G^-1, no product with the
-// solved columns) the call takes 8 N^3 products instead of 25 for a 60 nm slab in the
-// mixed form.  B200, whole image calls: four 1024 nm clips at N =
-// 625 (24 units, mixed) 11.64 -> 8.15 ms and 1.1e-5 -> 1.5e-6 of the exact image;
-// N = 961, 6 units, FP64 46.9 -> 27.2 ms; M3D at N = 2177, FP64 94.1 -> 53.5 ms.
+// eight-slice image was 1.6e-5 off, 7e-6 for the expansion about 0).  Products:
+// q - 1 for the powers and 2 (J - 1) for the two functions; q and J from poly_plan,
+// a double-angle step (two products, as many as one more block; it doubles the error
+// of its operands) only where degree q * jcap is not enough (orders near grazing) or
+// the terms outgrow their sum (kPolyWide).  With the row recursion of euv_amp (no
+// G^-1, no product with the solved columns) the call takes 8 N^3 products instead of
+// 25 for a 60 nm slab in the mixed form.  B200, whole image calls: four 1024 nm clips
+// at N = 625 (24 units, mixed) 11.64 -> 8.15 ms and 1.1e-5 -> 1.5e-6 of the exact
+// image; N = 961, 6 units, FP64 46.9 -> 27.2 ms; M3D at N = 2121, FP64 94.1 -> 53.5 ms.
 constexpr int PF_K = 30;       // largest degree (one per lane of a warp)
 constexpr int PF_Q = 6;        // largest q
 constexpr int PF_J = 5;        // largest block count
