@@ -588,7 +588,8 @@ constexpr double kPolyTolMixed = 5e-8;  // the split products carry ~1e-6
 // masks, steps by degree alone -> these -> one step without the diagonals apart:
 // 1088 x 272 nm, 25 x 25 orders (growth 5.4) 1.2e-5 -> 1.4e-6 -> 5.3e-6; 256 nm, 17 x 17
 // (5.2) 5.7e-6 -> 1.0e-6 -> 4.9e-6, 19 x 19 (6.4) 5.4e-6 -> 0.9e-6 (to growth 3.2: 4.7e-6).
-// Below the line the error is 0.3 to 3e-6 as it is (296 x 1104 nm, growth 3.9: 2.4e-6).
+// Below the line the error is 0.3 to 3e-6 as it is (296 x 1104 nm, growth 3.9: 2.4e-6),
+// up to 6e-6 for strong absorbers near grazing, where the products of the top interface set it.
 constexpr double kPolyWide = 4.0;
 constexpr double kPolyGrowth = 2.5;
 
